@@ -89,7 +89,7 @@ struct pach_run {
     int R = 0, T = 0, nsrc = 0;   // receivers and sources over all rooms
     // device buffers
     DevMem hE, hP, hDp, hDn, hAn, cnt, qa, qs0, qs1, qctl, drec, dsrc, de0, dgeo, ddirs, dw, sortbins, dprop, dcap;
-    DevMem droom, droomprim, btri, btri64, bnorm, bmat, btrans, bbvh, bbvhq;
+    DevMem droom, dsched, btri, btri64, bnorm, bmat, btrans, bbvh, bbvhq;
     // mapping receivers (has_map): the host grid and its device copy, histograms [M][8][Tm]
     bool has_map = false;
     MapGrid mg;
@@ -121,7 +121,7 @@ struct pach_run {
         }
         cudaSetDevice(scene ? scene->device : 0);
         for (DevMem *m : {&hE, &hP, &hDp, &hDn, &hAn, &cnt, &qa, &qs0, &qs1, &qctl, &drec, &dsrc, &de0, &dgeo, &ddirs, &dw,
-                          &sortbins, &dprop, &dcap, &droom, &droomprim, &btri, &btri64, &bnorm, &bmat, &btrans, &bbvh, &bbvhq,
+                          &sortbins, &dprop, &dcap, &droom, &dsched, &btri, &btri64, &bnorm, &bmat, &btrans, &bbvh, &bbvhq,
                           &mrec, &mdir, &mcell, &mentry, &mE, &mP, &mDp, &mDn, &drecid, &conv, &bak[0], &bak[1], &bak[2],
                           &bak[3], &bak[4], &bak[5]})
             m->release();
@@ -135,6 +135,20 @@ long long rprim_total(const pach_run *run) {
     long long n = 0;
     for (const RoomSpec &rm : run->rooms) n += rm.rays;
     return n;
+}
+
+// Primaries of room i among the first `done` of the run's feed order: every room's pilot, then every
+// room's other primaries (one room: its primaries in order).
+long long room_done(const pach_run *run, int i, long long done) {
+    long long pilots = 0, before_p = 0, before_r = 0;
+    for (int k = 0; k < (int)run->rooms.size(); ++k) {
+        const long long pilot = std::min(run->rooms[(size_t)k].rays, kPilotPrimaries);
+        pilots += pilot;
+        if (k < i) { before_p += pilot; before_r += run->rooms[(size_t)k].rays - pilot; }
+    }
+    const long long rays = run->rooms[(size_t)i].rays, pilot = std::min(rays, kPilotPrimaries);
+    return std::max(0ll, std::min(pilot, done - before_p)) +
+           std::max(0ll, std::min(rays - pilot, done - pilots - before_r));
 }
 
 cudaError_t upload(DevMem &m, const void *src, size_t bytes) {
@@ -324,7 +338,7 @@ bool room_setup(RoomSpec &rm, const pach_trace_params &p, std::string &err) {
 }
 
 // The run worker: uploads the run's inputs, then drives the wavefront loop on one stream --
-// iterations of feed -> broadband -> wave -> trace -> shade.  By default the whole loop is one CUDA
+// iterations of feed -> broadband -> trace -> shade.  By default the whole loop is one CUDA
 // graph launch: the iteration is captured into the body of a conditional while node whose last kernel
 // (k_cond) ends the loop when the run is done; progress and cancellation go through mapped host
 // memory.  With kernel_timing = 1 the host launches batches of iterations instead, with CUDA events
@@ -481,7 +495,20 @@ void run_worker_body(pach_run *run) {
         TRY(upload(run->dsrc, src.data(), src.size() * sizeof(float4)));
         TRY(upload(run->de0, e0.data(), e0.size() * sizeof(float)));
         TRY(upload(run->droom, rp.data(), rp.size() * sizeof(RoomParams)));
-        TRY(upload(run->droomprim, rprim.data(), rprim.size() * sizeof(long long)));
+        if (n_rooms > 1) {  // the batch's feed order (DevRun::sched_off, sched_prim), then its live counts and peaks
+            std::vector<long long> sched(5 * (size_t)n_rooms + 1, 0);
+            long long *off = sched.data(), *prim = off + 2 * n_rooms + 1;
+            long long q = rprim[0];
+            for (int k = 0; k < 2 * n_rooms; ++k) {
+                const RoomSpec &rm = run->rooms[(size_t)(k % n_rooms)];
+                const long long pilot = std::min(rm.rays, kPilotPrimaries);
+                off[k] = q;
+                prim[k] = rm.prim_begin + (k < n_rooms ? 0 : pilot);
+                q += k < n_rooms ? pilot : rm.rays - pilot;
+            }
+            off[2 * n_rooms] = q;
+            TRY(upload(run->dsched, sched.data(), sched.size() * sizeof(long long)));
+        }
         std::vector<double> gf;
         geodesic_faces(gf);
         std::vector<float4> geo(kGeoFaces * 3);
@@ -540,7 +567,7 @@ void run_worker_body(pach_run *run) {
         // default ring: room for the run's rays at up to 2048 live octave rays per primary, 2^22..2^28
         // (17 GB); default wave 8M rays -- measured against 2M: +7 % on a 20k-triangle hall and a
         // 500k-triangle arena, +19 % on a 12-triangle shoebox (fewer, fuller iterations)
-        int ring_default = 22;
+        int ring_default = n_rooms > 1 ? 24 : 22;  // a batch's pilots run several rooms at a time
         while (ring_default < 28 && (1ull << ring_default) < (unsigned long long)rprim_total(run) * 2048ull) ++ring_default;
         const int ring_log2 = run->p.ring_log2 > 0 ? std::min(32, std::max(16, run->p.ring_log2)) : ring_default;
         const unsigned long long ring_cap = 1ull << ring_log2;
@@ -572,7 +599,12 @@ void run_worker_body(pach_run *run) {
         DevRun r{};
         r.S = S;
         r.rooms = run->droom.as<RoomParams>();
-        r.room_prim = run->droomprim.as<long long>();
+        if (n_rooms > 1) {
+            r.sched_off = run->dsched.as<long long>();
+            r.sched_prim = r.sched_off + 2 * n_rooms + 1;
+            r.room_live = reinterpret_cast<unsigned *>(run->dsched.as<long long>() + 4 * n_rooms + 1);
+            r.room_peak = r.room_live + n_rooms;
+        }
         r.n_rooms = n_rooms;
         r.rec = run->drec.as<float4>();
         r.rec_id = run->drecid.as<int>();
@@ -656,7 +688,7 @@ void run_worker_body(pach_run *run) {
         r.feed_batch = run->p.feed_batch > 0 ? run->p.feed_batch : fb_default;
         const int bb_threads = 128;
         const int bb_blocks = (int)std::max<long long>(1, std::min<long long>((r.feed_batch + bb_threads - 1) / bb_threads,
-                                                                              (long long)dev_sms * 16));
+                                                                              (long long)dev_sms * 8));
         std::memset(h_ctl, 0, sizeof(WaveCtl));
         double t_trace = 0, t_shade = 0, t_bb = 0, t_sort = 0;
         long long launches = 0;
@@ -678,11 +710,10 @@ void run_worker_body(pach_run *run) {
         }
         auto one_iteration = [&](int k) -> cudaError_t {
             cudaError_t x;
-            if ((x = launch_feed(r, stream))) return x;
+            if (timing && (x = launch_feed(r, stream))) return x;  // graph mode: k_cond feeds
             if (timing && (x = cudaEventRecord(kev[6 * k], stream))) return x;
             if ((x = launch_broadband(r, bb_blocks, bb_threads, stream, map, ntri_max <= kFuseMaxTris))) return x;
             if (timing && (x = cudaEventRecord(kev[6 * k + 1], stream))) return x;
-            if ((x = launch_wave(r, stream))) return x;
             if (timing && (x = cudaEventRecord(kev[6 * k + 2], stream))) return x;
             if (sorting && (x = launch_sort(r, sort_blocks, stream))) return x;
             if (timing && (x = cudaEventRecord(kev[6 * k + 3], stream))) return x;
@@ -693,8 +724,17 @@ void run_worker_body(pach_run *run) {
             return cudaSuccess;
         };
         if (!timing) {
-            // the whole loop as one graph launch: while (k_cond says so) { one iteration }
+            // the whole loop as one graph launch: feed, then while (k_cond says so) { one iteration }
             TRY(cudaGraphCreate(&graph, 0));
+            TRY(cudaStreamBeginCaptureToGraph(stream, graph, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
+            cudaError_t fe = launch_feed(r, stream);
+            cudaGraph_t fed = nullptr;
+            cudaError_t fc = cudaStreamEndCapture(stream, &fed);
+            TRY(fe);
+            TRY(fc);
+            size_t n_first = 1;
+            cudaGraphNode_t first;
+            TRY(cudaGraphGetNodes(graph, &first, &n_first));
             cudaGraphConditionalHandle handle;
             TRY(cudaGraphConditionalHandleCreate(&handle, graph, 1, cudaGraphCondAssignDefault));
             cudaGraphNodeParams cp{};
@@ -703,7 +743,7 @@ void run_worker_body(pach_run *run) {
             cp.conditional.type = cudaGraphCondTypeWhile;
             cp.conditional.size = 1;
             cudaGraphNode_t node;
-            TRY(cudaGraphAddNode(&node, graph, nullptr, nullptr, 0, &cp));
+            TRY(cudaGraphAddNode(&node, graph, &first, nullptr, 1, &cp));
             cudaGraph_t body = cp.conditional.phGraph_out[0];
             TRY(cudaStreamBeginCaptureToGraph(stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
             cudaError_t ce = one_iteration(0);
@@ -743,7 +783,6 @@ void run_worker_body(pach_run *run) {
                 RTRY(cudaEventRecord(ev0, stream));
                 RTRY(cudaGraphLaunch(gexec, stream));
                 RTRY(cudaEventRecord(ev1, stream));
-                launches += 6;
                 // poll: progress from the mapped mirror, cancellation through the mapped flag (1: stop
                 // feeding; 2, two seconds later: stop the loop without waiting for the fed primaries)
                 auto t_cancel = std::chrono::steady_clock::now();
@@ -775,7 +814,7 @@ void run_worker_body(pach_run *run) {
                     }
                     for (int k = 0; k < batch; ++k, ++it) {
                         RTRY(one_iteration(k));
-                        launches += (sorting ? 8 : 5) - (fused ? 1 : 0);
+                        launches += (sorting ? 7 : 4) - (fused ? 1 : 0);
                     }
                     RTRY(cudaMemcpyAsync(h_ctl, run->qctl.p, sizeof(WaveCtl), cudaMemcpyDeviceToHost, stream));
                     RTRY(cudaMemcpyAsync(h_cnt, run->cnt.p, sizeof(DevCounters), cudaMemcpyDeviceToHost, stream));
@@ -918,7 +957,7 @@ void run_worker_body(pach_run *run) {
         s.broadband_ms = t_bb;
         s.sort_ms = t_sort;
         s.waves = (int64_t)h_ctl->waves;
-        s.kernel_launches = timing ? launches : (long long)h_ctl->iters * ((sorting ? 9 : 6) - (fused ? 1 : 0));
+        s.kernel_launches = timing ? launches : 1 + (long long)h_ctl->iters * ((sorting ? 7 : 4) - (fused ? 1 : 0));
         s.peak_live_rays = (int64_t)h_ctl->peak_live;
         s.bvh_nodes_visited = (int64_t)h_cnt->bvh_nodes;
         s.tri_tests = (int64_t)h_cnt->tri_tests;
@@ -1358,12 +1397,11 @@ pach_status pach_trace_get_histograms(pach_run *run, int32_t scaled, double *ene
             if (e != cudaSuccess) return fail(PACH_ERR_CUDA, cuda_msg(e, "histogram copy"));
             if (!scaled) continue;
             // Receiver_Bank.Scale(N) then, for a cluster, Scale(1/n_sources) (TaskAll:770-771), with N the
-            // primaries the receiver's room completed (rooms are fed in order)
+            // primaries the receiver's room completed
             const size_t per_rec = (size_t)it.lanes * kBands * run->T;
             double *dst = it.dst;
             for (const RoomSpec &rm : run->rooms) {
-                const long long off = rm.prim_begin - run->rooms[0].prim_begin;
-                const double N = (double)std::max(1ll, std::min(rm.rays, done - off));
+                const double N = (double)std::max(1ll, room_done(run, (int)(&rm - run->rooms.data()), done));
                 const double ns = (double)rm.src.size();
                 const double f = it.pressure ? std::sqrt(ns) / std::sqrt(N) : ns / N;
                 for (size_t i = 0; i < rm.rec.size() * per_rec; ++i) dst[i] *= f;
@@ -1391,8 +1429,7 @@ pach_status pach_trace_get_filters(pach_run *run, int32_t directional, const dou
         std::vector<double> scale;
         const long long done = run->rays_done.load();
         for (const RoomSpec &rm : run->rooms) {
-            const long long off = rm.prim_begin - run->rooms[0].prim_begin;
-            const double N = (double)std::max(1ll, std::min(rm.rays, done - off));
+            const double N = (double)std::max(1ll, room_done(run, (int)(&rm - run->rooms.data()), done));
             scale.insert(scale.end(), rm.rec.size(), std::sqrt((double)rm.src.size()) / std::sqrt(N));
         }
         const size_t wsb = filters_workspace_bytes(run->R * kinds, run->T);

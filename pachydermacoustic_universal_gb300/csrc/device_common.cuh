@@ -821,15 +821,19 @@ __device__ __forceinline__ Ray new_ray(float3 p, float3 d, float I, float scale,
     return R;
 }
 
-// Room of a primary: the last room whose first primary is <= prim (binary search of room_prim).
-__device__ __forceinline__ int room_of(const DevRun &r, long long prim) {
-    int lo = 0, hi = r.n_rooms - 1;
+// Primary and room at schedule position q: a plain run's positions are its primaries; a batch's are
+// looked up in its schedule segments (every room's pilot, then every room's rest; binary search).
+__device__ __forceinline__ long long scheduled_primary(const DevRun &r, long long q, int &room) {
+    room = 0;
+    if (r.n_rooms == 1) return q;
+    int lo = 0, hi = 2 * r.n_rooms - 1;
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
-        if (__ldg(r.room_prim + mid) <= prim) lo = mid;
+        if (__ldg(r.sched_off + mid) <= q) lo = mid;
         else hi = mid - 1;
     }
-    return lo;
+    room = lo < r.n_rooms ? lo : lo - r.n_rooms;
+    return __ldg(r.sched_prim + lo) + (q - __ldg(r.sched_off + lo));
 }
 
 // Reserves n consecutive queue slots only if they all fit; bounded retries under contention.

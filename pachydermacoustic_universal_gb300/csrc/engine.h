@@ -146,7 +146,7 @@ struct WaveCtl {
     long long pa_begin, pa_count;   // phase-A batch of the current iteration
     unsigned long long waves, overflow, peak_live;
     long long prim_first;           // first primary of the run
-    unsigned long long per_prim;    // peak ring footprint per primary measured by the pilot batch (0 = not yet)
+    unsigned long long per_prim;    // planned ring footprint per primary: 3x the pilots' largest peak (0 = none yet)
     unsigned long long trace_next;  // next wave item a trace thread takes (dynamic fetch)
     unsigned long long last_live;   // live count at the previous feed decision
     unsigned long long iters;       // loop iterations run (graph mode)
@@ -154,7 +154,9 @@ struct WaveCtl {
     int done, gave_up;
     long long pilot_count;          // primaries of the pilot in flight (0: none)
     unsigned long long pilot_peak;  // peak live count while the pilot runs
-    int pilot_room;                 // first room whose ring footprint has not been measured by a pilot
+    int pilot_first, pilot_room;    // rooms [pilot_first, pilot_room) are the pilot in flight; from pilot_room on
+                                    // no pilot has been fed
+    unsigned bb_blocks;             // blocks of the phase-A launch that have finished
     int pressure;                   // the ring passed three quarters full since the last batch was fed
 };
 
@@ -226,10 +228,14 @@ bool build_map_grid(const pach_map_desc &d, const double src[3], int nsrc, doubl
 // Launch-wide parameters (kernel argument).
 struct DevRun {
     DevScene S;
-    // rooms: room i holds primaries [room_prim[i], room_prim[i + 1])
     const RoomParams *rooms;    // [n_rooms]
-    const long long *room_prim; // [n_rooms + 1]
     int n_rooms;
+    // feed order of a batch (null for one room, whose primaries are fed in order): schedule segment i < n_rooms
+    // is room i's pilot, n_rooms + i its other primaries; segment s covers positions [sched_off[s],
+    // sched_off[s + 1]) and starts at primary sched_prim[s]
+    const long long *sched_off;   // [2 n_rooms + 1]
+    const long long *sched_prim;  // [2 n_rooms]
+    unsigned *room_live, *room_peak;  // [n_rooms] live rays of each room while pilots run, and their peaks
     // receivers of every room
     // each room's receivers ordered by the coordinate of their widest spread (measured 0.7-4.8 % faster
     // detection than the given order on a shoebox, a hall and an arena)
@@ -326,14 +332,13 @@ constexpr int kSortGrid = 8;                       // origin cells per axis
 constexpr int kSortBins = 8 * kSortGrid * kSortGrid * kSortGrid;  // x 8 direction octants
 
 // trace.cu entry points (host wrappers).  One wavefront iteration:
-//   feed (1 thread) -> broadband (phase A of the fed primaries) -> wave (1 thread: size the wave)
+//   feed (1 warp) -> broadband (phase A of the fed primaries; its last block sizes the wave)
 //   -> trace (BVH walk of every ray of the wave) -> shade (detect, absorb, scatter, append).
 cudaError_t launch_feed(const DevRun &r, cudaStream_t s);
 cudaError_t launch_cond(const DevRun &r, cudaGraphConditionalHandle h, cudaStream_t s);
 // small: every room has at most kFuseMaxTris triangles (walk with the plain stack)
 cudaError_t launch_broadband(const DevRun &r, int blocks, int threads, cudaStream_t s, bool map = false,
                              bool small = false);
-cudaError_t launch_wave(const DevRun &r, cudaStream_t s);
 cudaError_t launch_sort(const DevRun &r, int blocks, cudaStream_t s);  // count -> scan -> scatter
 // variant: 256-thread blocks per SM the trace kernel is compiled for (3..6; others -> 4), plus 16 for the
 // speculative BVH walk (compiled for 4 and 6 blocks per SM).  traversal 0 picks the speculative walk for

@@ -34,8 +34,7 @@ constexpr size_t kOffSrc = align256(kOffRec + kNaMaxReceivers * sizeof(float4));
 constexpr size_t kOffE0 = align256(kOffSrc + kNaMaxSources * sizeof(float4));
 constexpr size_t kOffGeo = align256(kOffE0 + kNaMaxSources * kBands * sizeof(float));
 constexpr size_t kOffRoom = align256(kOffGeo + kGeoFaces * 3 * sizeof(float4));
-constexpr size_t kOffRoomPrim = align256(kOffRoom + sizeof(RoomParams));
-constexpr size_t kScratchBytes = align256(kOffRoomPrim + 2 * sizeof(long long));  // ~4.7 MB
+constexpr size_t kScratchBytes = align256(kOffRoom + sizeof(RoomParams));  // ~4.7 MB
 
 // The working memory of every pach_trace_run_noalloc call on this device.  It is resident on each
 // GPU that loads the library until the process exits.  In host code the name stands for a
@@ -186,9 +185,7 @@ extern "C" pach_status pach_trace_run_noalloc(const pach_scene *scene, const pac
         room.is_order = p.is_order;
         room.pure_specular = p.pure_specular;
         room.max_broad = (int)std::fmin((double)max_broad, (double)(1u << 30));
-        const long long room_prim[2] = {room.prim_begin, room.prim_end};
         NA_TRY(cudaMemcpyAsync(base + kOffRoom, &room, sizeof(room), cudaMemcpyHostToDevice, stream));
-        NA_TRY(cudaMemcpyAsync(base + kOffRoomPrim, room_prim, sizeof(room_prim), cudaMemcpyHostToDevice, stream));
         NA_TRY(cudaMemcpyAsync(base + kOffCtl, &h_ctl, sizeof(WaveCtl), cudaMemcpyHostToDevice, stream));
         NA_TRY(cudaMemsetAsync(base + kOffCnt, 0, sizeof(DevCounters), stream));
         NA_TRY(cudaMemsetAsync(d_energy, 0, nE * sizeof(double), stream));
@@ -204,7 +201,6 @@ extern "C" pach_status pach_trace_run_noalloc(const pach_scene *scene, const pac
         r.T = (int)T;
         r.fs = (double)p.sample_rate;
         r.rooms = reinterpret_cast<const RoomParams *>(base + kOffRoom);
-        r.room_prim = reinterpret_cast<const long long *>(base + kOffRoomPrim);
         r.n_rooms = 1;
         r.src = reinterpret_cast<const float4 *>(base + kOffSrc);
         r.e0 = reinterpret_cast<const float *>(base + kOffE0);
@@ -244,11 +240,10 @@ extern "C" pach_status pach_trace_run_noalloc(const pach_scene *scene, const pac
             for (int k = 0; k < 32; ++k) {
                 NA_TRY(launch_feed(r, stream));
                 NA_TRY(launch_broadband(r, sms * 2, 128, stream, false, hs.ntri <= kFuseMaxTris));
-                NA_TRY(launch_wave(r, stream));
                 const bool fused = fused_walk(p.traversal, (int)hs.tri_poly.size());
                 if (!fused) NA_TRY(launch_trace(r, variant, tr_blocks, 256, stream));
                 NA_TRY(launch_shade(r, sh_blocks, 256, stream, fused));
-                launches += 5;
+                launches += fused ? 3 : 4;
             }
             NA_TRY(cudaMemcpyAsync(&h_ctl, base + kOffCtl, sizeof(WaveCtl), cudaMemcpyDeviceToHost, stream));
             NA_TRY(cudaStreamSynchronize(stream));

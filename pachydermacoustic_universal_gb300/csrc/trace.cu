@@ -2,14 +2,15 @@
 //
 // Hot path of SplitRayTracer.cast_ray_distributed / End_Trace ("Classes_Complete_Trace -
 // TaskAll.cs":335-536).  Octave rays live in a ring queue in HBM; every iteration of the device
-// loop runs five kernels on one stream:
-//   k_feed       1 thread: retire the last wave, hand the next batch of primaries to phase A while
+// loop runs these kernels on one stream:
+//   k_feed       1 warp: retire the last wave, hand the next batch of primaries to phase A while
 //                the ring runs low (primaries stream in until the run is done, so no launch tail).
+//                In graph mode it runs once before the loop; k_cond then does its step.
 //   k_broadband  phase A, one thread per fed primary: emission (Classes_Sources.cs:256-265,
 //                390-403), BVH walk, broadband detection (Classes_Receivers.cs:803-829), absorption
 //                (Classes_Materials.cs:166-178) and Scatter_Early (4498-4570); the band children of
-//                every bounce and the final split are appended to the ring (TaskAll:347-424).
-//   k_wave       1 thread: size the wave -- as many ring items as leave room for their outputs.
+//                every bounce and the final split are appended to the ring (TaskAll:347-424).  Its last
+//                block sizes the wave: as many ring items as leave room for their outputs.
 //   k_trace      one thread per wave item: the BVH walk only, a lean kernel that keeps many warps
 //                resident to hide L1/L2 latency; writes (triangle, t) per item.
 //   k_shade      one thread per wave item: receiver detection into FP64 histograms (837-877),
@@ -55,88 +56,164 @@ __device__ __forceinline__ unsigned long long warp_append(unsigned long long *ta
 }
 
 // ------------------------------------------------------------------------------------------
-// scheduling (single thread)
+// scheduling (one warp)
 // ------------------------------------------------------------------------------------------
-__global__ void k_feed(DevRun r) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+// Primaries are fed in schedule order.  A plain run's schedule is its primaries in order; a batch's is
+// every room's pilot (its first kPilotPrimaries primaries, room by room) and then every room's rest,
+// with sched_off / sched_prim (2 n_rooms segments) mapping schedule positions to primaries.
+//
+// Pilots measure the ring footprint the feed plans batches with: the peak live count per primary (x 3)
+// of the hungriest room.  The margin: a pilot fits in one wave, so each wave advances its trees by a
+// whole level, while a batch larger than a wave is traced first-in-first-out across two levels at once
+// and peaks higher per primary (measured up to 2.7x on 12-receiver shoeboxes at 20k primaries);
+// size_wave doubles the figure again when the ring passes three quarters full.
+//
+// A pilot counts as measured once its live count has fallen an eighth below its peak: split trees grow
+// while phase-B rays carry energy and only shrink afterwards, so the peak is over by then.  Waiting for
+// the pilot's last ray instead cost a second full chain of waves, each a few launch latencies long
+// (1003-primary shoebox 260 waves, now 228; 2500-primary hall with a map 228, now 182).  Rooms of a
+// batch are counted separately (room_live), so after the first room's pilot the others run together, as
+// many as the plan lets into half the ring: 8 rooms x 500 primaries take 381 waves and 288 ms where one
+// pilot after another took about 1100 waves and 445 ms.
+
+// Pilot footprint of the group in flight, or false while it may still grow.  All 32 lanes call.
+__device__ bool pilots_measured(const DevRun &r, WaveCtl *c, unsigned long long live, bool decaying,
+                                unsigned long long &pp) {
+    const int lane = threadIdx.x & 31;
+    if (r.n_rooms == 1) {
+        if (live != 0 && !(decaying && live <= c->pilot_peak - c->pilot_peak / 8)) return false;
+        pp = c->pilot_peak * 3 / (unsigned long long)c->pilot_count + 1;
+        return true;
+    }
+    const int g0 = c->pilot_first, g1 = c->pilot_room;
+    bool ok = true;
+    unsigned long long best = 0;
+    for (int i = g0 + lane; i < g1; i += 32) {
+        const unsigned peak = r.room_peak[i], now = r.room_live[i];
+        ok = ok && (now == 0 || now <= peak - peak / 8);
+        const long long n = g1 - g0 == 1 ? c->pilot_count : r.sched_off[i + 1] - r.sched_off[i];
+        const unsigned long long v = (unsigned long long)peak * 3 / (unsigned long long)n + 1;
+        if (v > best) best = v;
+    }
+    if (!__all_sync(FULL, ok)) return false;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long v = __shfl_xor_sync(FULL, best, o);
+        if (v > best) best = v;
+    }
+    pp = best;
+    return true;
+}
+
+// Retires the last wave and decides what phase A gets next.  All 32 lanes call; lane 0 writes.
+__device__ void feed_step(const DevRun &r) {
     WaveCtl *c = r.ctl;
-    c->head += c->m;  // retire the previous wave
+    const int lane = threadIdx.x & 31;
+    const unsigned long long head = c->head + c->m;
+    const unsigned long long live = c->tail - head;
+    const bool decaying = live <= c->last_live;
+    const bool done = c->done != 0;
+    long long prim_end = c->prim_end;
+    const long long next = c->next_prim;
+    // cancellation (graph mode): stop feeding; the primaries already fed run to completion
+    int cancelled = 0;
+    if (lane == 0 && r.cancel && prim_end > next) cancelled = *r.cancel;
+    if (__shfl_sync(FULL, cancelled, 0)) prim_end = next;
+    unsigned long long pp = 0;
+    const bool in_flight = c->pilot_count > 0;
+    const bool measured = !done && in_flight && pilots_measured(r, c, live, decaying, pp);
+    __syncwarp();
+    if (lane != 0) return;
+    c->head = head;
     c->m = 0;
     c->pa_count = 0;
-    if (c->done) return;
-    // cancellation (graph mode): stop feeding; the primaries already fed run to completion
-    if (r.cancel && *r.cancel && c->prim_end > c->next_prim) c->prim_end = c->next_prim;
-    const unsigned long long live = c->tail - c->head;
-    // Pilots: the first kPilotPrimaries primaries of every room (of a plain run: of the run) are fed
-    // alone; once their split trees are done, their peak live count per primary (x 3) is the ring
-    // footprint the feed plans batches with -- the largest over the rooms measured so far, so a room
-    // whose split trees outgrow an earlier room's cannot overfill the ring.  The margin: a pilot fits
-    // in one wave, so each wave advances its trees by a whole level, while a batch larger than a wave
-    // is traced first-in-first-out across two levels at once and peaks higher per primary (measured
-    // up to 2.7x on 12-receiver shoeboxes at 20k primaries); k_wave doubles the figure again when the
-    // ring passes three quarters full.
-    if (c->pilot_count > 0) {
-        if (live != 0) return;
-        unsigned long long pp = c->pilot_peak * 3 / (unsigned long long)c->pilot_count + 1;
+    if (done) return;
+    c->prim_end = prim_end;
+    c->last_live = live;
+    if (in_flight) {
+        if (!measured) return;
         if (pp < r.feed_bound) pp = r.feed_bound;
         if (pp > c->per_prim) c->per_prim = pp;
         c->pilot_count = 0;
     }
-    if (c->next_prim >= c->prim_end) return;
-    const int room = room_of(r, c->next_prim);
-    if (room >= c->pilot_room) {
-        if (live != 0) return;  // the pilot runs alone: the ring drains first
-        const long long room_end = room + 1 < r.n_rooms ? __ldg(r.room_prim + room + 1) : c->prim_end;
-        long long n = room_end - c->next_prim;
-        if (n > kPilotPrimaries) n = kPilotPrimaries;
-        if (n > r.feed_batch) n = r.feed_batch;
-        if (n > c->prim_end - c->next_prim) n = c->prim_end - c->next_prim;
-        const long long fit = (long long)(r.ring_cap / r.feed_bound);  // >= 4: checked at set-up
-        if (n > fit) n = fit;
-        if (n < 1) n = 1;
-        c->pa_begin = c->next_prim;
-        c->pa_count = n;
-        c->next_prim += n;
-        c->pilot_count = n;
-        c->pilot_peak = 0;
-        c->pilot_room = room + 1;
-        c->last_live = 0;
-        return;
+    if (next >= prim_end) return;
+    const unsigned long long half = r.ring_cap / 2;
+    const unsigned long long per_prim = c->per_prim ? c->per_prim : r.feed_bound;
+    // hard limit: the phase-A output of every fed primary must fit
+    unsigned long long fit = (r.ring_cap - live) / r.feed_bound;
+    if (fit > (unsigned long long)r.feed_batch) fit = (unsigned long long)r.feed_batch;
+    if (fit > (unsigned long long)(prim_end - next)) fit = (unsigned long long)(prim_end - next);
+    long long lim = prim_end - next;
+    if (c->pilot_room < r.n_rooms) {
+        // a batch never reaches into a pilot that has not run
+        const long long first = r.n_rooms == 1 ? next : __ldg(r.sched_off + c->pilot_room);
+        if (next >= first) {
+            int k = c->pilot_room;
+            unsigned long long n = 0;
+            if (r.n_rooms == 1 || c->per_prim == 0) {  // the first pilot runs alone
+                if (live != 0) return;
+                n = r.n_rooms == 1 ? (unsigned long long)kPilotPrimaries
+                                   : (unsigned long long)(__ldg(r.sched_off + k + 1) - next);
+                ++k;
+            } else {
+                unsigned long long plan = live < half ? (half - live) / per_prim : 0;
+                if (plan > fit) plan = fit;
+                while (k < r.n_rooms) {
+                    const unsigned long long q = (unsigned long long)(__ldg(r.sched_off + k + 1) - next);
+                    if (q > plan && !(n == 0 && live == 0)) break;
+                    n = q;
+                    ++k;
+                    if (q > plan) break;  // alone and larger than the plan: fed in part
+                }
+                if (n == 0) return;
+            }
+            if (n > (unsigned long long)kPilotPrimaries && r.n_rooms == 1) n = kPilotPrimaries;
+            if (n > fit) n = fit;
+            if (n < 1) n = 1;  // the ring holds the phase-A output of at least 4 primaries: checked at set-up
+            c->pa_begin = next;
+            c->pa_count = (long long)n;
+            c->next_prim = next + (long long)n;
+            c->pilot_count = (long long)n;
+            c->pilot_peak = 0;
+            c->pilot_first = c->pilot_room;
+            c->pilot_room = k;
+            c->last_live = 0;
+            return;
+        }
+        if (lim > first - next) lim = first - next;
     }
     // Split trees grow for many waves after phase A, so a batch is fed only once the previous one
     // has peaked: the live count is low and no longer rising (generations of primaries).
-    const bool decaying = live <= c->last_live;
-    c->last_live = live;
     if (live <= r.low_water && (decaying || live == 0)) {
-        // Hard limit: the phase-A output of every fed primary must fit.  Soft limit: the new batch's
-        // peak keeps the ring at most half full.
-        unsigned long long room_n = (r.ring_cap - live) / r.feed_bound;
-        const unsigned long long per_prim = c->per_prim ? c->per_prim : r.feed_bound;
-        const unsigned long long half = r.ring_cap / 2;
+        // soft limit: the new batch's peak keeps the ring at most half full
         const unsigned long long soft = live < half ? (half - live) / per_prim : 0;
-        if (soft < room_n) room_n = soft > 0 ? soft : (live == 0 ? 1 : 0);
-        long long n = c->prim_end - c->next_prim;
-        if (n > r.feed_batch) n = r.feed_batch;
-        // a batch never reaches into a room whose pilot has not run
-        if (c->pilot_room < r.n_rooms) {
-            const long long lim = __ldg(r.room_prim + c->pilot_room) - c->next_prim;
-            if (n > lim) n = lim;
-        }
-        if ((unsigned long long)n > room_n) n = (long long)room_n;
+        unsigned long long n = fit;
+        if (soft < n) n = soft > 0 ? soft : (live == 0 ? 1 : 0);
+        if (n > (unsigned long long)lim) n = (unsigned long long)lim;
         if (n > 0) {
-            c->pa_begin = c->next_prim;
-            c->pa_count = n;
-            c->next_prim += n;
+            c->pa_begin = next;
+            c->pa_count = (long long)n;
+            c->next_prim = next + (long long)n;
             c->pressure = 0;
         }
     }
 }
 
-__global__ void k_wave(DevRun r) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+__global__ void k_feed(DevRun r) { feed_step(r); }
+
+// Sizes the wave: as many ring items as leave room for their outputs.  One warp, after every append of
+// the phase-A batch (tail is read past L1: other blocks of this kernel have moved it).
+__device__ void size_wave(const DevRun &r) {
     WaveCtl *c = r.ctl;
+    const int lane = threadIdx.x & 31;
+    if (r.n_rooms > 1 && c->pilot_count > 0)
+        for (int i = c->pilot_first + lane; i < c->pilot_room; i += 32) {
+            const unsigned now = __ldcg(r.room_live + i);
+            if (now > r.room_peak[i]) r.room_peak[i] = now;
+        }
+    if (lane != 0) return;
     if (c->done) { c->m = 0; return; }
-    const unsigned long long live = c->tail - c->head;
+    const unsigned long long live = __ldcg(&c->tail) - c->head;
     if (live > c->peak_live) c->peak_live = live;
     if (c->pilot_count > 0 && live > c->pilot_peak) c->pilot_peak = live;
     // the batches outgrew their plan: plan the next ones with twice the footprint per primary
@@ -154,36 +231,39 @@ __global__ void k_wave(DevRun r) {
     if (live > 0 && m == 0) { ++c->overflow; c->done = 1; }  // ring full: cannot make progress
 }
 
-// Last node of a graph-mode iteration: decides whether the while loop runs again.  The loop ends
-// when the run is done, and also -- as a failure -- after max_iters iterations or 4096 consecutive
-// iterations that neither traced nor fed, so it always terminates.  Progress goes to mapped host
-// memory for the polling host thread.
+// Last node of a graph-mode iteration: decides whether the while loop runs again, and feeds the next
+// iteration.  The loop ends when the run is done, and also -- as a failure -- after max_iters
+// iterations or 4096 consecutive iterations that neither traced nor fed, so it always terminates.
+// Progress goes to mapped host memory for the polling host thread.
 __global__ void k_cond(DevRun r, cudaGraphConditionalHandle h) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
     WaveCtl *c = r.ctl;
-    ++c->iters;
-    if (c->m == 0 && c->pa_count == 0 && !c->done) ++c->idle;
-    else c->idle = 0;
-    bool stop = c->done != 0;
-    if (!stop && (c->iters >= r.max_iters || c->idle >= 4096)) {
-        c->gave_up = 1;
-        stop = true;
+    int stop = 0;
+    if (threadIdx.x == 0) {
+        ++c->iters;
+        if (c->m == 0 && c->pa_count == 0 && !c->done) ++c->idle;
+        else c->idle = 0;
+        stop = c->done != 0;
+        if (!stop && (c->iters >= r.max_iters || c->idle >= 4096)) {
+            c->gave_up = 1;
+            stop = 1;
+        }
+        if (!stop && r.cancel && *r.cancel >= 2) {  // abort: the host stops waiting for fed primaries
+            c->gave_up = 2;
+            stop = 1;
+        }
+        if (r.mirror) {
+            HostMirror *hm = r.mirror;
+            hm->next_prim = c->next_prim;
+            hm->iters = c->iters;
+            hm->segments = r.cnt->seg_broad + r.cnt->seg_b + r.cnt->seg_c;
+            hm->end_traces = r.cnt->end_traces;
+            hm->gave_up = c->gave_up;
+            hm->done = stop;
+        }
+        cudaGraphSetConditional(h, stop ? 0u : 1u);
     }
-    if (!stop && r.cancel && *r.cancel >= 2) {  // abort: the host stops waiting for fed primaries
-        c->gave_up = 2;
-        stop = true;
-    }
-    if (r.mirror) {
-        HostMirror *hm = r.mirror;
-        hm->next_prim = c->next_prim;
-        hm->iters = c->iters;
-        hm->segments = r.cnt->seg_broad + r.cnt->seg_b + r.cnt->seg_c;
-        hm->end_traces = r.cnt->end_traces;
-        hm->gave_up = c->gave_up;
-        __threadfence_system();
-        hm->done = stop ? 1 : 0;
-    }
-    cudaGraphSetConditional(h, stop ? 0u : 1u);
+    if (__shfl_sync(FULL, stop, 0)) return;
+    feed_step(r);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -193,16 +273,26 @@ __global__ void k_cond(DevRun r, cudaGraphConditionalHandle h) {
 template <bool MAP, bool SMALL>
 __global__ void __launch_bounds__(128) k_broadband(DevRun r) {
     extern __shared__ float4 s_rec_buf[];
+    __shared__ int s_last;
+    WaveCtl *c = r.ctl;
+    const long long p0 = c->pa_begin, cnt = c->pa_count;
+    // most iterations have nothing to emit: all blocks but one leave at once (13 us of empty blocks
+    // staging receivers and flushing counters before, 3 us of the same iteration's kernels now)
+    if (cnt == 0) {
+        if (blockIdx.x == 0 && threadIdx.x < 32) size_wave(r);
+        return;
+    }
+    const long long used = (cnt + blockDim.x - 1) / blockDim.x;  // blocks with work
+    if ((long long)blockIdx.x >= used) return;
     const int *s_rid;
     const float4 *s_rec = stage_receivers(r, s_rec_buf, s_rid);
     LocalCounters L;
     const DevScene &S = r.S;
-    WaveCtl *c = r.ctl;
-    const long long p0 = c->pa_begin, cnt = c->pa_count;
+    const bool count_room = r.n_rooms > 1 && c->pilot_count > 0;
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += stride) {
-        const long long prim = p0 + i;
-        const int room = room_of(r, prim);
+        int room;
+        const long long prim = scheduled_primary(r, p0 + i, room);
         const RoomParams &P = r.rooms[room];
         // SourceCluster round robin (Classes_Sources.cs:712-722)
         const int s = P.src_begin + (int)((prim + 1) % P.nsrc);
@@ -265,6 +355,7 @@ __global__ void __launch_bounds__(128) k_broadband(DevRun r) {
 #pragma unroll
             for (int o = 0; o < kBands; ++o) nchild += (E[o] != 0.f) ? (tau[o] > 0.f ? 3 : 1) : 0;
             unsigned long long slot = nchild ? atomicAdd(&c->tail, (unsigned long long)nchild) : 0ull;
+            if (count_room && nchild) atomicAdd(r.room_live + room, (unsigned)nchild);
 #pragma unroll
             for (int o = 0; o < kBands; ++o) {
                 if (E[o] == 0.f) continue;
@@ -298,6 +389,7 @@ __global__ void __launch_bounds__(128) k_broadband(DevRun r) {
         if (!lost) {
             const int nfin = P.oct_hi - P.oct_lo + 1;
             unsigned long long slot = atomicAdd(&c->tail, (unsigned long long)nfin);
+            if (count_room) atomicAdd(r.room_live + room, (unsigned)nfin);
 #pragma unroll
             for (int o = 0; o < kBands; ++o) {
                 if (o < P.oct_lo || o > P.oct_hi) continue;
@@ -309,6 +401,17 @@ __global__ void __launch_bounds__(128) k_broadband(DevRun r) {
         ++L.v[C_PRIM];
     }
     flush_counters(r, L);
+    // the last block with work sizes the wave
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        const unsigned n = (unsigned)(used < (long long)gridDim.x ? used : (long long)gridDim.x);
+        s_last = atomicAdd(&c->bb_blocks, 1u) == n - 1;
+        if (s_last) c->bb_blocks = 0;
+        __threadfence();
+    }
+    __syncthreads();
+    if (s_last && threadIdx.x < 32) size_wave(r);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -598,6 +701,7 @@ __global__ void __launch_bounds__(256, FUSED ? 2 : (WIDE ? 4 : kShadeMinBlocks))
     WaveCtl *c = r.ctl;
     const unsigned long long m = c->m, head = c->head;
     const unsigned long long m32 = (m + 31) & ~31ull;
+    const bool count_room = r.n_rooms > 1 && c->pilot_count > 0;
     const int lane = threadIdx.x & 31;
     const unsigned long long warp0 = ((unsigned long long)blockIdx.x * blockDim.x + threadIdx.x) & ~31ull;
     const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
@@ -691,6 +795,12 @@ __global__ void __launch_bounds__(256, FUSED ? 2 : (WIDE ? 4 : kShadeMinBlocks))
                 if (!alive && split) { R = C; split = false; alive = true; }
                 nout = (alive ? 1 : 0) + (split ? 1 : 0);
             }
+        }
+        if (count_room) {  // live count of each ray's room (pilots of a batch)
+            const int room = j < m ? (int)R.room : -1;
+            const unsigned peers = __match_any_sync(FULL, room);
+            const int d = __reduce_add_sync(peers, nout - 1);
+            if (room >= 0 && d != 0 && lane == __ffs(peers) - 1) atomicAdd(r.room_live + room, (unsigned)d);
         }
         const unsigned long long slot = warp_append(&c->tail, nout);
         if (nout >= 1) ring_store(r, slot, to_item(R));
@@ -808,11 +918,6 @@ cudaError_t launch_broadband(const DevRun &r, int blocks, int threads, cudaStrea
         if (small) k_broadband<false, true><<<blocks, threads, rec_smem(r), s>>>(r);
         else k_broadband<false, false><<<blocks, threads, rec_smem(r), s>>>(r);
     }
-    return cudaGetLastError();
-}
-
-cudaError_t launch_wave(const DevRun &r, cudaStream_t s) {
-    k_wave<<<1, 32, 0, s>>>(r);
     return cudaGetLastError();
 }
 

@@ -126,3 +126,24 @@ def test_scenes_built_together_equal_scenes_built_one_by_one():
     assert sa["segments"] == sb["segments"] and sa["accel"] == sb["accel"]
     for x, y in zip(ha, hb):
         np.testing.assert_allclose(x["energy"], y["energy"], rtol=1e-12, atol=1e-300)
+
+
+@pytest.mark.parametrize("rays,ring_log2,feed_batch", [([1, 255, 256, 257, 900], 0, 0), ([300, 40, 700, 256, 513], 19, 0),
+                                                       ([257, 600, 1, 300, 256], 0, 100)])
+def test_batch_feed_order_traces_every_primary_once(rays, ring_log2, feed_batch):
+    """Pilots first (several rooms at a time where the plan lets them), then the rest, with rooms below,
+    at and above a pilot's size, a ring that takes few pilots at once and feeds smaller than a pilot:
+    each room equals its single run (FP64 sums of the same terms in another order: 1e-9)."""
+    ws = [rooms.proposal_room_c4(10 + i) for i in range(len(rays))]
+    for w in ws:
+        w.cutoff_s = 0.4
+    ds = [tracer.DeviceScene(w.scene) for w in ws]
+    kw = dict(seed=4, ring_log2=ring_log2, feed_batch=feed_batch)
+    hb, sb = tracer.trace_batch(ws, dscenes=ds, rays=rays, **kw)
+    assert sb["primaries"] == sum(rays) and sb["queue_overflows"] == 0
+    off = 0
+    for i, w in enumerate(ws):
+        hs, _ = tracer.trace(w, dscene=ds[i], rays=rays[i], seed=4, ray_begin=off)
+        for name in ("energy", "pressure", "dir_pos", "dir_neg", "analysis"):
+            np.testing.assert_allclose(hb[i][name], hs[name], rtol=1e-9, atol=1e-30, err_msg=f"{i} {name}")
+        off += rays[i]
