@@ -18,9 +18,35 @@
 #include <tuple>
 #include <vector>
 
+#include <unistd.h>
+
 #include "engine.h"
 
 using namespace pach;
+
+void pach::touch_pages(const std::vector<std::pair<void *, size_t>> &ranges) {
+    const size_t page = (size_t)std::max(4096l, sysconf(_SC_PAGESIZE));
+    std::vector<std::pair<char *, size_t>> runs;  // first byte to write, pages
+    size_t total = 0;
+    for (const auto &r : ranges) {
+        if (!r.first || r.second < page) continue;  // too small to matter
+        runs.emplace_back(static_cast<char *>(r.first), (r.second + page - 1) / page);
+        total += runs.back().second;
+    }
+    auto touch = [&](size_t a, size_t b) {
+        size_t first = 0;
+        for (const auto &r : runs) {
+            for (size_t i = std::max(a, first); i < std::min(b, first + r.second); ++i)
+                *const_cast<volatile char *>(r.first + (i - first) * page) = 0;
+            first += r.second;
+        }
+    };
+    try {
+        parallel_chunks(total, std::max<size_t>(1, (size_t(2) << 20) / page), touch);
+    } catch (const std::exception &) {
+        // no thread to be had: the copy faults the pages in
+    }
+}
 
 namespace {
 
@@ -103,6 +129,9 @@ struct pach_run {
     bool conv_converged = false;
     std::vector<ConvCheck> conv_checks;
     DevMem conv, bak[6];
+    // scaled copies on their way to the host (one caller at a time)
+    DevMem stage;
+    std::mutex stage_mu;
     // worker
     std::thread worker;
     std::mutex mu;
@@ -123,7 +152,7 @@ struct pach_run {
         for (DevMem *m : {&hE, &hP, &hDp, &hDn, &hAn, &cnt, &qa, &qs0, &qs1, &qctl, &drec, &dsrc, &de0, &dgeo, &ddirs, &dw,
                           &sortbins, &dprop, &dcap, &droom, &dsched, &btri, &btri64, &bnorm, &bmat, &btrans, &bbvh, &bbvhq,
                           &mrec, &mdir, &mcell, &mentry, &mE, &mP, &mDp, &mDn, &drecid, &conv, &bak[0], &bak[1], &bak[2],
-                          &bak[3], &bak[4], &bak[5]})
+                          &bak[3], &bak[4], &bak[5], &stage})
             m->release();
     }
 };
@@ -149,6 +178,28 @@ long long room_done(const pach_run *run, int i, long long done) {
     const long long rays = run->rooms[(size_t)i].rays, pilot = std::min(rays, kPilotPrimaries);
     return std::max(0ll, std::min(pilot, done - before_p)) +
            std::max(0ll, std::min(rays - pilot, done - pilots - before_r));
+}
+
+// Copies n doubles to the host scaled by f, or by rows[i / per_row] (device): scaled on the device into
+// the run's staging buffer, or on the host when that cannot be had.
+cudaError_t download_scaled(pach_run *run, double *dst, const double *src, size_t n, double f,
+                            const std::vector<double> &rows, size_t per_row) {
+    std::lock_guard<std::mutex> lk(run->stage_mu);
+    const size_t need = (n + rows.size()) * sizeof(double);
+    if (run->stage.bytes < need && run->stage.alloc(need) != cudaSuccess) {
+        cudaGetLastError();
+        run->stage.bytes = 0;
+        const cudaError_t e = cudaMemcpy(dst, src, n * sizeof(double), cudaMemcpyDeviceToHost);
+        if (e == cudaSuccess)
+            for (size_t i = 0; i < n; ++i) dst[i] *= rows.empty() ? f : rows[i / per_row];
+        return e;
+    }
+    double *st = run->stage.as<double>(), *dr = rows.empty() ? nullptr : st + n;
+    cudaError_t e = cudaSuccess;
+    if (dr) e = cudaMemcpy(dr, rows.data(), rows.size() * sizeof(double), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = launch_scale(st, src, n, f, dr, per_row, nullptr);
+    if (e == cudaSuccess) e = cudaMemcpy(dst, st, n * sizeof(double), cudaMemcpyDeviceToHost);
+    return e;
 }
 
 cudaError_t upload(DevMem &m, const void *src, size_t bytes) {
@@ -1391,22 +1442,31 @@ pach_status pach_trace_get_histograms(pach_run *run, int32_t scaled, double *ene
                                {dir_pos, &run->hDp, nD, 3, false}, {dir_neg, &run->hDn, nD, 3, false},
                                {analysis, &run->hAn, nD, 3, false}};
         const long long done = run->rays_done.load();
+        // Receiver_Bank.Scale(N) then, for a cluster, Scale(1/n_sources) (TaskAll:770-771), with N the
+        // primaries the receiver's room completed: one factor for a run of one room, else one per receiver
+        std::vector<double> rows, prows;
+        double f = 1, fp = 1;
+        if (scaled)
+            for (size_t k = 0; k < run->rooms.size(); ++k) {
+                const RoomSpec &rm = run->rooms[k];
+                const double N = (double)std::max(1ll, room_done(run, (int)k, done)), ns = (double)rm.src.size();
+                f = ns / N;
+                fp = std::sqrt(ns) / std::sqrt(N);
+                if (run->rooms.size() == 1) break;
+                rows.insert(rows.end(), rm.rec.size(), f);
+                prows.insert(prows.end(), rm.rec.size(), fp);
+            }
+        std::vector<std::pair<void *, size_t>> dsts;
+        for (const Item &it : items)
+            if (it.dst && it.n) dsts.emplace_back(it.dst, it.n * sizeof(double));
+        touch_pages(dsts);
         for (const Item &it : items) {
             if (!it.dst || it.n == 0) continue;
-            cudaError_t e = cudaMemcpy(it.dst, it.src->p, it.n * sizeof(double), cudaMemcpyDeviceToHost);
+            const double *src = it.src->as<double>();
+            const cudaError_t e = scaled ? download_scaled(run, it.dst, src, it.n, it.pressure ? fp : f,
+                                                           it.pressure ? prows : rows, (size_t)it.lanes * kBands * run->T)
+                                         : cudaMemcpy(it.dst, src, it.n * sizeof(double), cudaMemcpyDeviceToHost);
             if (e != cudaSuccess) return fail(PACH_ERR_CUDA, cuda_msg(e, "histogram copy"));
-            if (!scaled) continue;
-            // Receiver_Bank.Scale(N) then, for a cluster, Scale(1/n_sources) (TaskAll:770-771), with N the
-            // primaries the receiver's room completed
-            const size_t per_rec = (size_t)it.lanes * kBands * run->T;
-            double *dst = it.dst;
-            for (const RoomSpec &rm : run->rooms) {
-                const double N = (double)std::max(1ll, room_done(run, (int)(&rm - run->rooms.data()), done));
-                const double ns = (double)rm.src.size();
-                const double f = it.pressure ? std::sqrt(ns) / std::sqrt(N) : ns / N;
-                for (size_t i = 0; i < rm.rec.size() * per_rec; ++i) dst[i] *= f;
-                dst += rm.rec.size() * per_rec;
-            }
         }
         return PACH_OK;
     }, fail);
@@ -1444,6 +1504,7 @@ pach_status pach_trace_get_filters(pach_run *run, int32_t directional, const dou
                                        run->hDn.as<double>(), dscale.as<double>(), run->R, run->T, kinds,
                                        run->p.sample_rate, swl, 4096, dout.as<double>(), ws.p, wsb, nullptr);
         if (s != PACH_OK) return s;
+        touch_pages({{out, n_out * sizeof(double)}});  // while the kernels run
         if ((e = cudaMemcpy(out, dout.p, n_out * sizeof(double), cudaMemcpyDeviceToHost)) != cudaSuccess)
             return fail(PACH_ERR_CUDA, cuda_msg(e, "filters"));
         return PACH_OK;
@@ -1491,12 +1552,12 @@ pach_status pach_trace_get_map(pach_run *run, int32_t scaled, double *energy, do
         const double N = (double)std::max(1ll, run->rays_done.load());
         const double f = (double)run->nsrc / N;
         const double fp = g.directional ? std::sqrt((double)run->nsrc / N) : f;
+        touch_pages({{energy, n * sizeof(double)}, {pressure, n * sizeof(double)}});
         for (auto [dst, src, k] : {std::tuple<double *, DevMem *, double>{energy, &run->mE, f}, {pressure, &run->mP, fp}}) {
             if (!dst) continue;
-            cudaError_t e = cudaMemcpy(dst, src->p, n * sizeof(double), cudaMemcpyDeviceToHost);
+            const cudaError_t e = scaled ? download_scaled(run, dst, src->as<double>(), n, k, {}, 1)
+                                         : cudaMemcpy(dst, src->p, n * sizeof(double), cudaMemcpyDeviceToHost);
             if (e != cudaSuccess) return fail(PACH_ERR_CUDA, cuda_msg(e, "map copy"));
-            if (scaled)
-                for (size_t i = 0; i < n; ++i) dst[i] *= k;
         }
         return PACH_OK;
     }, fail);
@@ -1517,12 +1578,12 @@ pach_status pach_trace_get_map_directions(pach_run *run, int32_t scaled, double 
         if (cap_bins < n) return fail(PACH_ERR_INVALID_ARGUMENT, "cap_bins < map receivers * 3 * 8 * bins");
         cudaSetDevice(run->scene->device);
         const double f = (double)run->nsrc / (double)std::max(1ll, run->rays_done.load());
+        touch_pages({{dir_pos, n * sizeof(double)}, {dir_neg, n * sizeof(double)}});
         for (auto [dst, src] : {std::pair<double *, DevMem *>{dir_pos, &run->mDp}, {dir_neg, &run->mDn}}) {
             if (!dst) continue;
-            cudaError_t e = cudaMemcpy(dst, src->p, n * sizeof(double), cudaMemcpyDeviceToHost);
+            const cudaError_t e = scaled ? download_scaled(run, dst, src->as<double>(), n, f, {}, 1)
+                                         : cudaMemcpy(dst, src->p, n * sizeof(double), cudaMemcpyDeviceToHost);
             if (e != cudaSuccess) return fail(PACH_ERR_CUDA, cuda_msg(e, "map direction copy"));
-            if (scaled)
-                for (size_t i = 0; i < n; ++i) dst[i] *= f;
         }
         return PACH_OK;
     }, fail);

@@ -76,6 +76,11 @@ void parallel_chunks(size_t n, size_t grain, F &&f) {
     for (auto &p : parts) p.get();
 }
 
+// Writes one byte of every page of the given host ranges, on several threads when there are many: memory
+// that the caller has just allocated gets its pages here.  Left to the copy they are faulted in by the
+// GPU one after another, 55 us each (34 MB of fresh histogram arrays: 30 ms, against 3 ms touched).
+void touch_pages(const std::vector<std::pair<void *, size_t>> &ranges);
+
 // Host-side prepared scene (FP64 master copy + FP32 device layout sources).
 struct HostScene {
     int npoly = 0, ntri = 0;
@@ -375,6 +380,9 @@ cudaError_t launch_shade(const DevRun &r, int blocks, int threads, cudaStream_t 
 cudaError_t launch_map_params(const double *etc, int n, int T, double fs, double scale, int decay_depth,
                               double clarity_s, double *t_x, double *edt, double *clarity, double *definition,
                               double *sum, cudaStream_t s);
+// dst = src x f, or x rows[i / per_row] when rows is not null, for n doubles (trace.cu)
+cudaError_t launch_scale(double *dst, const double *src, size_t n, double f, const double *rows, size_t per_row,
+                         cudaStream_t s);
 constexpr int kFuseMaxTris = 64;
 inline bool fused_walk(int traversal, int ntri) { return traversal == 3 || (traversal == 0 && ntri <= kFuseMaxTris); }
 cudaError_t wave_kernel_occupancy(int variant, int threads, int smem_shade, int *bpsm_trace, int *bpsm_shade,

@@ -506,6 +506,7 @@ pach_status filters_host(const double *E, const double *P, const double *Dp, con
         cudaStreamSynchronize(st);
         return s;
     }
+    touch_pages({{out, n_out * sizeof(double)}});  // while the kernels run
     if ((e = cudaMemcpyAsync(out, bOut.p, n_out * sizeof(double), cudaMemcpyDeviceToHost, st)) != cudaSuccess)
         return cuda_fail(e, "filter copy");
     if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return cuda_fail(e, "filter kernels");

@@ -128,7 +128,7 @@ def test_scenes_built_together_equal_scenes_built_one_by_one():
         np.testing.assert_allclose(x["energy"], y["energy"], rtol=1e-12, atol=1e-300)
 
 
-@pytest.mark.parametrize("rays,ring_log2,feed_batch", [([1, 255, 256, 257, 900], 0, 0), ([300, 40, 700, 256, 513], 19, 0),
+@pytest.mark.parametrize("rays,ring_log2,feed_batch", [([1, 255, 256, 257, 900], 0, 0), ([300, 40, 700, 256, 513], 20, 0),
                                                        ([257, 600, 1, 300, 256], 0, 100)])
 def test_batch_feed_order_traces_every_primary_once(rays, ring_log2, feed_batch):
     """Pilots first (several rooms at a time where the plan lets them), then the rest, with rooms below,
