@@ -55,6 +55,22 @@ def test_loss_and_gradient_match_oracle():
             assert err < 2e-2, (l, what, err)
 
 
+@pytest.mark.parametrize("rows", [1, 128, 129, 513, 1300])
+def test_gradient_at_tile_and_range_edges(rows):
+    """Row tiles of 128 and row ranges of the weight gradients (one range below 512 rows, two at 513, five at
+    1300): the oracle comparison of test_loss_and_gradient_match_oracle with its tolerances."""
+    net = proposal.ProposalNet(seed=5, max_rows=rows)
+    cond, target = _problem(rows, seed=rows)
+    net.set_data(cond, target)
+    loss, g = net.loss_grad()
+    bins = proposal.direction_bins()[0].astype(np.float64)
+    ref_loss, ref_g = MO.loss_grad(net.params().astype(np.float64), cond, target, bins, emulate_bf16=True)
+    assert loss == pytest.approx(ref_loss, rel=2e-3)
+    assert np.linalg.norm(g - ref_g) / np.linalg.norm(ref_g) < 2e-2
+    loss2, g2 = net.loss_grad()  # a second pass starts from cleared sums
+    assert loss2 == loss and np.linalg.norm(g2 - g) <= 1e-5 * np.linalg.norm(g)
+
+
 def test_training_reduces_loss_and_forward_is_consistent():
     net = proposal.ProposalNet(seed=3, max_rows=512)
     rng = np.random.default_rng(9)
