@@ -1602,25 +1602,27 @@ pach_status pach_map_parameters(pach_run *run, int32_t decay_depth, int32_t clar
         const MapGrid &g = run->mg;
         const int n = g.M * kBands;
         cudaSetDevice(run->scene->device);
-        DevMem out;
-        struct Release {
-            DevMem &m;
-            ~Release() { m.release(); }
-        } release_out{out};
-        cudaError_t e = out.alloc((size_t)5 * n * sizeof(double));
-        if (e != cudaSuccess) return fail(PACH_ERR_OUT_OF_MEMORY, cuda_msg(e, "parameter map buffers"));
-        double *d = out.as<double>();
+        std::lock_guard<std::mutex> lk(run->stage_mu);
+        const size_t bytes = (size_t)5 * n * sizeof(double);
+        cudaError_t e = cudaSuccess;
+        if (run->stage.bytes < bytes) {
+            e = run->stage.alloc(bytes);
+            if (e != cudaSuccess) {
+                run->stage.bytes = 0;
+                return fail(PACH_ERR_OUT_OF_MEMORY, cuda_msg(e, "parameter map buffers"));
+            }
+        }
+        double *d = run->stage.as<double>();
         const double scale = (double)run->nsrc / (double)std::max(1ll, run->rays_done.load());
         e = launch_map_params(run->mE.as<double>(), n, g.T, 1000.0, scale, decay_depth, clarity_ms / 1000.0, d, d + n,
                               d + 2 * (size_t)n, d + 3 * (size_t)n, d + 4 * (size_t)n, nullptr);
-        if (e == cudaSuccess) e = cudaDeviceSynchronize();
         if (e != cudaSuccess) return fail(PACH_ERR_CUDA, cuda_msg(e, "parameter map kernel"));
+        hvec<double> host((size_t)5 * n);  // the five maps in one copy
+        e = cudaMemcpy(host.data(), d, bytes, cudaMemcpyDeviceToHost);
+        if (e != cudaSuccess) return fail(PACH_ERR_CUDA, cuda_msg(e, "parameter map copy"));
         double *dst[5] = {t_x, edt, clarity, definition, energy_sum};
-        for (int i = 0; i < 5; ++i) {
-            if (!dst[i]) continue;
-            e = cudaMemcpy(dst[i], d + (size_t)i * n, (size_t)n * sizeof(double), cudaMemcpyDeviceToHost);
-            if (e != cudaSuccess) return fail(PACH_ERR_CUDA, cuda_msg(e, "parameter map copy"));
-        }
+        for (int i = 0; i < 5; ++i)
+            if (dst[i]) std::memcpy(dst[i], host.data() + (size_t)i * n, (size_t)n * sizeof(double));
         return PACH_OK;
     }, fail);
 }

@@ -16,7 +16,7 @@ import numpy as np
 import pytest
 
 from oracle import oracle as O
-from pachydermacoustic_universal_gb300 import rooms, tracer
+from pachydermacoustic_universal_gb300 import _capi, rooms, tracer
 from pachydermacoustic_universal_gb300.simulation import AcousticalMath
 
 pytestmark = pytest.mark.gpu
@@ -146,6 +146,34 @@ def test_parameter_kernel_matches_host_math():
                        pg["energy"][i, o])
                 np.testing.assert_allclose(got, ref, rtol=1e-9, equal_nan=True)
     run.close()
+
+
+@pytest.mark.parametrize("T,depth,cms", [(1, 30, 80), (2, 30, 80), (33, 15, 10), (95, 30, 50), (1024, 20, 80), (3001, 30, 80),
+                                         (6000, 60, 500), (6001, 30, 80)])
+def test_parameter_kernel_over_curve_lengths_and_kinds(T, depth, cms):
+    """Curves in shared memory (up to 6000 bins) and streamed ones, against AcousticalMath: smooth and sparse
+    decays, one impulse, a plateau between two, an early and a late start, no energy, a negative bin.  FP64 sums
+    of T terms are good to about T x 1e-16 and the slopes lose at most three digits of that: 1e-9."""
+    rng = np.random.default_rng(T)
+    t = np.arange(T)
+    curves = [np.exp(-t / (0.02 * T + 1)), np.exp(-t / (0.2 * T + 1)) * rng.gamma(0.5, 1.0, T),
+              np.where(rng.random(T) < 0.05, np.exp(-t / (0.1 * T + 1)), 0.0), np.where(t == T // 2, 1.0, 0.0),
+              np.where(t == 0, 1.0, 0.0) + np.where(t == T - 1, 0.01, 0.0), np.where(t < T // 3, 1e-3, 0.0),
+              np.where(t >= T // 3, np.exp(-t / (0.05 * T + 1)), 0.0), np.zeros(T),
+              np.exp(-t / (0.1 * T + 1)) - np.where(t == T // 4, 0.5, 0.0)]
+    etc = np.ascontiguousarray(curves) * 1e-5
+    n = len(curves)
+    out = {k: np.zeros(n) for k in ("t_x", "edt", "clarity", "definition", "energy")}
+    L = _capi.lib()
+    _capi.check(L.pach_etc_parameters(_capi.dptr(etc), n, T, 1000, depth, cms / 1000.0, *(_capi.dptr(v) for v in out.values())))
+    with np.errstate(all="ignore"):
+        for i in range(n):
+            sch = AcousticalMath.Schroeder_Integral(etc[i])
+            ref = {"t_x": AcousticalMath.T_X(sch, depth, 1000), "edt": AcousticalMath.EarlyDecayTime(sch, 1000),
+                   "clarity": AcousticalMath.Clarity(etc[i], 1000, cms / 1000.0, 0.0, False),
+                   "definition": AcousticalMath.Definition(etc[i], 1000, 0.05, 0.0, False), "energy": etc[i].sum()}
+            for k, v in ref.items():
+                np.testing.assert_allclose(out[k][i], v, rtol=1e-9, atol=1e-300, equal_nan=True, err_msg=f"{k} {i}")
 
 
 def test_one_point_map_matches_oracle():
