@@ -35,6 +35,34 @@ def test_etc_to_filter_matches_oracle(T, fs):
     _close(tracer.etc_to_filter(P, swl, fs), F.etc_to_filter(P, swl, fs))
 
 
+@pytest.mark.parametrize("T", [2, 255, 4095, 4096, 4097, 8193, 16384, 49153, 49154])
+@pytest.mark.parametrize("fs", [1000, 44100])
+def test_integer_transforms_over_lengths(T, fs):
+    """The integer transforms' classes (T + 16383 points up to 16384, 32768, 65536; folds of 4096 samples) and the
+    first length of the FP64 transforms, with an envelope that falls over 200 dB, a silent band and one outlier.
+    Inputs are rounded at 2^-60 of their largest value, so only numpy's transforms round: 1e-14 of the peak."""
+    rng = np.random.default_rng(T)
+    P = rng.random((8, T)) * 10.0 ** (-10.0 * np.arange(T) / T)
+    P[3] = 0.0
+    P[5, T // 2] += 40.0
+    swl = rng.uniform(80, 130, 8)
+    got, ref = tracer.etc_to_filter(P, swl, fs), F.etc_to_filter(P, swl, fs)
+    assert np.abs(got - ref).max() <= 1e-14 * np.abs(ref).max()
+
+
+def test_silent_and_undefined_envelopes():
+    """A filter of silence is zero; a value that is not finite makes its whole filter undefined (as every
+    output of a transform of it is), and no other filter of the call."""
+    P = np.random.default_rng(3).random((4, 8, 600))
+    P[1] = 0.0
+    P[2, 4, 100] = np.inf
+    P[3, 7, 5] = np.nan
+    got = tracer.etc_to_filter(P, None, 1000)
+    _close(got[0], F.etc_to_filter(P[0], [120] * 8, 1000))
+    assert not got[1].any()
+    assert np.isnan(got[2]).all() and np.isnan(got[3]).all()
+
+
 def test_etc_to_filter_batch_and_default_level():
     rng = np.random.default_rng(9)
     P = rng.random((5, 8, 700))
