@@ -83,14 +83,15 @@ struct pach_scene {
     int device = 0;
     HostScene hs;
     DevScene dev{};
-    DevMem tri, tri64, norm, mat, trans, bvh, bvhq;
+    DevMem tri, tri64, norm, mat, trans, bvh, bvhq, plane;
+    int n_planes = 0;  // of the device copy
     // the device copy above exists (pach_scene_create makes it at once; pach_scenes_create leaves it to the
     // first single-room use, since a batch run uploads the concatenation of its rooms instead)
     bool on_device = false;
     std::mutex mu;  // guards the first upload
     ~pach_scene() {
         cudaSetDevice(device);
-        for (DevMem *m : {&tri, &tri64, &norm, &mat, &trans, &bvh, &bvhq}) m->release();
+        for (DevMem *m : {&tri, &tri64, &norm, &mat, &trans, &bvh, &bvhq, &plane}) m->release();
     }
 };
 
@@ -115,7 +116,7 @@ struct pach_run {
     int R = 0, T = 0, nsrc = 0;   // receivers and sources over all rooms
     // device buffers
     DevMem hE, hP, hDp, hDn, hAn, cnt, qa, qs0, qs1, qctl, drec, dsrc, de0, dgeo, ddirs, dw, sortbins, dprop, dcap;
-    DevMem droom, dsched, btri, btri64, bnorm, bmat, btrans, bbvh, bbvhq;
+    DevMem droom, dsched, btri, btri64, bnorm, bmat, btrans, bbvh, bbvhq, bplane;
     // mapping receivers (has_map): the host grid and its device copy, histograms [M][8][Tm]
     bool has_map = false;
     MapGrid mg;
@@ -150,7 +151,7 @@ struct pach_run {
         }
         cudaSetDevice(scene ? scene->device : 0);
         for (DevMem *m : {&hE, &hP, &hDp, &hDn, &hAn, &cnt, &qa, &qs0, &qs1, &qctl, &drec, &dsrc, &de0, &dgeo, &ddirs, &dw,
-                          &sortbins, &dprop, &dcap, &droom, &dsched, &btri, &btri64, &bnorm, &bmat, &btrans, &bbvh, &bbvhq,
+                          &sortbins, &dprop, &dcap, &droom, &dsched, &btri, &btri64, &bnorm, &bmat, &btrans, &bbvh, &bbvhq, &bplane,
                           &mrec, &mdir, &mcell, &mentry, &mE, &mP, &mDp, &mDn, &drecid, &conv, &bak[0], &bak[1], &bak[2],
                           &bak[3], &bak[4], &bak[5], &stage})
             m->release();
@@ -215,6 +216,8 @@ struct SceneArrays {
     hvec<float4> tri, norm, mat;
     hvec<float> trans, bvh, bvhq;
     hvec<double> tri64;
+    std::vector<float4> plane;   // two per plane (DevScene::plane)
+    std::vector<int> plane_tri;
     int planes = 0;
     float t_eps = 0.f;
     bool has_trans = false;
@@ -257,7 +260,57 @@ static void rebase_qnodes(float *nodes, size_t count, int node_off, int tri_off)
     });
 }
 
-int append_scene(const HostScene &hs, SceneArrays &A) {
+// Appends the scene's planes (see kMaxPlanes); returns how many, 0 when the scene does not qualify.
+int append_planes(const HostScene &hs, SceneArrays &A, int tri_off, int plane_off) {
+    if (hs.ntri > kFuseMaxTris) return 0;
+    struct Rec {
+        double n[3], d;
+        int id;
+        std::vector<int> tri;
+    };
+    std::vector<Rec> recs;
+    const double near = 1e-6 * hs.scale;
+    for (int i = 0; i < hs.ntri; ++i) {
+        const double *t = &hs.tri64[9 * (size_t)i];
+        const double nx = t[4] * t[8] - t[5] * t[7], ny = t[5] * t[6] - t[3] * t[8], nz = t[3] * t[7] - t[4] * t[6];
+        const double area = std::sqrt(nx * nx + ny * ny + nz * nz);
+        const double a = std::sqrt(t[3] * t[3] + t[4] * t[4] + t[5] * t[5]), b = std::sqrt(t[6] * t[6] + t[7] * t[7] + t[8] * t[8]);
+        if (!(area > 0.05 * a * b)) return 0;
+        Rec *to = nullptr;
+        for (Rec &q : recs) {
+            if (q.id != hs.tri_plane[(size_t)i]) continue;
+            double far = 0;
+            for (int k = 0; k < 3; ++k) {
+                const double v[3] = {t[0] + (k == 1 ? t[3] : k == 2 ? t[6] : 0), t[1] + (k == 1 ? t[4] : k == 2 ? t[7] : 0),
+                                     t[2] + (k == 1 ? t[5] : k == 2 ? t[8] : 0)};
+                far = std::max(far, std::fabs(q.n[0] * v[0] + q.n[1] * v[1] + q.n[2] * v[2] + q.d));
+            }
+            if (far <= near) { to = &q; break; }
+        }
+        if (!to) {
+            if ((int)recs.size() == kMaxPlanes) return 0;
+            recs.push_back(Rec());
+            to = &recs.back();
+            to->n[0] = nx / area; to->n[1] = ny / area; to->n[2] = nz / area;
+            to->d = -(to->n[0] * t[0] + to->n[1] * t[1] + to->n[2] * t[2]);
+            to->id = hs.tri_plane[(size_t)i];
+        }
+        to->tri.push_back(i);
+    }
+    auto bits = [](int v) {
+        float f;
+        std::memcpy(&f, &v, 4);
+        return f;
+    };
+    for (const Rec &q : recs) {
+        A.plane.push_back(make_float4((float)q.n[0], (float)q.n[1], (float)q.n[2], (float)q.d));
+        A.plane.push_back(make_float4(bits((int)A.plane_tri.size()), bits((int)q.tri.size()), bits(q.id + plane_off), 0.f));
+        for (int i : q.tri) A.plane_tri.push_back(i + tri_off);
+    }
+    return (int)recs.size();
+}
+
+int append_scene(const HostScene &hs, SceneArrays &A, int *n_planes = nullptr) {
     const int tri_off = (int)(A.tri.size() / 3), poly_off = (int)A.norm.size(), plane_off = A.planes;
     const int node_off = (int)(A.bvh.size() / kBvhNodeFloats);
     const size_t t0 = A.tri.size(), d0 = A.tri64.size(), n0 = A.norm.size(), m0 = A.mat.size();
@@ -290,6 +343,8 @@ int append_scene(const HostScene &hs, SceneArrays &A) {
     int max_plane = -1;
     for (int m : chunk_plane) max_plane = std::max(max_plane, m);
     A.planes = plane_off + max_plane + 1;
+    const int np = append_planes(hs, A, tri_off, plane_off);
+    if (n_planes) *n_planes = np;
     parallel_chunks((size_t)hs.npoly, 16384, [&](size_t p0, size_t p1) {
         for (size_t p = p0; p < p1; ++p) {
             A.norm[n0 + p] = make_float4((float)hs.normal[3 * p], (float)hs.normal[3 * p + 1], (float)hs.normal[3 * p + 2], 0.f);
@@ -322,8 +377,16 @@ int append_scene(const HostScene &hs, SceneArrays &A) {
 }
 
 cudaError_t upload_scene(const SceneArrays &A, DevMem &tri, DevMem &tri64, DevMem &norm, DevMem &mat, DevMem &trans,
-                         DevMem &bvh, DevMem &bvhq, DevScene &d) {
+                         DevMem &bvh, DevMem &bvhq, DevMem &plane, DevScene &d) {
     cudaError_t e;
+    // the planes and their triangle list in one buffer
+    const size_t pb = A.plane.size() * sizeof(float4), tb = A.plane_tri.size() * sizeof(int);
+    std::vector<char> pl(pb + tb);
+    if (pb) std::memcpy(pl.data(), A.plane.data(), pb);
+    if (tb) std::memcpy(pl.data() + pb, A.plane_tri.data(), tb);
+    if ((e = upload(plane, pl.data(), pl.size())) != cudaSuccess) return e;
+    d.plane = plane.as<float4>();
+    d.plane_tri = reinterpret_cast<const int *>(plane.as<char>() + pb);
     if ((e = upload(tri, A.tri.data(), A.tri.size() * sizeof(float4))) ||
         (e = upload(tri64, A.tri64.data(), A.tri64.size() * sizeof(double))) ||
         (e = upload(norm, A.norm.data(), A.norm.size() * sizeof(float4))) ||
@@ -351,8 +414,9 @@ cudaError_t scene_upload(pach_scene *sc) {
     std::lock_guard<std::mutex> lk(sc->mu);
     if (sc->on_device) return cudaSuccess;
     SceneArrays A;
-    append_scene(sc->hs, A);
-    const cudaError_t e = upload_scene(A, sc->tri, sc->tri64, sc->norm, sc->mat, sc->trans, sc->bvh, sc->bvhq, sc->dev);
+    append_scene(sc->hs, A, &sc->n_planes);
+    const cudaError_t e = upload_scene(A, sc->tri, sc->tri64, sc->norm, sc->mat, sc->trans, sc->bvh, sc->bvhq, sc->plane,
+                                       sc->dev);
     if (e == cudaSuccess) sc->on_device = true;
     return e;
 }
@@ -465,11 +529,15 @@ void run_worker_body(pach_run *run) {
         // scene: the first room's own device arrays, or the concatenation of every room's
         if (n_rooms == 1) TRY(scene_upload(sc));
         DevScene S = sc->dev;
-        std::vector<int> roots(n_rooms, 0);
+        std::vector<int> roots(n_rooms, 0), planes(n_rooms, sc->n_planes), plane_begin(n_rooms, 0);
         if (n_rooms > 1) {
             SceneArrays A;
-            for (int i = 0; i < n_rooms; ++i) roots[i] = append_scene(run->rooms[i].scene->hs, A);
-            TRY(upload_scene(A, run->btri, run->btri64, run->bnorm, run->bmat, run->btrans, run->bbvh, run->bbvhq, S));
+            for (int i = 0; i < n_rooms; ++i) {
+                plane_begin[i] = (int)(A.plane.size() / 2);
+                roots[i] = append_scene(run->rooms[i].scene->hs, A, &planes[i]);
+            }
+            TRY(upload_scene(A, run->btri, run->btri64, run->bnorm, run->bmat, run->btrans, run->bbvh, run->bbvhq,
+                             run->bplane, S));
         }
         // receivers, sources, powers and room table over all rooms
         std::vector<float4> rec(std::max(R, 1)), src;
@@ -495,6 +563,8 @@ void run_worker_body(pach_run *run) {
             P.rho_c = (float)hs.rho_c;
             for (int o = 0; o < kBands; ++o) P.atten_k[o] = (float)(-0.1 * std::log2(10.0) * hs.atten[o] * hs.c);
             P.bvh_root = roots[i];
+            P.plane_begin = plane_begin[i];
+            P.n_planes = planes[i];
             P.t_eps = (float)(2e-7 * hs.scale);
             P.rec_begin = k;
             P.R = (int)rm.rec.size();
@@ -612,6 +682,9 @@ void run_worker_body(pach_run *run) {
         for (const RoomSpec &rm : run->rooms) rec_max = std::max(rec_max, rm.rec.size());
         const bool wide = rec_max >= (size_t)kShadeWideReceivers;
         TRY(wave_kernel_occupancy(tr_variant, threads, receiver_smem_bytes(R), &bps_tr, &bps_sh, fused, wide));
+        const bool bounce = fused && !map;
+        const bool by_planes = bounce && *std::min_element(planes.begin(), planes.end()) > 0;
+        if (bounce) TRY(bounce_occupancy(threads, receiver_smem_bytes(R), &bps_sh, by_planes));
         const int tr_blocks = dev_sms * std::max(bps_tr, 1), sh_blocks = dev_sms * std::max(bps_sh, 1);
 
         // ring and wave sizing
@@ -732,6 +805,7 @@ void run_worker_body(pach_run *run) {
             r.sort_inv[k] = (float)(kSortGrid / std::max(bmax[k] - bmin[k], 1e-9));
         }
         r.max_wave = std::min(max_wave, ring_cap);
+        r.max_bounces = bounce ? kMaxBounces : 1;
         r.feed_bound = bound;
         r.low_water = std::min(ring_cap / 4, 2 * r.max_wave);
         const long long N = rprim[n_rooms] - rprim[0];
@@ -770,7 +844,9 @@ void run_worker_body(pach_run *run) {
             if (timing && (x = cudaEventRecord(kev[6 * k + 3], stream))) return x;
             if (!fused && (x = launch_trace(r, tr_variant, tr_blocks, threads, stream))) return x;
             if (timing && (x = cudaEventRecord(kev[6 * k + 4], stream))) return x;
-            if ((x = launch_shade(r, sh_blocks, threads, stream, fused, map, wide))) return x;
+            if ((x = bounce ? launch_bounce(r, sh_blocks, threads, stream, by_planes)
+                            : launch_shade(r, sh_blocks, threads, stream, fused, map, wide)))
+                return x;
             if (timing && (x = cudaEventRecord(kev[6 * k + 5], stream))) return x;
             return cudaSuccess;
         };
@@ -1055,7 +1131,7 @@ void run_worker_body(pach_run *run) {
     if (h_cancel) cudaFreeHost(h_cancel);
     // release the ring and the batch scene; histograms and counters stay until the run is destroyed
     for (DevMem *m : {&run->qa, &run->qs0, &run->qs1, &run->ddirs, &run->dw, &run->sortbins, &run->btri, &run->btri64,
-                      &run->bnorm, &run->bmat, &run->btrans, &run->bbvh, &run->bbvhq, &run->conv, &run->bak[0],
+                      &run->bnorm, &run->bmat, &run->btrans, &run->bbvh, &run->bbvhq, &run->bplane, &run->conv, &run->bak[0],
                       &run->bak[1], &run->bak[2], &run->bak[3], &run->bak[4], &run->bak[5]})
         m->release();
     if (e != cudaSuccess) return finish(PACH_ERR_CUDA, cuda_msg(e, where.c_str()), PACH_RUN_FAILED);
@@ -1851,6 +1927,7 @@ pach_status pach_proposal_sample(const float *proposal, int32_t n_prop, double m
 namespace pach {
 const HostScene *scene_host(const pach_scene *s) { return s ? &s->hs : nullptr; }
 const DevScene *scene_dev(const pach_scene *s) { return s && s->on_device ? &s->dev : nullptr; }
+int scene_planes(const pach_scene *s) { return s && s->on_device ? s->n_planes : 0; }
 int scene_device(const pach_scene *s) { return s ? s->device : -1; }
 void set_last_error(const char *msg) { g_err = msg; }
 }  // namespace pach

@@ -145,6 +145,40 @@ __device__ __forceinline__ void test_tri(const DevScene &S, float t_eps, int i, 
     }
 }
 
+// test_tri that also notes a tie: an accepted candidate at exactly the best distance, where the first one
+// tested wins.  A walk in another order than the BVH's then has to ask the BVH.
+__device__ __forceinline__ void test_tri_tie(const DevScene &S, float t_eps, int i, float3 o, float3 d, int skip,
+                                             float &best, int &bi, TraceWork &w, bool &tie) {
+    const float4 A = __ldg(S.tri + 3 * i);
+    if (__float_as_int(A.w) == skip) return;
+    const float4 B = __ldg(S.tri + 3 * i + 1);
+    const float4 C = __ldg(S.tri + 3 * i + 2);
+    const float3 e1 = f3(B), e2 = f3(C);
+    const float3 p = cross3(d, e2);
+    const float det = dot3(e1, p);
+    const float3 s = o - f3(A);
+    const float inv = 1.0f / det;
+    const float u = dot3(s, p) * inv;
+    const float3 q = cross3(s, e1);
+    const float v = dot3(d, q) * inv;
+    float t = dot3(e2, q) * inv;
+    const float margin = fminf(fminf(u, v), 1.0f - u - v);
+    const bool grazing = fabsf(det) < C.w;
+    if (grazing || !(fabsf(margin) > kBaryEps)) {
+        if (!grazing && isfinite(t) && (t < 0.5f * t_eps || t > 1.0001f * best)) return;
+        double td;
+        ++w.retests;
+        if (!retest64(S, i, o, d, td)) return;
+        t = (float)td;
+    } else if (!(margin > 0.f)) {
+        return;
+    }
+    if (t > t_eps) {
+        tie = tie || t == best;
+        if (t < best) { best = t; bi = i; }
+    }
+}
+
 // Empty child slot of a 4-wide node (no leaf can have this code below 2^27 triangles).
 constexpr int kEmptyChild = (int)0x80000000;
 
@@ -333,6 +367,59 @@ __device__ __forceinline__ bool trace_ray(const DevScene &S, int root, float t_e
             node = stack[--sp];
         }
     }
+    if (bi < 0) return false;
+    t_best = best;
+    tri_best = bi;
+    return true;
+}
+
+// The plain walk, out of line: the rare second opinion of plane_walk.
+__device__ __noinline__ bool trace_ray_again(const DevScene &S, int root, float t_eps, float3 o, float3 d, int skip,
+                                             float &t_best, int &tri_best, TraceWork &w) {
+    return trace_ray<int>(S, root, t_eps, o, d, skip, t_best, tri_best, w);
+}
+
+// Nearest hit in a scene of at most kMaxPlanes planes (see PlaneSet in engine.h): the distances to the planes
+// first, then the triangles of the nearest ones, nearest plane first, until the next plane begins beyond the hit.
+// A plane begins at its distance less a margin, kPlaneMargin t_eps / |n d| (1e-5 of the room's extent along the
+// normal: the planes' and distances' rounding is at most a tenth of it); a nearly parallel plane counts as near.
+// So every triangle that the BVH could find nearer has been tested, with the same test; ties go to the BVH.  In a
+// convex room a ray tests the two triangles of one plane, without a branch but near edges: about 260
+// instructions where the two-level BVH walk takes 600.
+constexpr float kPlaneMargin = 50.f;  // x t_eps (2e-7 of the extent)
+__device__ __forceinline__ bool plane_walk(const DevScene &S, const float4 *planes, int n, int root, float t_eps, float3 o,
+                                           float3 d, int skip, float &t_best, int &tri_best, TraceWork &w) {
+    float tl[kMaxPlanes];
+#pragma unroll
+    for (int k = 0; k < kMaxPlanes; ++k) {
+        tl[k] = INFINITY;
+        if (k >= n) continue;
+        const float4 N = planes[2 * k];
+        const float nd = fmaf(N.x, d.x, fmaf(N.y, d.y, N.z * d.z));
+        const float no = fmaf(N.x, o.x, fmaf(N.y, o.y, fmaf(N.z, o.z, N.w)));
+        const float inv = __fdividef(1.0f, nd);
+        const float t = -no * inv, e = kPlaneMargin * t_eps * fabsf(inv);
+        const bool parallel = fabsf(nd) < 3e-4f;
+        if ((parallel || t + e > 0.f) && __float_as_int(planes[2 * k + 1].z) != skip) tl[k] = parallel ? -1.f : t - e;
+    }
+    float best = FLT_MAX;
+    int bi = -1;
+    bool tie = false;
+    for (;;) {
+        float m = INFINITY;
+        int i = -1;
+#pragma unroll
+        for (int k = 0; k < kMaxPlanes; ++k)
+            if (tl[k] < m) { m = tl[k]; i = k; }
+        if (!(m <= best)) break;
+        const float4 rec = planes[2 * i + 1];
+        const int f0 = __float_as_int(rec.x), cnt = __float_as_int(rec.y);
+        for (int j = 0; j < cnt; ++j)
+            test_tri_tie(S, t_eps, __ldg(S.plane_tri + f0 + j), o, d, skip, best, bi, w, tie);
+#pragma unroll
+        for (int k = 0; k < kMaxPlanes; ++k) tl[k] = k == i ? INFINITY : tl[k];
+    }
+    if (tie) return trace_ray_again(S, root, t_eps, o, d, skip, t_best, tri_best, w);
     if (bi < 0) return false;
     t_best = best;
     tri_best = bi;
@@ -866,33 +953,41 @@ __device__ __forceinline__ ORayItem load_item(const ORayItem *q, unsigned long l
 // ------------------------------------------------------------------------------------------
 // counters
 // ------------------------------------------------------------------------------------------
+// Work of one thread in one launch (32-bit: a thread takes a few hundred rays at most; blocks sum into 64 bits).
 struct LocalCounters {
-    unsigned long long v[11] = {0};  // prim, seg_broad, seg_b, seg_c, oct, end_traces, det, capped, retests, overflow, spills
+    unsigned v[11] = {0};  // prim, seg_broad, seg_b, seg_c, oct, end_traces, det, capped, retests, overflow, spills
     double lost = 0, init = 0;
 };
 enum { C_PRIM, C_SEGA, C_SEGB, C_SEGC, C_OCT, C_END, C_DET, C_CAP, C_RET, C_OVF, C_SPILL };
 
+// Every thread of the block calls.  One warp reduction per counter, one global atomic per block and counter.
 __device__ void flush_counters(const DevRun &r, const LocalCounters &L) {
-    __shared__ unsigned long long s_u[11];
+    __shared__ unsigned s_u[11];
     __shared__ double s_d[2];
     if (threadIdx.x < 11) s_u[threadIdx.x] = 0;
     if (threadIdx.x < 2) s_d[threadIdx.x] = 0;
     __syncthreads();
 #pragma unroll
-    for (int i = 0; i < 11; ++i)
-        if (L.v[i]) atomicAdd(&s_u[i], L.v[i]);
+    for (int i = 0; i < 11; ++i) {
+        const unsigned n = __reduce_add_sync(0xffffffffu, L.v[i]);
+        if ((threadIdx.x & 31) == 0 && n) atomicAdd(&s_u[i], n);
+    }
     if (L.lost != 0) atomicAdd(&s_d[0], L.lost);
     if (L.init != 0) atomicAdd(&s_d[1], L.init);
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (threadIdx.x < 11 && s_u[threadIdx.x]) {
         DevCounters *c = r.cnt;
         unsigned long long *dst[11] = {&c->primaries, &c->seg_broad, &c->seg_b, &c->seg_c, &c->octave_rays,
                                        &c->end_traces, &c->detections, &c->capped, &c->retests, &c->queue_overflow,
                                        &c->stack_spills};
-        for (int i = 0; i < 11; ++i)
-            if (s_u[i]) atomicAdd(dst[i], s_u[i]);
-        if (s_d[0] != 0) atomicAdd(&c->lost_energy, s_d[0]);
-        if (s_d[1] != 0) atomicAdd(&c->initial_energy, s_d[1]);
+        unsigned long long *d = dst[0];
+#pragma unroll
+        for (int i = 1; i < 11; ++i) d = (int)threadIdx.x == i ? dst[i] : d;
+        atomicAdd(d, (unsigned long long)s_u[threadIdx.x]);
+    }
+    if (threadIdx.x == 32 % blockDim.x) {
+        if (s_d[0] != 0) atomicAdd(&r.cnt->lost_energy, s_d[0]);
+        if (s_d[1] != 0) atomicAdd(&r.cnt->initial_energy, s_d[1]);
     }
 }
 

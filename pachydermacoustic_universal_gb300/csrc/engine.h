@@ -110,6 +110,12 @@ constexpr int kBvhQNodeFloats = 12;  // 48-byte quantised nodes
 constexpr int kLeafMax = 8;      // largest leaf the node encoding holds
 constexpr int kLeafDefault = 3;  // leaf size used when the scene does not ask for one (measured best of 2..8)
 
+// Scenes of at most kFuseMaxTris triangles in at most kMaxPlanes planes (shoeboxes, simple shells) also carry
+// their planes: two float4 each, (unit normal, offset: n x + offset = 0) and (first entry, entries, coplanar group
+// as int bits) into a list of triangles.  Every vertex lies within 1e-6 of the extent of its plane and no
+// triangle is a sliver (sine of an angle below 0.05), which the walk over planes relies on.
+constexpr int kMaxPlanes = 8;
+
 // Device scene view (passed by value to kernels).
 struct DevScene {
     const float4 *tri;          // [ntri*3]: (v0, plane bits) (e1, poly bits) (e2, grazing threshold)
@@ -119,6 +125,8 @@ struct DevScene {
     const float *trans;         // [npoly*8]
     const float4 *bvh;          // [nodes*8] 128-byte nodes
     const float4 *bvhq;         // [nodes*3] 48-byte quantised nodes (null: walk the 128-byte ones)
+    const float4 *plane;        // [planes*2] every room's planes (RoomParams::plane_begin)
+    const int *plane_tri;       // the planes' triangles
     int ntri;
     float t_eps;
     int has_trans;
@@ -161,6 +169,7 @@ struct WaveCtl {
     unsigned long long pilot_peak;  // peak live count while the pilot runs
     int pilot_first, pilot_room;    // rooms [pilot_first, pilot_room) are the pilot in flight; from pilot_room on
                                     // no pilot has been fed
+    int bounces;                    // surface interactions a ray of this wave may take before it goes back (fused walk)
     unsigned bb_blocks;             // blocks of the phase-A launch that have finished
     int pressure;                   // the ring passed three quarters full since the last batch was fed
 };
@@ -184,6 +193,7 @@ struct RoomParams {
     int rec_begin, R;                // its receivers [rec_begin, rec_begin + R) (run-wide receiver index)
     int src_begin, nsrc;             // its sources
     int h_oct, oct_lo, oct_hi, is_order, pure_specular, max_broad;
+    int plane_begin, n_planes;       // its planes (0: walk the BVH)
 };
 constexpr int kMaxRooms = 4096;
 // Receiver tables up to this size are staged in shared memory by the detection kernels.
@@ -271,6 +281,7 @@ struct DevRun {
                                    // miss.  The walk writes the hit's polygon and group so that the shading
                                    // pass loads normal and material directly, one dependent load fewer
     unsigned long long max_wave;   // items per wave at most
+    int max_bounces;               // interactions per wave item at most (1: one; more: k_bounce)
     long long feed_batch;          // primaries per phase-A launch at most
     unsigned long long feed_bound; // ring slots one primary can fill in phase A
     unsigned long long low_water;  // feed new primaries when fewer live items remain
@@ -384,6 +395,11 @@ cudaError_t launch_map_params(const double *etc, int n, int T, double fs, double
 cudaError_t launch_scale(double *dst, const double *src, size_t n, double f, const double *rows, size_t per_row,
                          cudaStream_t s);
 constexpr int kFuseMaxTris = 64;
+// k_bounce: walk and shade in one kernel, rays staying in registers over up to kMaxBounces interactions; planes:
+// every room has its planes.  Used for fused scenes without mapping receivers.
+constexpr int kMaxBounces = 32;
+cudaError_t launch_bounce(const DevRun &r, int blocks, int threads, cudaStream_t s, bool planes);
+cudaError_t bounce_occupancy(int threads, int smem, int *blocks_per_sm, bool planes);
 inline bool fused_walk(int traversal, int ntri) { return traversal == 3 || (traversal == 0 && ntri <= kFuseMaxTris); }
 cudaError_t wave_kernel_occupancy(int variant, int threads, int smem_shade, int *bpsm_trace, int *bpsm_shade,
                                   bool fused = false, bool wide = false);
@@ -419,6 +435,7 @@ constexpr int kConvKinds = 4;        // energy, analysis 0..2
 
 // capi.cpp: read access to a scene handle (for entry points in other translation units)
 const HostScene *scene_host(const pach_scene *s);
+int scene_planes(const pach_scene *s);  // planes of the scene's own device copy (0: none)
 const DevScene *scene_dev(const pach_scene *s);
 int scene_device(const pach_scene *s);
 void set_last_error(const char *msg);

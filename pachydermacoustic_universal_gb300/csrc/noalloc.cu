@@ -184,6 +184,7 @@ extern "C" pach_status pach_trace_run_noalloc(const pach_scene *scene, const pac
         room.oct_hi = p.oct_hi;
         room.is_order = p.is_order;
         room.pure_specular = p.pure_specular;
+        room.n_planes = scene_planes(scene);
         room.max_broad = (int)std::fmin((double)max_broad, (double)(1u << 30));
         NA_TRY(cudaMemcpyAsync(base + kOffRoom, &room, sizeof(room), cudaMemcpyHostToDevice, stream));
         NA_TRY(cudaMemcpyAsync(base + kOffCtl, &h_ctl, sizeof(WaveCtl), cudaMemcpyHostToDevice, stream));
@@ -228,6 +229,9 @@ extern "C" pach_status pach_trace_run_noalloc(const pach_scene *scene, const pac
         const int variant = trace_variant(p.blocks_per_sm, p.traversal, (int)hs.tri_poly.size(), quant);
         NA_TRY(wave_kernel_occupancy(variant, 256, receiver_smem_bytes(n_receivers), &bps_tr, &bps_sh,
                                      fused_walk(p.traversal, (int)hs.tri_poly.size())));
+        const bool fused = fused_walk(p.traversal, (int)hs.tri_poly.size()), by_planes = fused && room.n_planes > 0;
+        if (fused) NA_TRY(bounce_occupancy(256, receiver_smem_bytes(n_receivers), &bps_sh, by_planes));
+        r.max_bounces = fused ? kMaxBounces : 1;
         const int tr_blocks = sms * (bps_tr > 0 ? bps_tr : 1), sh_blocks = sms * (bps_sh > 0 ? bps_sh : 1);
         long long launches = 0;
         // Every iteration of the loop either traces a wave or feeds primaries, so the schedule moves on
@@ -240,9 +244,8 @@ extern "C" pach_status pach_trace_run_noalloc(const pach_scene *scene, const pac
             for (int k = 0; k < 32; ++k) {
                 NA_TRY(launch_feed(r, stream));
                 NA_TRY(launch_broadband(r, sms * 2, 128, stream, false, hs.ntri <= kFuseMaxTris));
-                const bool fused = fused_walk(p.traversal, (int)hs.tri_poly.size());
                 if (!fused) NA_TRY(launch_trace(r, variant, tr_blocks, 256, stream));
-                NA_TRY(launch_shade(r, sh_blocks, 256, stream, fused));
+                NA_TRY(fused ? launch_bounce(r, sh_blocks, 256, stream, by_planes) : launch_shade(r, sh_blocks, 256, stream));
                 launches += fused ? 3 : 4;
             }
             NA_TRY(cudaMemcpyAsync(&h_ctl, base + kOffCtl, sizeof(WaveCtl), cudaMemcpyDeviceToHost, stream));

@@ -26,10 +26,6 @@ namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
 
-__device__ __forceinline__ ORayItem ring_load(const DevRun &r, unsigned long long i) {
-    return load_item(r.ring, i & (r.ring_cap - 1));
-}
-
 __device__ __forceinline__ void ring_store(const DevRun &r, unsigned long long i, const ORayItem &it) {
     store_item(r.ring, i & (r.ring_cap - 1), it);
 }
@@ -225,6 +221,9 @@ __device__ void size_wave(const DevRun &r) {
     if (m > live) m = live;
     if (m > r.max_wave) m = r.max_wave;
     c->m = m;
+    // an item that takes k interactions leaves at most k + 1 (one split each, and itself)
+    const unsigned long long per = m ? (r.ring_cap - live) / m - 1 : 1;
+    c->bounces = (int)(per < (unsigned long long)r.max_bounces ? per : (unsigned long long)r.max_bounces);
     c->trace_next = 0;
     if (m) ++c->waves;
     if (live == 0 && c->next_prim >= c->prim_end) c->done = 1;
@@ -682,6 +681,78 @@ __global__ void __launch_bounds__(256, MINB) k_trace(DevRun r) {
     }
 }
 
+// The part of a split child that differs from its parent.
+struct Child {
+    float I;
+    float3 d;
+    unsigned long long sid;
+    int mask;
+};
+__device__ __forceinline__ Ray child_ray(const Ray &R, const Child &C) {
+    Ray c = R;
+    c.I = C.I; c.d = C.d; c.sid = C.sid; c.mask = C.mask;
+    c.nb = 0;
+    c.phase = 0;
+    return c;
+}
+
+// One surface interaction at hit h (triangle, t bits, polygon, coplanar group): the ray moves to the surface, is
+// absorbed and scattered.  Returns whether it goes on; split: C is its split child (at the same place).
+__device__ __forceinline__ bool surface(const DevRun &r, const DevScene &S, const RoomParams &P, int4 h, Ray &R,
+                                        bool &split, Child &C, LocalCounters &L) {
+    const float t = __int_as_float(h.y);
+    R.t_sum += (double)t * P.inv_c_d;
+    R.p = R.p + R.d * t;
+    R.plane = h.w;
+    const int poly = h.z;
+    const float3 n = f3(__ldg(S.pnormal + poly));
+    const float cos_t = dot3(n, R.d);
+    const float4 mt = __ldg(S.mat + poly * kBands + R.oct);  // (1-alpha, s_lo, s_mid, s_hi)
+    R.I *= mt.x;
+    const float4 U = draw(r.seed, R.prim, R.sid, 1u + R.nb);
+    const uint32_t nb = R.nb++;
+    const bool transmit = S.has_trans && !P.pure_specular && U.x < __ldg(S.trans + poly * kBands + R.oct);
+    const float3 spec = R.d - n * (2.f * cos_t);
+    const float3 nn = cos_t > 0.f ? n * -1.f : n;
+    bool alive = true;
+    if (R.phase == 0) {
+        // Scatter_Late
+        if (P.pure_specular || U.y > mt.w) {
+            R.d = transmit ? spec * -1.f : spec;
+            R.mask &= ~1;
+        } else {
+            if (U.y > mt.y) {
+                split = true;
+                C.I = R.I * (1.f - mt.z);
+                R.I *= mt.z;
+                C.mask = R.mask & ~1;
+                C.d = transmit ? spec * -1.f : spec;
+                C.sid = sid_late(R.sid, nb);
+                ++L.v[C_OCT];
+            }
+            const float3 ld = lambert(nn, U.z, U.w);
+            R.d = transmit ? ld * -1.f : ld;
+            R.mask |= 3;
+        }
+        // phase-B loop test (TaskAll:473): failing it enters End_Trace, which always traces at least one
+        // more segment
+        if (!(R.t_sum < P.cotime && R.I > kTP2)) { R.phase = 1; ++L.v[C_END]; }
+    } else {
+        // Scatter_VeryLate
+        if (!P.pure_specular && U.y < mt.z) {
+            R.d = lambert(nn, U.z, U.w);
+            R.mask |= 3;
+        } else {
+            R.d = spec;
+            R.mask &= ~1;
+        }
+        if (transmit) R.d = R.d * -1.f;
+        alive = R.t_sum < P.cotime && R.I > kTP3;  // TaskAll:534
+    }
+    if (alive && (long long)R.nb >= r.max_seg) { ++L.v[C_CAP]; alive = false; }
+    return alive;
+}
+
 // FUSED: walk the ray here instead of reading k_trace's hit (small scenes, whose walk is a few
 // cached nodes: the separate trace pass would only re-read the ray and round-trip its hit via HBM).
 // the shading pass alone fits three 256-thread blocks per SM (80 registers; +1.6 % on a 500k-triangle
@@ -739,59 +810,10 @@ __global__ void __launch_bounds__(256, FUSED ? 2 : (WIDE ? 4 : kShadeMinBlocks))
                 // lost: no End_Trace after a miss in phase B (TaskAll:437-443), loop exit in phase C (500-505)
                 L.lost += (double)(R.I * R.scale);
             } else {
-                R.t_sum += (double)t * P.inv_c_d;
-                R.p = R.p + R.d * t;
-                R.plane = h.w;
-                const int poly = h.z;
-                const float3 n = f3(__ldg(S.pnormal + poly));
-                const float cos_t = dot3(n, R.d);
-                const float4 mt = __ldg(S.mat + poly * kBands + R.oct);  // (1-alpha, s_lo, s_mid, s_hi)
-                R.I *= mt.x;
-                const float4 U = draw(r.seed, R.prim, R.sid, 1u + R.nb);
-                const uint32_t nb = R.nb++;
-                const bool transmit = S.has_trans && !P.pure_specular && U.x < __ldg(S.trans + poly * kBands + R.oct);
-                const float3 spec = R.d - n * (2.f * cos_t);
-                const float3 nn = cos_t > 0.f ? n * -1.f : n;
-                bool alive = true;
+                Child ch;
                 bool split = false;
-                if (R.phase == 0) {
-                    // Scatter_Late
-                    if (P.pure_specular || U.y > mt.w) {
-                        R.d = transmit ? spec * -1.f : spec;
-                        R.mask &= ~1;
-                    } else {
-                        if (U.y > mt.y) {
-                            split = true;
-                            C = R;
-                            C.I = R.I * (1.f - mt.z);
-                            R.I *= mt.z;
-                            C.mask &= ~1;
-                            C.d = transmit ? spec * -1.f : spec;
-                            C.sid = sid_late(R.sid, nb);
-                            C.nb = 0;
-                            C.phase = 0;
-                            ++L.v[C_OCT];
-                        }
-                        const float3 ld = lambert(nn, U.z, U.w);
-                        R.d = transmit ? ld * -1.f : ld;
-                        R.mask |= 3;
-                    }
-                    // phase-B loop test (TaskAll:473): failing it enters End_Trace, which always
-                    // traces at least one more segment
-                    if (!(R.t_sum < P.cotime && R.I > kTP2)) { R.phase = 1; ++L.v[C_END]; }
-                } else {
-                    // Scatter_VeryLate
-                    if (!P.pure_specular && U.y < mt.z) {
-                        R.d = lambert(nn, U.z, U.w);
-                        R.mask |= 3;
-                    } else {
-                        R.d = spec;
-                        R.mask &= ~1;
-                    }
-                    if (transmit) R.d = R.d * -1.f;
-                    alive = R.t_sum < P.cotime && R.I > kTP3;  // TaskAll:534
-                }
-                if (alive && (long long)R.nb >= r.max_seg) { ++L.v[C_CAP]; alive = false; }
+                bool alive = surface(r, S, P, h, R, split, ch, L);
+                if (split) C = child_ray(R, ch);
                 if (!alive && split) { R = C; split = false; alive = true; }
                 nout = (alive ? 1 : 0) + (split ? 1 : 0);
             }
@@ -805,6 +827,116 @@ __global__ void __launch_bounds__(256, FUSED ? 2 : (WIDE ? 4 : kShadeMinBlocks))
         const unsigned long long slot = warp_append(&c->tail, nout);
         if (nout >= 1) ring_store(r, slot, to_item(R));
         if (nout == 2) ring_store(r, slot + 1, to_item(C));
+    }
+    flush_counters(r, L);
+}
+
+// Small scenes: walk and shade, each lane keeping its ray in registers over up to ctl->bounces interactions, then
+// taking the next wave item (a lane whose ray ends takes one at once).  Split children go to the ring as they
+// arise; rays that have used up their interactions go back to it.
+// Bound: latency of the walk's and the interaction's dependent loads, three blocks an SM.  One interaction a
+// launch read and wrote every ray (128 bytes) and appended it each time, and a chain of 200 interactions was 200
+// waves: a 1003-primary shoebox took 228 waves and 19 ms, BNC1; 100k primaries 1180 ms, BNC2.
+template <bool PLANES>
+__global__ void __launch_bounds__(256, 3) k_bounce(DevRun r) {
+    extern __shared__ float4 s_rec_buf[];
+    __shared__ float4 s_plane[2 * kMaxPlanes];
+    const int *s_rid;
+    const float4 *s_rec = stage_receivers(r, s_rec_buf, s_rid);
+    LocalCounters L;
+    const DevScene &S = r.S;
+    WaveCtl *c = r.ctl;
+    const unsigned long long m = c->m, head = c->head;
+    const int bounces = c->bounces, lane = threadIdx.x & 31;
+    const bool count_room = r.n_rooms > 1 && c->pilot_count > 0;
+    if constexpr (PLANES) {
+        if (r.n_rooms == 1) {
+            const int np = 2 * r.rooms[0].n_planes;
+            if ((int)threadIdx.x < np) s_plane[threadIdx.x] = S.plane[2 * r.rooms[0].plane_begin + threadIdx.x];
+            __syncthreads();
+        }
+    }
+    Ray R;
+    bool have = false, exhausted = false;
+    int left = 0;
+    for (;;) {
+        const unsigned need = __ballot_sync(FULL, !have && !exhausted);
+        if (need) {
+            const int leader = __ffs(need) - 1;
+            unsigned long long base = 0;
+            if (lane == leader) base = atomicAdd(&c->trace_next, (unsigned long long)__popc(need));
+            base = __shfl_sync(FULL, base, leader);
+            if (!have && !exhausted) {
+                const unsigned long long j = base + __popc(need & ((1u << lane) - 1u));
+                if (j < m) {
+                    R = to_ray(load_item(r.ring, (head + j) & (r.ring_cap - 1)));
+                    left = bounces;
+                    have = true;
+                } else {
+                    exhausted = true;
+                }
+            }
+        }
+        if (!__any_sync(FULL, have)) break;
+        if (have) {
+            const RoomParams &P = r.rooms[R.room];
+            float t = 0.f;
+            int tri = -1;
+            TraceWork tw;
+            bool hit;
+            const int root = r.n_rooms > 1 ? P.bvh_root : 0;
+            const float teps = r.n_rooms > 1 ? P.t_eps : S.t_eps;
+            if constexpr (PLANES)
+                hit = plane_walk(S, r.n_rooms == 1 ? s_plane : S.plane + 2 * P.plane_begin, P.n_planes, root, teps, R.p,
+                                 R.d, R.plane, t, tri, tw);
+            else
+                hit = trace_ray<int>(S, root, teps, R.p, R.d, R.plane, t, tri, tw);
+            L.v[C_RET] += tw.retests;
+            ++L.v[R.phase == 0 ? C_SEGB : C_SEGC];
+            L.v[C_DET] += detect_octave<false>(r, P, s_rec, s_rid, R.p, R.d, hit ? t : 1e6f, R.t_sum, R.I * R.scale, R.oct,
+                                               R.mask, R.prim);
+            bool alive = false, split = false;
+            Child ch;
+            if (!hit) {
+                // lost: no End_Trace after a miss in phase B (TaskAll:437-443), loop exit in phase C (500-505)
+                L.lost += (double)(R.I * R.scale);
+            } else {
+                const float4 A = __ldg(S.tri + 3 * tri), B = __ldg(S.tri + 3 * tri + 1);
+                alive = surface(r, S, P, make_int4(tri, __float_as_int(t), __float_as_int(B.w), __float_as_int(A.w)), R,
+                                split, ch, L);
+            }
+            if (split) {
+                if (alive) {
+                    // one atomic for the lanes that are here together
+                    const unsigned here = __activemask();
+                    const int first = __ffs(here) - 1;
+                    unsigned long long slot = 0;
+                    if (lane == first) slot = atomicAdd(&c->tail, (unsigned long long)__popc(here));
+                    slot = __shfl_sync(here, slot, first) + __popc(here & ((1u << lane) - 1u));
+                    ring_store(r, slot, to_item(child_ray(R, ch)));
+                    if (count_room) atomicAdd(r.room_live + R.room, 1u);
+                } else {
+                    R = child_ray(R, ch);  // the child takes the parent's place
+                    alive = true;
+                }
+            }
+            if (!alive) {
+                have = false;
+                if (count_room) atomicSub(r.room_live + R.room, 1u);
+            }
+            --left;
+        }
+        const unsigned back = __ballot_sync(FULL, have && left <= 0);
+        if (back) {
+            const int first = __ffs(back) - 1;
+            unsigned long long slot = 0;
+            if (lane == first) slot = atomicAdd(&c->tail, (unsigned long long)__popc(back));
+            slot = __shfl_sync(FULL, slot, first) + __popc(back & ((1u << lane) - 1u));
+            if (have && left <= 0) {
+                ring_store(r, slot, to_item(R));
+                have = false;
+            }
+        }
     }
     flush_counters(r, L);
 }
@@ -963,11 +1095,21 @@ cudaError_t launch_shade(const DevRun &r, int blocks, int threads, cudaStream_t 
         if (fused) k_shade<true, true><<<blocks, threads, rec_smem(r), s>>>(r);
         else k_shade<false, true><<<blocks, threads, rec_smem(r), s>>>(r);
     } else {
-        if (fused) k_shade<true, false><<<blocks, threads, rec_smem(r), s>>>(r);
-        else if (wide) k_shade<false, false, true><<<blocks, threads, rec_smem(r), s>>>(r);
+        if (wide) k_shade<false, false, true><<<blocks, threads, rec_smem(r), s>>>(r);
         else k_shade<false, false><<<blocks, threads, rec_smem(r), s>>>(r);
     }
     return cudaGetLastError();
+}
+
+cudaError_t launch_bounce(const DevRun &r, int blocks, int threads, cudaStream_t s, bool planes) {
+    if (planes) k_bounce<true><<<blocks, threads, rec_smem(r), s>>>(r);
+    else k_bounce<false><<<blocks, threads, rec_smem(r), s>>>(r);
+    return cudaGetLastError();
+}
+
+cudaError_t bounce_occupancy(int threads, int smem, int *blocks_per_sm, bool planes) {
+    return planes ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_bounce<true>, threads, smem)
+                  : cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_bounce<false>, threads, smem);
 }
 
 cudaError_t wave_kernel_occupancy(int variant, int threads, int smem_shade, int *bpsm_trace, int *bpsm_shade,
@@ -983,7 +1125,7 @@ cudaError_t wave_kernel_occupancy(int variant, int threads, int smem_shade, int 
         default: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(bpsm_trace, k_trace<4, false, false>, threads, 0); break;
     }
     if (e != cudaSuccess) return e;
-    if (fused) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(bpsm_shade, k_shade<true, false>, threads, smem_shade);
+    if (fused) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(bpsm_shade, k_shade<true, true>, threads, smem_shade);
     if (wide) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(bpsm_shade, k_shade<false, false, true>, threads, smem_shade);
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(bpsm_shade, k_shade<false, false>, threads, smem_shade);
 }
