@@ -691,7 +691,8 @@ void run_worker_body(pach_run *run) {
         // default ring: room for the run's rays at up to 2048 live octave rays per primary, 2^22..2^28
         // (17 GB); default wave 8M rays -- measured against 2M: +7 % on a 20k-triangle hall and a
         // 500k-triangle arena, +19 % on a 12-triangle shoebox (fewer, fuller iterations)
-        int ring_default = n_rooms > 1 ? 24 : 22;  // a batch's pilots run several rooms at a time
+        // a batch's pilots run several rooms at a time, and rays of small scenes leave several children a wave
+        int ring_default = n_rooms > 1 || bounce ? kRingMin : 22;
         while (ring_default < 28 && (1ull << ring_default) < (unsigned long long)rprim_total(run) * 2048ull) ++ring_default;
         const int ring_log2 = run->p.ring_log2 > 0 ? std::min(32, std::max(16, run->p.ring_log2)) : ring_default;
         const unsigned long long ring_cap = 1ull << ring_log2;
@@ -806,6 +807,7 @@ void run_worker_body(pach_run *run) {
         }
         r.max_wave = std::min(max_wave, ring_cap);
         r.max_bounces = bounce ? kMaxBounces : 1;
+        r.full_wave = kFullFactor * (unsigned long long)sh_blocks * threads;
         r.feed_bound = bound;
         r.low_water = std::min(ring_cap / 4, 2 * r.max_wave);
         const long long N = rprim[n_rooms] - rprim[0];

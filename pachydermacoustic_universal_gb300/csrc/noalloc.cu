@@ -233,6 +233,7 @@ extern "C" pach_status pach_trace_run_noalloc(const pach_scene *scene, const pac
         if (fused) NA_TRY(bounce_occupancy(256, receiver_smem_bytes(n_receivers), &bps_sh, by_planes));
         r.max_bounces = fused ? kMaxBounces : 1;
         const int tr_blocks = sms * (bps_tr > 0 ? bps_tr : 1), sh_blocks = sms * (bps_sh > 0 ? bps_sh : 1);
+        r.full_wave = kFullFactor * (unsigned long long)sh_blocks * 256;
         long long launches = 0;
         // Every iteration of the loop either traces a wave or feeds primaries, so the schedule moves on
         // each time; if it stops moving for kNaStall synchronisations in a row (kNaStall x 32

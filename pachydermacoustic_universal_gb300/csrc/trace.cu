@@ -221,9 +221,12 @@ __device__ void size_wave(const DevRun &r) {
     if (m > live) m = live;
     if (m > r.max_wave) m = r.max_wave;
     c->m = m;
-    // an item that takes k interactions leaves at most k + 1 (one split each, and itself)
-    const unsigned long long per = m ? (r.ring_cap - live) / m - 1 : 1;
-    c->bounces = (int)(per < (unsigned long long)r.max_bounces ? per : (unsigned long long)r.max_bounces);
+    // a wave of k interactions leaves its items and at most k children of each phase-B ray in the ring
+    const unsigned long long splitting = (unsigned long long)max(__ldcg(&c->live_b), 1ll);
+    const unsigned long long per = max((r.ring_cap - live - m) / min(splitting, max(m, 1ull)), 1ull);
+    // a wave that does not fill the machine is a matter of latency: its split children should not wait long
+    const unsigned long long most = (unsigned long long)(m < r.full_wave ? min(r.max_bounces, kSmallBounces) : r.max_bounces);
+    c->bounces = (int)(per < most ? per : most);
     c->trace_next = 0;
     if (m) ++c->waves;
     if (live == 0 && c->next_prim >= c->prim_end) c->done = 1;
@@ -288,6 +291,7 @@ __global__ void __launch_bounds__(128) k_broadband(DevRun r) {
     LocalCounters L;
     const DevScene &S = r.S;
     const bool count_room = r.n_rooms > 1 && c->pilot_count > 0;
+    int born = 0;
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += stride) {
         int room;
@@ -355,6 +359,7 @@ __global__ void __launch_bounds__(128) k_broadband(DevRun r) {
             for (int o = 0; o < kBands; ++o) nchild += (E[o] != 0.f) ? (tau[o] > 0.f ? 3 : 1) : 0;
             unsigned long long slot = nchild ? atomicAdd(&c->tail, (unsigned long long)nchild) : 0ull;
             if (count_room && nchild) atomicAdd(r.room_live + room, (unsigned)nchild);
+            born += nchild;
 #pragma unroll
             for (int o = 0; o < kBands; ++o) {
                 if (E[o] == 0.f) continue;
@@ -389,6 +394,7 @@ __global__ void __launch_bounds__(128) k_broadband(DevRun r) {
             const int nfin = P.oct_hi - P.oct_lo + 1;
             unsigned long long slot = atomicAdd(&c->tail, (unsigned long long)nfin);
             if (count_room) atomicAdd(r.room_live + room, (unsigned)nfin);
+            born += nfin;
 #pragma unroll
             for (int o = 0; o < kBands; ++o) {
                 if (o < P.oct_lo || o > P.oct_hi) continue;
@@ -399,6 +405,8 @@ __global__ void __launch_bounds__(128) k_broadband(DevRun r) {
         }
         ++L.v[C_PRIM];
     }
+    born = (int)__reduce_add_sync(FULL, (unsigned)born);
+    if ((threadIdx.x & 31) == 0 && born) atomicAdd(reinterpret_cast<unsigned long long *>(&c->live_b), (unsigned long long)born);
     flush_counters(r, L);
     // the last block with work sizes the wave
     __syncthreads();
@@ -834,12 +842,27 @@ __global__ void __launch_bounds__(256, FUSED ? 2 : (WIDE ? 4 : kShadeMinBlocks))
 // Small scenes: walk and shade, each lane keeping its ray in registers over up to ctl->bounces interactions, then
 // taking the next wave item (a lane whose ray ends takes one at once).  Split children go to the ring as they
 // arise; rays that have used up their interactions go back to it.
-// Bound: latency of the walk's and the interaction's dependent loads, three blocks an SM.  One interaction a
+// Bound: issue (61 % of slots, 19.6 of 32 lanes active: interactions differ) at three blocks an SM; two or four
+// blocks 848 and 834 ms where three take 753.  One interaction a
 // launch read and wrote every ray (128 bytes) and appended it each time, and a chain of 200 interactions was 200
-// waves: a 1003-primary shoebox took 228 waves and 19 ms, BNC1; 100k primaries 1180 ms, BNC2.
+// waves: a 1003-primary shoebox took 228 waves and 19.1 ms, now 30 and 9.6 ms; 100k primaries 1180 ms, now 753.
+//
+// Detections wait in a queue of the warp until 32 are there, so that a lane's detection (FP64 time and bin, six
+// atomics) does not hold the other 31: in a 3-receiver shoebox 3 % of the segments, two of three iterations.
+struct Detection {
+    double t_sum;
+    float t, half, I;      // chord midpoint and half length, absolute energy
+    float dx, dy, dz;
+    unsigned at;           // receiver slot << 5 | band << 2 | mask
+    uint32_t prim;
+    unsigned room, pad;
+};
+constexpr int kQueue = 64;
+
 template <bool PLANES>
 __global__ void __launch_bounds__(256, 3) k_bounce(DevRun r) {
     extern __shared__ float4 s_rec_buf[];
+    __shared__ Detection s_det[8][kQueue];
     __shared__ float4 s_plane[2 * kMaxPlanes];
     const int *s_rid;
     const float4 *s_rec = stage_receivers(r, s_rec_buf, s_rid);
@@ -856,9 +879,17 @@ __global__ void __launch_bounds__(256, 3) k_bounce(DevRun r) {
             __syncthreads();
         }
     }
+    Detection *queue = s_det[threadIdx.x >> 5];
+    int queued = 0;
+    auto detect = [&](int i) {
+        const Detection e = queue[i];
+        const int s = (int)(e.at >> 5);
+        detect_octave_one(r, r.rooms[e.room], s_rid, s, s_rec[s], make_float3(e.dx, e.dy, e.dz), e.t, e.half, e.t_sum, e.I,
+                          (int)(e.at >> 2) & 7, (int)e.at & 3, e.prim);
+    };
     Ray R;
     bool have = false, exhausted = false;
-    int left = 0;
+    int left = 0, splitting = 0;  // phase-B rays put into the ring less those taken out
     for (;;) {
         const unsigned need = __ballot_sync(FULL, !have && !exhausted);
         if (need) {
@@ -871,6 +902,7 @@ __global__ void __launch_bounds__(256, 3) k_bounce(DevRun r) {
                 if (j < m) {
                     R = to_ray(load_item(r.ring, (head + j) & (r.ring_cap - 1)));
                     left = bounces;
+                    splitting -= R.phase == 0;
                     have = true;
                 } else {
                     exhausted = true;
@@ -878,12 +910,12 @@ __global__ void __launch_bounds__(256, 3) k_bounce(DevRun r) {
             }
         }
         if (!__any_sync(FULL, have)) break;
+        float t = 0.f;
+        int tri = -1, s0 = 0, s1 = 0;
+        bool hit = false;
         if (have) {
             const RoomParams &P = r.rooms[R.room];
-            float t = 0.f;
-            int tri = -1;
             TraceWork tw;
-            bool hit;
             const int root = r.n_rooms > 1 ? P.bvh_root : 0;
             const float teps = r.n_rooms > 1 ? P.t_eps : S.t_eps;
             if constexpr (PLANES)
@@ -893,8 +925,38 @@ __global__ void __launch_bounds__(256, 3) k_bounce(DevRun r) {
                 hit = trace_ray<int>(S, root, teps, R.p, R.d, R.plane, t, tri, tw);
             L.v[C_RET] += tw.retests;
             ++L.v[R.phase == 0 ? C_SEGB : C_SEGC];
-            L.v[C_DET] += detect_octave<false>(r, P, s_rec, s_rid, R.p, R.d, hit ? t : 1e6f, R.t_sum, R.I * R.scale, R.oct,
-                                               R.mask, R.prim);
+            s0 = P.rec_begin;
+            s1 = s0 + P.R;
+        }
+        // Spherical_Receiver.CheckRay over the room's receivers
+        for (;; ++s0) {
+            if (!__any_sync(FULL, s0 < s1)) break;
+            float tc = 0.f, half = 0.f;
+            const bool found = s0 < s1 && sphere_hit(s_rec[s0], R.p, R.d, hit ? t : 1e6f, tc, half);
+            const unsigned who = __ballot_sync(FULL, found);
+            if (!who) continue;
+            if (found) {
+                ++L.v[C_DET];
+                Detection e;
+                e.t_sum = R.t_sum;
+                e.t = tc; e.half = half; e.I = R.I * R.scale;
+                e.dx = R.d.x; e.dy = R.d.y; e.dz = R.d.z;
+                e.at = (unsigned)s0 << 5 | (unsigned)R.oct << 2 | (unsigned)R.mask;
+                e.prim = R.prim;
+                e.room = (unsigned)R.room;
+                e.pad = 0;
+                queue[queued + __popc(who & ((1u << lane) - 1u))] = e;
+            }
+            queued += __popc(who);
+            if (queued >= 32) {
+                __syncwarp();
+                queued -= 32;
+                detect(queued + lane);
+                __syncwarp();
+            }
+        }
+        if (have) {
+            const RoomParams &P = r.rooms[R.room];
             bool alive = false, split = false;
             Child ch;
             if (!hit) {
@@ -914,6 +976,7 @@ __global__ void __launch_bounds__(256, 3) k_bounce(DevRun r) {
                     if (lane == first) slot = atomicAdd(&c->tail, (unsigned long long)__popc(here));
                     slot = __shfl_sync(here, slot, first) + __popc(here & ((1u << lane) - 1u));
                     ring_store(r, slot, to_item(child_ray(R, ch)));
+                    ++splitting;
                     if (count_room) atomicAdd(r.room_live + R.room, 1u);
                 } else {
                     R = child_ray(R, ch);  // the child takes the parent's place
@@ -934,10 +997,16 @@ __global__ void __launch_bounds__(256, 3) k_bounce(DevRun r) {
             slot = __shfl_sync(FULL, slot, first) + __popc(back & ((1u << lane) - 1u));
             if (have && left <= 0) {
                 ring_store(r, slot, to_item(R));
+                splitting += R.phase == 0;
                 have = false;
             }
         }
     }
+    __syncwarp();
+    if (lane < queued) detect(lane);
+    splitting = (int)__reduce_add_sync(FULL, (unsigned)splitting);
+    if (lane == 0 && splitting)
+        atomicAdd(reinterpret_cast<unsigned long long *>(&c->live_b), (unsigned long long)(long long)splitting);
     flush_counters(r, L);
 }
 

@@ -147,3 +147,45 @@ def test_batch_feed_order_traces_every_primary_once(rays, ring_log2, feed_batch)
         for name in ("energy", "pressure", "dir_pos", "dir_neg", "analysis"):
             np.testing.assert_allclose(hb[i][name], hs[name], rtol=1e-9, atol=1e-30, err_msg=f"{i} {name}")
         off += rays[i]
+
+
+def _l_room():
+    """An L-shaped room (8 planes, not convex) of quads in two triangles."""
+    x = [(0, 0), (8, 0), (8, 3), (4, 3), (4, 7), (0, 7)]
+    b = rooms._Builder()
+    lo, hi = [b.vertex((*p, 0.0)) for p in x], [b.vertex((*p, 3.0)) for p in x]
+    for i in range(6):
+        j = (i + 1) % 6
+        b.quad_tris(lo[i], lo[j], hi[j], hi[i])
+    for v in (lo, hi):
+        b.quad_tris(v[0], v[1], v[2], v[3])
+        b.quad_tris(v[0], v[3], v[4], v[5])
+    v, offs, idx = b.arrays()
+    n = offs.size - 1
+    rng = np.random.default_rng(6)
+    scene = rooms.SceneArrays(v, offs, idx, rng.uniform(0.1, 0.4, (n, 8)), np.full((n, 8), 0.3), np.zeros((n, 8)))
+    return rooms.Workload("l_room", scene, [rooms.SourceSpec((1.0, 1.0, 1.5))],
+                          [rooms.ReceiverSpec(p) for p in ((7.0, 1.0, 1.2), (1.0, 6.0, 1.6))], 1000, 0.8)
+
+
+@pytest.mark.parametrize("ring_log2,rays", [(0, 700), (20, 60), (0, 1)])
+@pytest.mark.parametrize("kind", ["box", "l", "diffusers"])
+def test_rays_kept_over_interactions_equal_one_walk_per_launch(kind, ring_log2, rays):
+    """Small scenes (rays kept in registers, the walk over planes where there are at most 8, the BVH for the
+    diffusers' 12 + 36 triangles) against the BVH walk in a launch of its own: the same hits, so the same terms in
+    every bin.  The small ring leaves few interactions a wave; ties go to the BVH in both."""
+    if kind == "box":
+        w = rooms.shoebox_c1()
+    elif kind == "l":
+        w = _l_room()
+    else:
+        w = rooms.shoebox_c1()
+        w.scene = rooms._jittered_room(np.random.default_rng(2), (10.0, 8.0, 4.0), 12, 3, 0.0, (0.1, 0.4), (0.1, 0.5))
+        assert 12 < w.scene.n_triangles <= 64
+    w.cutoff_s = 0.8
+    ds = tracer.DeviceScene(w.scene)
+    ha, sa = tracer.trace(w, dscene=ds, rays=rays, seed=8, ring_log2=ring_log2)
+    hb, sb = tracer.trace(w, dscene=ds, rays=rays, seed=8, traversal=1)
+    assert sa["segments"] == sb["segments"] and sa["detections"] == sb["detections"] and sa["queue_overflows"] == 0
+    for name in ("energy", "pressure", "dir_pos", "dir_neg", "analysis"):
+        np.testing.assert_allclose(ha[name], hb[name], rtol=1e-9, atol=1e-30, err_msg=name)
