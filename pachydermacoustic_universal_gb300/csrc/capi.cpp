@@ -133,6 +133,9 @@ struct pach_run {
     // scaled copies on their way to the host (one caller at a time)
     DevMem stage;
     std::mutex stage_mu;
+    // independent device loops the run's primaries were shared out to, and the feed positions each has finished
+    int pipes = 1;
+    long long pipe_done[kMaxPipes] = {0};
     // worker
     std::thread worker;
     std::mutex mu;
@@ -167,18 +170,29 @@ long long rprim_total(const pach_run *run) {
     return n;
 }
 
-// Primaries of room i among the first `done` of the run's feed order: every room's pilot, then every
-// room's other primaries (one room: its primaries in order).
+// Pipe k's share of a room of n primaries: [share(n, k, P), share(n, k + 1, P)).
+long long share(long long n, int k, int P) { return n * k / P; }
+
+// Primaries of room i that have been traced: `done` of a run of one room; of a batch, the part of each pipe's feed
+// order (every room's pilot, then every room's other primaries) that it has finished.
 long long room_done(const pach_run *run, int i, long long done) {
-    long long pilots = 0, before_p = 0, before_r = 0;
-    for (int k = 0; k < (int)run->rooms.size(); ++k) {
-        const long long pilot = std::min(run->rooms[(size_t)k].rays, kPilotPrimaries);
-        pilots += pilot;
-        if (k < i) { before_p += pilot; before_r += run->rooms[(size_t)k].rays - pilot; }
+    const long long rays = run->rooms[(size_t)i].rays;
+    if (run->rooms.size() == 1 || done >= rprim_total(run)) return std::min(rays, done);
+    long long sum = 0;
+    for (int p = 0; p < run->pipes; ++p) {
+        long long pilots = 0, before_p = 0, before_r = 0, mine = 0, mine_p = 0;
+        for (int k = 0; k < (int)run->rooms.size(); ++k) {
+            const long long n = run->rooms[(size_t)k].rays;
+            const long long part = share(n, p + 1, run->pipes) - share(n, p, run->pipes);
+            const long long pilot = std::min(part, kPilotPrimaries);
+            pilots += pilot;
+            if (k < i) { before_p += pilot; before_r += part - pilot; }
+            if (k == i) { mine = part; mine_p = pilot; }
+        }
+        sum += std::max(0ll, std::min(mine_p, run->pipe_done[p] - before_p)) +
+               std::max(0ll, std::min(mine - mine_p, run->pipe_done[p] - pilots - before_r));
     }
-    const long long rays = run->rooms[(size_t)i].rays, pilot = std::min(rays, kPilotPrimaries);
-    return std::max(0ll, std::min(pilot, done - before_p)) +
-           std::max(0ll, std::min(rays - pilot, done - pilots - before_r));
+    return sum;
 }
 
 // Copies n doubles to the host scaled by f, or by rows[i / per_row] (device): scaled on the device into
@@ -491,8 +505,17 @@ void run_worker_body(pach_run *run) {
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     std::vector<cudaEvent_t> kev;  // per-kernel timing events (kernel_timing = 1)
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t gexec = nullptr;
+    // one device loop: its stream, end event and graph (pipe 0 runs on `stream`)
+    struct Pipe {
+        cudaStream_t stream = nullptr;
+        cudaEvent_t end = nullptr;
+        cudaGraph_t graph = nullptr;
+        cudaGraphExec_t exec = nullptr;
+        DevRun r{};
+        long long p0 = 0;  // first feed position of the current range
+    };
+    Pipe pipes[kMaxPipes];
+    int P = 1;
     std::string where;
     pach_status status = PACH_OK;
     std::string msg;
@@ -511,7 +534,7 @@ void run_worker_body(pach_run *run) {
         TRY(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
         TRY(cudaEventCreate(&ev0));
         TRY(cudaEventCreate(&ev1));
-        TRY(cudaMallocHost(&h_ctl, sizeof(WaveCtl)));
+        TRY(cudaMallocHost(&h_ctl, kMaxPipes * sizeof(WaveCtl)));
         TRY(cudaMallocHost(&h_cnt, sizeof(DevCounters)));
         const int R = run->R, T = run->T;
         const size_t nE = (size_t)R * kBands * T, nD = (size_t)R * 3 * kBands * T;
@@ -521,7 +544,7 @@ void run_worker_body(pach_run *run) {
         TRY(run->hDn.alloc(std::max<size_t>(nD, 1) * 8));
         TRY(run->hAn.alloc(std::max<size_t>(nD, 1) * 8));
         TRY(run->cnt.alloc(sizeof(DevCounters)));
-        TRY(run->qctl.alloc(sizeof(WaveCtl)));
+        TRY(run->qctl.alloc(kMaxPipes * kCtlStride));
         for (DevMem *m : {&run->hE, &run->hP, &run->hDp, &run->hDn, &run->hAn, &run->cnt, &run->qctl})
             TRY(cudaMemsetAsync(m->p, 0, m->bytes, stream));
         if (e) break;
@@ -616,20 +639,6 @@ void run_worker_body(pach_run *run) {
         TRY(upload(run->dsrc, src.data(), src.size() * sizeof(float4)));
         TRY(upload(run->de0, e0.data(), e0.size() * sizeof(float)));
         TRY(upload(run->droom, rp.data(), rp.size() * sizeof(RoomParams)));
-        if (n_rooms > 1) {  // the batch's feed order (DevRun::sched_off, sched_prim), then its live counts and peaks
-            std::vector<long long> sched(5 * (size_t)n_rooms + 1, 0);
-            long long *off = sched.data(), *prim = off + 2 * n_rooms + 1;
-            long long q = rprim[0];
-            for (int k = 0; k < 2 * n_rooms; ++k) {
-                const RoomSpec &rm = run->rooms[(size_t)(k % n_rooms)];
-                const long long pilot = std::min(rm.rays, kPilotPrimaries);
-                off[k] = q;
-                prim[k] = rm.prim_begin + (k < n_rooms ? 0 : pilot);
-                q += k < n_rooms ? pilot : rm.rays - pilot;
-            }
-            off[2 * n_rooms] = q;
-            TRY(upload(run->dsched, sched.data(), sched.size() * sizeof(long long)));
-        }
         std::vector<double> gf;
         geodesic_faces(gf);
         std::vector<float4> geo(kGeoFaces * 3);
@@ -685,7 +694,6 @@ void run_worker_body(pach_run *run) {
         const bool bounce = fused && !map;
         const bool by_planes = bounce && *std::min_element(planes.begin(), planes.end()) > 0;
         if (bounce) TRY(bounce_occupancy(threads, receiver_smem_bytes(R), &bps_sh, by_planes));
-        const int tr_blocks = dev_sms * std::max(bps_tr, 1), sh_blocks = dev_sms * std::max(bps_sh, 1);
 
         // ring and wave sizing
         // default ring: room for the run's rays at up to 2048 live octave rays per primary, 2^22..2^28
@@ -694,9 +702,31 @@ void run_worker_body(pach_run *run) {
         // a batch's pilots run several rooms at a time, and rays of small scenes leave several children a wave
         int ring_default = n_rooms > 1 || bounce ? kRingMin : 22;
         while (ring_default < 28 && (1ull << ring_default) < (unsigned long long)rprim_total(run) * 2048ull) ++ring_default;
+        const bool sorting = run->p.ray_sort > 0;
+        const bool timing = run->p.kernel_timing != 0;
+        const bool conv_mode = run->conv_mode >= 0;
+        // Pipes: the primaries are shared out to independent device loops on streams of their own, so that the ends of
+        // one's waves (60 us in which the last rays finish, of the 150 to 550 us of an iteration) and its launches
+        // overlap the others' work.  Device time with 1 / 2 / 3 / 4 loops: hall of 20k triangles, 2500 primaries and
+        // an audience map 46.8 / 45.0 / 42.3 / 43.5 ms; 20k primaries 145 / 143.5 / 142.5 / 140.9; arena of 500k
+        // triangles, 60k primaries 95 / 91.5 / 91.3 / 91.1; 8 small rooms of 500 primaries 287 / - / 248 / -.  Below a
+        // pilot's size there is one wave front to share and more loops only split it (hall, 128 primaries: 8.7 ms with
+        // one, 9.2 with two; 300: 13.6, 9.7, with three 9.3).  Runs that the caller shapes (ring, feed, sorted
+        // waves, kernel times) and convergence runs, whose revolutions are smaller, keep one.
+        const long long N = rprim[n_rooms] - rprim[0];
+        P = timing || conv_mode || sorting || run->p.ring_log2 > 0 || run->p.feed_batch > 0 || N <= kPilotPrimaries ? 1 : kPipes;
         const int ring_log2 = run->p.ring_log2 > 0 ? std::min(32, std::max(16, run->p.ring_log2)) : ring_default;
-        const unsigned long long ring_cap = 1ull << ring_log2;
-        const unsigned long long max_wave = run->p.wave_kilo_items > 0 ? 1024ull * run->p.wave_kilo_items : (1ull << 23);
+        // A loop's ring is a quarter of the whole one, but no less than what keeps its waves full (a batch's pilots run
+        // several rooms at a time: 8 rooms of 500 primaries 258 ms with 2^22 rays, 248 with 2^23, 257 with 2^24).
+        const int pipe_log2 = std::max(n_rooms > 1 ? 23 : 22, ring_log2 - 2);
+        if (bound * 4 > (1ull << pipe_log2)) P = 1;
+        unsigned long long ring_cap = 1ull << (P > 1 ? pipe_log2 : ring_log2);
+        const unsigned long long max_wave =
+            run->p.wave_kilo_items > 0 ? 1024ull * run->p.wave_kilo_items : (1ull << (P > 1 ? 22 : 23));
+        // Half the blocks that fit for each trace kernel: the loops' kernels run side by side instead of one after the
+        // other (three loops, all blocks / half: hall with the map 44.3 / 42.3 ms, 20k primaries 148.4 / 142.5).
+        const int tr_blocks = dev_sms * (P > 1 ? (std::max(bps_tr, 1) + 1) / 2 : std::max(bps_tr, 1));
+        const int sh_blocks = dev_sms * std::max(bps_sh, 1);
         if (bound * 4 > ring_cap) {
             status = PACH_ERR_BOUNDS;
             msg = "the ring queue (2^" + std::to_string(ring_log2) + " rays) cannot hold the phase-A output of one "
@@ -704,32 +734,32 @@ void run_worker_body(pach_run *run) {
             final_state = PACH_RUN_FAILED;
             break;
         }
-        TRY(run->qa.alloc(ring_cap * sizeof(ORayItem)));
-        TRY(run->qs0.alloc(std::min(max_wave, ring_cap) * sizeof(int4)));
-        const bool sorting = run->p.ray_sort > 0;
+        if (P > 1 && (run->qa.alloc(P * ring_cap * sizeof(ORayItem)) || run->qs0.alloc(P * std::min(max_wave, ring_cap) * sizeof(int4)))) {
+            cudaGetLastError();  // memory for one ring may be left
+            run->qs0.release();
+            P = 1;
+            ring_cap = 1ull << ring_log2;
+        }
+        if (P == 1) {
+            TRY(run->qa.alloc(ring_cap * sizeof(ORayItem)));
+            TRY(run->qs0.alloc(std::min(max_wave, ring_cap) * sizeof(int4)));
+        }
         if (sorting) {
             TRY(run->qs1.alloc(std::min(max_wave, ring_cap) * sizeof(ORayItem)));
             TRY(run->sortbins.alloc(2 * kSortBins * sizeof(unsigned)));
             TRY(cudaMemsetAsync(run->sortbins.p, 0, run->sortbins.bytes, stream));
         }
         const int sort_blocks = dev_sms * 4;
-        const bool timing = run->p.kernel_timing != 0;
         if (!timing) {
-            TRY(cudaHostAlloc(&h_mirror, sizeof(HostMirror), cudaHostAllocMapped));
+            TRY(cudaHostAlloc(&h_mirror, kMaxPipes * sizeof(HostMirror), cudaHostAllocMapped));
             TRY(cudaHostAlloc(&h_cancel, sizeof(int), cudaHostAllocMapped));
-            std::memset(h_mirror, 0, sizeof(HostMirror));
+            std::memset(h_mirror, 0, kMaxPipes * sizeof(HostMirror));
             *h_cancel = 0;
         }
 
         DevRun r{};
         r.S = S;
         r.rooms = run->droom.as<RoomParams>();
-        if (n_rooms > 1) {
-            r.sched_off = run->dsched.as<long long>();
-            r.sched_prim = r.sched_off + 2 * n_rooms + 1;
-            r.room_live = reinterpret_cast<unsigned *>(run->dsched.as<long long>() + 4 * n_rooms + 1);
-            r.room_peak = r.room_live + n_rooms;
-        }
         r.n_rooms = n_rooms;
         r.rec = run->drec.as<float4>();
         r.rec_id = run->drecid.as<int>();
@@ -786,7 +816,7 @@ void run_worker_body(pach_run *run) {
         if (!timing) {
             void *dp = nullptr;
             TRY(cudaHostGetDevicePointer(&dp, h_mirror, 0));
-            r.mirror = reinterpret_cast<HostMirror *>(dp);
+            r.mirror = reinterpret_cast<HostMirror *>(dp);  // pipe 0's
             TRY(cudaHostGetDevicePointer(&dp, h_cancel, 0));
             r.cancel = reinterpret_cast<volatile int *>(dp);
         }
@@ -794,10 +824,6 @@ void run_worker_body(pach_run *run) {
         r.hE = run->hE.as<double>(); r.hP = run->hP.as<double>(); r.hDp = run->hDp.as<double>();
         r.hDn = run->hDn.as<double>(); r.hAn = run->hAn.as<double>();
         r.cnt = run->cnt.as<DevCounters>();
-        r.ring = run->qa.as<ORayItem>();
-        r.ring_cap = ring_cap;
-        r.ctl = run->qctl.as<WaveCtl>();
-        r.hits = run->qs0.as<int4>();
         r.wave_buf = sorting ? run->qs1.as<ORayItem>() : nullptr;
         r.bin_count = sorting ? run->sortbins.as<unsigned>() : nullptr;
         r.bin_cursor = sorting ? run->sortbins.as<unsigned>() + kSortBins : nullptr;
@@ -805,22 +831,18 @@ void run_worker_body(pach_run *run) {
             r.sort_lo[k] = (float)bmin[k];
             r.sort_inv[k] = (float)(kSortGrid / std::max(bmax[k] - bmin[k], 1e-9));
         }
-        r.max_wave = std::min(max_wave, ring_cap);
         r.max_bounces = bounce ? kMaxBounces : 1;
         r.full_wave = kFullFactor * (unsigned long long)sh_blocks * threads;
         r.feed_bound = bound;
-        r.low_water = std::min(ring_cap / 4, 2 * r.max_wave);
-        const long long N = rprim[n_rooms] - rprim[0];
-        const long long fb_default = std::max<long long>(4096, (long long)(r.max_wave / 32));
+        const long long fb_default = std::max<long long>(4096, (long long)(std::min(max_wave, ring_cap) / 32));
         r.feed_batch = run->p.feed_batch > 0 ? run->p.feed_batch : fb_default;
         const int bb_threads = 128;
         const int bb_blocks = (int)std::max<long long>(1, std::min<long long>((r.feed_batch + bb_threads - 1) / bb_threads,
                                                                               (long long)dev_sms * 8));
-        std::memset(h_ctl, 0, sizeof(WaveCtl));
+        std::memset(h_ctl, 0, kMaxPipes * sizeof(WaveCtl));
         double t_trace = 0, t_shade = 0, t_bb = 0, t_sort = 0;
         long long launches = 0;
         bool cancelled = false;
-        const bool conv_mode = run->conv_mode >= 0;
         if (conv_mode) {
             // per-revolution capture of the check receivers, and a copy of the histograms and counters
             // taken before each chunk (restored when the checks agree inside a chunk)
@@ -835,8 +857,10 @@ void run_worker_body(pach_run *run) {
             for (int i = 0; i < 6; ++i) TRY(run->bak[i].alloc(src_[i]->bytes));
             if (e) break;
         }
-        auto one_iteration = [&](int k) -> cudaError_t {
+        auto one_iteration = [&](const Pipe &q, int k) -> cudaError_t {
             cudaError_t x;
+            const DevRun &r = q.r;
+            const cudaStream_t stream = q.stream;
             if (timing && (x = launch_feed(r, stream))) return x;  // graph mode: k_cond feeds
             if (timing && (x = cudaEventRecord(kev[6 * k], stream))) return x;
             if ((x = launch_broadband(r, bb_blocks, bb_threads, stream, map, ntri_max <= kFuseMaxTris))) return x;
@@ -852,37 +876,87 @@ void run_worker_body(pach_run *run) {
             if (timing && (x = cudaEventRecord(kev[6 * k + 5], stream))) return x;
             return cudaSuccess;
         };
-        if (!timing) {
-            // the whole loop as one graph launch: feed, then while (k_cond says so) { one iteration }
-            TRY(cudaGraphCreate(&graph, 0));
-            TRY(cudaStreamBeginCaptureToGraph(stream, graph, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-            cudaError_t fe = launch_feed(r, stream);
+        // the whole loop of a pipe as one graph launch: feed, then while (k_cond says so) { one iteration }
+        auto make_graph = [&](Pipe &q) -> cudaError_t {
+            cudaError_t x;
+            if ((x = cudaGraphCreate(&q.graph, 0))) return x;
+            if ((x = cudaStreamBeginCaptureToGraph(q.stream, q.graph, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal)))
+                return x;
+            const cudaError_t fe = launch_feed(q.r, q.stream);
             cudaGraph_t fed = nullptr;
-            cudaError_t fc = cudaStreamEndCapture(stream, &fed);
-            TRY(fe);
-            TRY(fc);
+            const cudaError_t fc = cudaStreamEndCapture(q.stream, &fed);
+            if (fe || fc) return fe ? fe : fc;
             size_t n_first = 1;
-            cudaGraphNode_t first;
-            TRY(cudaGraphGetNodes(graph, &first, &n_first));
+            cudaGraphNode_t first, node;
+            if ((x = cudaGraphGetNodes(q.graph, &first, &n_first))) return x;
             cudaGraphConditionalHandle handle;
-            TRY(cudaGraphConditionalHandleCreate(&handle, graph, 1, cudaGraphCondAssignDefault));
+            if ((x = cudaGraphConditionalHandleCreate(&handle, q.graph, 1, cudaGraphCondAssignDefault))) return x;
             cudaGraphNodeParams cp{};
             cp.type = cudaGraphNodeTypeConditional;
             cp.conditional.handle = handle;
             cp.conditional.type = cudaGraphCondTypeWhile;
             cp.conditional.size = 1;
-            cudaGraphNode_t node;
-            TRY(cudaGraphAddNode(&node, graph, &first, nullptr, 1, &cp));
-            cudaGraph_t body = cp.conditional.phGraph_out[0];
-            TRY(cudaStreamBeginCaptureToGraph(stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-            cudaError_t ce = one_iteration(0);
-            if (ce == cudaSuccess) ce = launch_cond(r, handle, stream);
+            if ((x = cudaGraphAddNode(&node, q.graph, &first, nullptr, 1, &cp))) return x;
+            if ((x = cudaStreamBeginCaptureToGraph(q.stream, cp.conditional.phGraph_out[0], nullptr, nullptr, 0,
+                                                   cudaStreamCaptureModeThreadLocal)))
+                return x;
+            cudaError_t ce = one_iteration(q, 0);
+            if (ce == cudaSuccess) ce = launch_cond(q.r, handle, q.stream);
             cudaGraph_t captured = nullptr;
-            cudaError_t ee = cudaStreamEndCapture(stream, &captured);
-            TRY(ce);
-            TRY(ee);
-            TRY(cudaGraphInstantiate(&gexec, graph, 0));
-        }
+            const cudaError_t ee = cudaStreamEndCapture(q.stream, &captured);
+            if (ce || ee) return ce ? ce : ee;
+            return cudaGraphInstantiate(&q.exec, q.graph, 0);
+        };
+        // sets up P pipes of ring_cap rays each in the run's buffers
+        auto make_pipes = [&]() -> cudaError_t {
+            cudaError_t x;
+            const int n = n_rooms;
+            if (n > 1) {  // each pipe's feed order (DevRun::sched_off, sched_prim), then its live counts and peaks
+                const size_t each = 5 * (size_t)n + 1;
+                std::vector<long long> sched(each * P, 0);
+                for (int k = 0; k < P; ++k) {
+                    long long *off = sched.data() + each * k, *prim = off + 2 * n + 1, q = rprim[0];
+                    for (int g = 0; g < 2 * n; ++g) {
+                        const RoomSpec &rm = run->rooms[(size_t)(g % n)];
+                        const long long first = share(rm.rays, k, P), part = share(rm.rays, k + 1, P) - first;
+                        const long long pilot = std::min(part, kPilotPrimaries);
+                        off[g] = q;
+                        prim[g] = rm.prim_begin + first + (g < n ? 0 : pilot);
+                        q += g < n ? pilot : part - pilot;
+                    }
+                    off[2 * n] = q;
+                }
+                if ((x = upload(run->dsched, sched.data(), sched.size() * sizeof(long long)))) return x;
+            }
+            for (int k = 0; k < P; ++k) {
+                Pipe &q = pipes[k];
+                if (k == 0) q.stream = stream;
+                else if (!q.stream && (x = cudaStreamCreateWithFlags(&q.stream, cudaStreamNonBlocking))) return x;
+                if (!q.end && (x = cudaEventCreate(&q.end))) return x;
+                q.r = r;
+                if (q.r.mirror) q.r.mirror += k;
+                q.r.ring = run->qa.as<ORayItem>() + k * ring_cap;
+                q.r.ring_cap = ring_cap;
+                q.r.ctl = reinterpret_cast<WaveCtl *>(run->qctl.as<char>() + k * kCtlStride);
+                q.r.max_wave = std::min(max_wave, ring_cap);
+                q.r.hits = run->qs0.as<int4>() + k * q.r.max_wave;
+                q.r.low_water = std::min(ring_cap / 4, 2 * q.r.max_wave);
+                if (n > 1) {
+                    const long long *at = run->dsched.as<long long>() + (5 * (size_t)n + 1) * k;
+                    q.r.sched_off = at;
+                    q.r.sched_prim = at + 2 * n + 1;
+                    q.r.room_live = reinterpret_cast<unsigned *>(const_cast<long long *>(at) + 4 * n + 1);
+                    q.r.room_peak = q.r.room_live + n;
+                }
+                if (q.exec) cudaGraphExecDestroy(q.exec);
+                if (q.graph) cudaGraphDestroy(q.graph);
+                q.exec = nullptr;
+                q.graph = nullptr;
+                if (!timing && (x = make_graph(q))) return x;
+            }
+            return cudaSuccess;
+        };
+        TRY(make_pipes());
         double dev_ms_total = 0;
         long long done_before = 0;  // primaries of the ranges already run (progress offset)
         // Runs the device loop over primaries [p0, p1): the graph launch (progress and cancellation through
@@ -895,41 +969,70 @@ void run_worker_body(pach_run *run) {
     }
         auto run_range = [&](long long p0, long long p1) -> cudaError_t {
             // the schedule starts afresh; the pilots' per-primary ring footprint carries over
-            const unsigned long long per_prim = h_ctl->per_prim;
-            const int pilot_room = h_ctl->pilot_room;
-            std::memset(h_ctl, 0, sizeof(WaveCtl));
-            h_ctl->next_prim = p0;
-            h_ctl->prim_end = p1;
-            h_ctl->prim_first = p0;
-            h_ctl->per_prim = per_prim;
-            h_ctl->pilot_room = pilot_room;
-            RTRY(cudaMemcpyAsync(run->qctl.p, h_ctl, sizeof(WaveCtl), cudaMemcpyHostToDevice, stream));
+            for (int k = 0; k < P; ++k) {
+                WaveCtl &c = h_ctl[k];
+                const unsigned long long per_prim = c.per_prim;
+                const int pilot_room = c.pilot_room;
+                std::memset(&c, 0, sizeof(WaveCtl));
+                long long a = p0 + share(p1 - p0, k, P), b = p0 + share(p1 - p0, k + 1, P);
+                if (n_rooms > 1) {  // positions of the pipe's own feed order
+                    a = b = p0;
+                    for (const RoomSpec &rm : run->rooms) b += share(rm.rays, k + 1, P) - share(rm.rays, k, P);
+                }
+                c.next_prim = a;
+                c.prim_end = b;
+                c.prim_first = p0;
+                c.per_prim = per_prim;
+                c.pilot_room = pilot_room;
+                pipes[k].p0 = a;
+                RTRY(cudaMemcpyAsync(pipes[k].r.ctl, &c, sizeof(WaveCtl), cudaMemcpyHostToDevice, stream));
+            }
+            float ms = 0.f;
             if (!timing) {
                 *reinterpret_cast<volatile int *>(h_cancel) = 0;
-                std::memset(h_mirror, 0, sizeof(HostMirror));
-                h_mirror->next_prim = p0;
-                // device time of the loop alone: the host's graph construction is not inside the events
+                std::memset(h_mirror, 0, kMaxPipes * sizeof(HostMirror));
+                for (int k = 0; k < P; ++k) h_mirror[k].next_prim = pipes[k].p0;
+                // device time of the loops alone: the host's graph construction is not inside the events
                 RTRY(cudaEventRecord(ev0, stream));
-                RTRY(cudaGraphLaunch(gexec, stream));
-                RTRY(cudaEventRecord(ev1, stream));
-                // poll: progress from the mapped mirror, cancellation through the mapped flag (1: stop
-                // feeding; 2, two seconds later: stop the loop without waiting for the fed primaries)
-                auto t_cancel = std::chrono::steady_clock::now();
+                for (int k = 0; k < P; ++k) {
+                    if (k) RTRY(cudaStreamWaitEvent(pipes[k].stream, ev0, 0));
+                    RTRY(cudaGraphLaunch(pipes[k].exec, pipes[k].stream));
+                    RTRY(cudaEventRecord(pipes[k].end, pipes[k].stream));
+                }
+                // poll: progress from the mapped mirrors, cancellation through the mapped flag (1: stop
+                // feeding; 2, two seconds later: stop the loops without waiting for the fed primaries)
+                const auto t_start = std::chrono::steady_clock::now();
+                auto t_cancel = t_start;
                 for (;;) {
-                    const cudaError_t q = cudaEventQuery(ev1);
-                    run->rays_done = done_before + std::max(0ll, (long long)h_mirror->next_prim - p0);
-                    run->end_traces = (long long)h_mirror->end_traces;
-                    run->segments = (long long)h_mirror->segments;
+                    cudaError_t q = cudaSuccess;
+                    long long fed = 0;
+                    unsigned long long ended = 0;
+                    for (int k = 0; k < P; ++k) {
+                        if (q == cudaSuccess) q = cudaEventQuery(pipes[k].end);
+                        fed += std::max(0ll, (long long)h_mirror[k].next_prim - pipes[k].p0);
+                        ended = std::max(ended, (unsigned long long)h_mirror[k].end_traces);
+                        run->segments = std::max<long long>(run->segments, (long long)h_mirror[k].segments);
+                    }
+                    run->rays_done = done_before + fed;
+                    run->end_traces = (long long)ended;
                     if (q == cudaSuccess) break;
                     if (q != cudaErrorNotReady) { where = "graph run"; return q; }
+                    const auto now = std::chrono::steady_clock::now();
                     if (run->cancel && !cancelled) {
                         cancelled = true;
-                        t_cancel = std::chrono::steady_clock::now();
+                        t_cancel = now;
                         *reinterpret_cast<volatile int *>(h_cancel) = 1;
-                    } else if (cancelled && std::chrono::steady_clock::now() - t_cancel > std::chrono::seconds(2)) {
+                    } else if (cancelled && now - t_cancel > std::chrono::seconds(2)) {
                         *reinterpret_cast<volatile int *>(h_cancel) = 2;
                     }
-                    std::this_thread::sleep_for(std::chrono::microseconds(500));
+                    // short runs should not wait half a millisecond for their end to be seen
+                    std::this_thread::sleep_for(std::chrono::microseconds(now - t_start < std::chrono::milliseconds(50) ? 50 : 500));
+                }
+                for (int k = 0; k < P; ++k) {
+                    float t = 0.f;
+                    RTRY(cudaStreamSynchronize(pipes[k].stream));
+                    RTRY(cudaEventElapsedTime(&t, ev0, pipes[k].end));
+                    ms = std::max(ms, t);
                 }
             } else {
                 RTRY(cudaEventRecord(ev0, stream));
@@ -942,7 +1045,7 @@ void run_worker_body(pach_run *run) {
                         kev.push_back(x);
                     }
                     for (int k = 0; k < batch; ++k, ++it) {
-                        RTRY(one_iteration(k));
+                        RTRY(one_iteration(pipes[0], k));
                         launches += (sorting ? 7 : 4) - (fused ? 1 : 0);
                     }
                     RTRY(cudaMemcpyAsync(h_ctl, run->qctl.p, sizeof(WaveCtl), cudaMemcpyDeviceToHost, stream));
@@ -982,17 +1085,34 @@ void run_worker_body(pach_run *run) {
                     }
                 }
                 RTRY(cudaEventRecord(ev1, stream));
+                RTRY(cudaStreamSynchronize(stream));
+                RTRY(cudaEventElapsedTime(&ms, ev0, ev1));
             }
-            RTRY(cudaStreamSynchronize(stream));
-            float ms = 0.f;
-            RTRY(cudaEventElapsedTime(&ms, ev0, ev1));
             dev_ms_total += ms;
-            RTRY(cudaMemcpy(h_ctl, run->qctl.p, sizeof(WaveCtl), cudaMemcpyDeviceToHost));
+            for (int k = 0; k < P; ++k) RTRY(cudaMemcpy(&h_ctl[k], pipes[k].r.ctl, sizeof(WaveCtl), cudaMemcpyDeviceToHost));
             return cudaSuccess;
         };
 #undef RTRY
         if (!conv_mode) {
             if ((e = run_range(rprim[0], rprim[0] + N)) != cudaSuccess || status) break;
+            bool full = false;
+            for (int k = 0; k < P; ++k) full = full || h_ctl[k].overflow;
+            if (full && P > 1 && !cancelled) {
+                // a pipe's ring was too small: once more from nothing, as one loop in the ring that one loop gets
+                for (DevMem *m : {&run->hE, &run->hP, &run->hDp, &run->hDn, &run->hAn, &run->cnt, &run->qctl, &run->dcap, &run->mE,
+                                  &run->mP, &run->mDp, &run->mDn})
+                    if (m->p) TRY(cudaMemsetAsync(m->p, 0, m->bytes, stream));
+                if (e) break;
+                P = 1;
+                ring_cap = 1ull << ring_log2;
+                TRY(run->qa.alloc(ring_cap * sizeof(ORayItem)));
+                TRY(run->qs0.alloc(std::min(max_wave, ring_cap) * sizeof(int4)));
+                if (e) break;
+                run->segments = run->end_traces = 0;
+                std::memset(h_ctl, 0, kMaxPipes * sizeof(WaveCtl));
+                TRY(make_pipes());
+                if ((e = run_range(rprim[0], rprim[0] + N)) != cudaSuccess || status) break;
+            }
         } else {
             // Convergence mode (TaskAll:300-330): revolutions of conv_period primaries until every check
             // agrees.  Chunks of revolutions run as one device loop that also records each revolution's
@@ -1056,7 +1176,18 @@ void run_worker_body(pach_run *run) {
         }
         const float dev_ms = (float)dev_ms_total;
         TRY(cudaMemcpy(h_cnt, run->cnt.p, sizeof(DevCounters), cudaMemcpyDeviceToHost));
-        TRY(cudaMemcpy(h_ctl, run->qctl.p, sizeof(WaveCtl), cudaMemcpyDeviceToHost));
+        // the pipes' schedules as one: their sums, and the worst of their ends
+        WaveCtl all = h_ctl[0];
+        run->pipes = P;
+        run->pipe_done[0] = h_ctl[0].next_prim - pipes[0].p0;
+        for (int k = 1; k < P; ++k) {
+            all.overflow += h_ctl[k].overflow;
+            all.waves += h_ctl[k].waves;
+            all.iters += h_ctl[k].iters;
+            all.peak_live += h_ctl[k].peak_live;
+            all.gave_up = std::max(all.gave_up, h_ctl[k].gave_up);
+            run->pipe_done[k] = h_ctl[k].next_prim - pipes[k].p0;
+        }
         const HostScene &hs = sc->hs;
         pach_stats &s = run->stats;
         s.primaries = (int64_t)h_cnt->primaries;
@@ -1069,7 +1200,7 @@ void run_worker_body(pach_run *run) {
         s.detections = (int64_t)h_cnt->detections;
         s.capped = (int64_t)h_cnt->capped;
         s.fp64_retests = (int64_t)h_cnt->retests;
-        s.queue_overflows = (int64_t)h_ctl->overflow;
+        s.queue_overflows = (int64_t)all.overflow;
         s.stack_spills = 0;
         s.lost_energy = h_cnt->lost_energy;
         s.initial_energy = h_cnt->initial_energy;
@@ -1085,9 +1216,9 @@ void run_worker_body(pach_run *run) {
         s.shade_ms = t_shade;
         s.broadband_ms = t_bb;
         s.sort_ms = t_sort;
-        s.waves = (int64_t)h_ctl->waves;
-        s.kernel_launches = timing ? launches : 1 + (long long)h_ctl->iters * ((sorting ? 7 : 4) - (fused ? 1 : 0));
-        s.peak_live_rays = (int64_t)h_ctl->peak_live;
+        s.waves = (int64_t)all.waves;
+        s.kernel_launches = timing ? launches : P + (long long)all.iters * ((sorting ? 7 : 4) - (fused ? 1 : 0));
+        s.peak_live_rays = (int64_t)all.peak_live;
         s.bvh_nodes_visited = (int64_t)h_cnt->bvh_nodes;
         s.tri_tests = (int64_t)h_cnt->tri_tests;
         s.accel[0] = (int32_t)(n_rooms > 1 ? run->bbvh.bytes / (kBvhNodeFloats * sizeof(float)) : hs.bvh_nodes);
@@ -1101,15 +1232,15 @@ void run_worker_body(pach_run *run) {
         run->rays_done = (long long)h_cnt->primaries;
         run->segments = s.segments;
         run->end_traces = s.end_traces;
-        if (h_ctl->overflow) {
+        if (all.overflow) {
             status = PACH_ERR_BOUNDS;
             msg = "ring queue full: raise ring_log2";
             final_state = PACH_RUN_FAILED;
-        } else if (h_ctl->gave_up == 2) {
+        } else if (all.gave_up == 2) {
             status = PACH_ERR_CANCELLED;
             msg = "run cancelled; the loop stopped before every fed primary finished";
             final_state = PACH_RUN_CANCELLED;
-        } else if (h_ctl->gave_up) {
+        } else if (all.gave_up) {
             status = PACH_ERR_GAVE_UP;
             msg = "wavefront loop stopped without finishing (iteration cap or no progress)";
             final_state = PACH_RUN_FAILED;
@@ -1121,8 +1252,14 @@ void run_worker_body(pach_run *run) {
 #undef TRY
     } while (0);
     run->stats.wall_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - wall0).count();
-    if (gexec) cudaGraphExecDestroy(gexec);
-    if (graph) cudaGraphDestroy(graph);
+    if (h_cancel && (e || status)) *reinterpret_cast<volatile int *>(h_cancel) = 2;  // no loop outlives the run
+    for (Pipe &q : pipes) {
+        if (q.stream) cudaStreamSynchronize(q.stream);
+        if (q.exec) cudaGraphExecDestroy(q.exec);
+        if (q.graph) cudaGraphDestroy(q.graph);
+        if (q.end) cudaEventDestroy(q.end);
+        if (q.stream && q.stream != stream) cudaStreamDestroy(q.stream);
+    }
     for (cudaEvent_t ev : kev) cudaEventDestroy(ev);
     for (cudaEvent_t ev : {ev0, ev1})
         if (ev) cudaEventDestroy(ev);

@@ -88,7 +88,7 @@ __device__ bool pilots_measured(const DevRun &r, WaveCtl *c, unsigned long long 
         const unsigned peak = r.room_peak[i], now = r.room_live[i];
         ok = ok && (now == 0 || now <= peak - peak / 8);
         const long long n = g1 - g0 == 1 ? c->pilot_count : r.sched_off[i + 1] - r.sched_off[i];
-        const unsigned long long v = (unsigned long long)peak * 3 / (unsigned long long)n + 1;
+        const unsigned long long v = (unsigned long long)peak * 3 / (unsigned long long)max(n, 1ll) + 1;
         if (v > best) best = v;
     }
     if (!__all_sync(FULL, ok)) return false;
@@ -140,6 +140,10 @@ __device__ void feed_step(const DevRun &r) {
     if (fit > (unsigned long long)r.feed_batch) fit = (unsigned long long)r.feed_batch;
     if (fit > (unsigned long long)(prim_end - next)) fit = (unsigned long long)(prim_end - next);
     long long lim = prim_end - next;
+    // rooms without a primary in this schedule have no pilot
+    while (r.n_rooms > 1 && c->pilot_room < r.n_rooms &&
+           __ldg(r.sched_off + c->pilot_room + 1) == __ldg(r.sched_off + c->pilot_room))
+        ++c->pilot_room;
     if (c->pilot_room < r.n_rooms) {
         // a batch never reaches into a pilot that has not run
         const long long first = r.n_rooms == 1 ? next : __ldg(r.sched_off + c->pilot_room);

@@ -189,3 +189,43 @@ def test_rays_kept_over_interactions_equal_one_walk_per_launch(kind, ring_log2, 
     assert sa["segments"] == sb["segments"] and sa["detections"] == sb["detections"] and sa["queue_overflows"] == 0
     for name in ("energy", "pressure", "dir_pos", "dir_neg", "analysis"):
         np.testing.assert_allclose(ha[name], hb[name], rtol=1e-9, atol=1e-30, err_msg=name)
+
+
+@pytest.mark.parametrize("kind", ["hall", "map", "capture", "batch"])
+@pytest.mark.parametrize("rays", [256, 257, 1001])
+def test_primaries_shared_out_to_several_loops_equal_one_loop(kind, rays):
+    """Above 256 primaries a run is shared out to loops with rings of their own; a given feed size keeps one.  The
+    same rays, so the same terms in every bin (FP64 sums in another order: 1e-9; a primary's captures are FP32 sums
+    of at most a thousand detections: 2 x 1000 x 2^-24)."""
+    if kind == "batch":
+        ws = [rooms.proposal_room_c4(20 + i) for i in range(4)]
+        n = [rays, 1, rays // 2, 2]
+    else:
+        ws = [rooms.irregular_hall_c2(target_tris=2000)]
+    kw = {}
+    if kind == "map":
+        lo, hi = ws[0].scene.bounds()
+        org = rooms.audience_plane(lo[:2] + 2.0, hi[:2] - 2.0, 1.2, 2.0)
+        kw["map_receivers"] = tracer.MapReceivers(org, 2.0, 400.0)
+    elif kind == "capture":
+        kw["capture"] = 2
+    for w in ws:
+        w.cutoff_s = 0.4
+    ds = [tracer.DeviceScene(w.scene) for w in ws]
+    got = []
+    for feed in (0, 64):
+        if kind == "batch":
+            got.append(tracer.trace_batch(ws, dscenes=ds, rays=n, seed=6, feed_batch=feed))
+        else:
+            h, s = tracer.trace(ws[0], dscene=ds[0], rays=rays, seed=6, feed_batch=feed, **kw)
+            got.append(([{**h, **{"map " + k: v for k, v in h.get("map", {}).items()}}], s))
+    (ha, sa), (hb, sb) = got
+    for name in ("primaries", "segments", "octave_rays", "end_traces", "detections", "queue_overflows"):
+        assert sa[name] == sb[name], name
+    assert sa["segments"] > 0 and sa["queue_overflows"] == 0
+    for a, b in zip(ha, hb):
+        assert "map energy" in a or kind != "map"
+        for name, x in a.items():
+            if isinstance(x, np.ndarray):
+                rtol = 1.2e-4 if name == "capture" else 1e-9
+                np.testing.assert_allclose(x, b[name], rtol=rtol, atol=1e-30, err_msg=name)
