@@ -509,6 +509,8 @@ void run_worker_body(pach_run *run) {
     struct Pipe {
         cudaStream_t stream = nullptr;
         cudaEvent_t end = nullptr;
+        cudaStream_t side = nullptr;  // captured into the graph only
+        cudaEvent_t fork = nullptr, join = nullptr;
         cudaGraph_t graph = nullptr;
         cudaGraphExec_t exec = nullptr;
         DevRun r{};
@@ -727,6 +729,7 @@ void run_worker_body(pach_run *run) {
         // other (three loops, all blocks / half: hall with the map 44.3 / 42.3 ms, 20k primaries 148.4 / 142.5).
         const int tr_blocks = dev_sms * (P > 1 ? (std::max(bps_tr, 1) + 1) / 2 : std::max(bps_tr, 1));
         const int sh_blocks = dev_sms * std::max(bps_sh, 1);
+        const int map_blocks = dev_sms * kMapBlocks;
         if (bound * 4 > ring_cap) {
             status = PACH_ERR_BOUNDS;
             msg = "the ring queue (2^" + std::to_string(ring_log2) + " rays) cannot hold the phase-A output of one "
@@ -870,9 +873,20 @@ void run_worker_body(pach_run *run) {
             if (timing && (x = cudaEventRecord(kev[6 * k + 3], stream))) return x;
             if (!fused && (x = launch_trace(r, tr_variant, tr_blocks, threads, stream))) return x;
             if (timing && (x = cudaEventRecord(kev[6 * k + 4], stream))) return x;
+            // the map's kernel only reads the wave: beside the shading kernel, unless that finds the hits or is timed
+            const bool beside = map && !fused && !timing;
+            if (beside) {
+                if ((x = cudaEventRecord(q.fork, stream))) return x;
+                if ((x = cudaStreamWaitEvent(q.side, q.fork, 0))) return x;
+                if ((x = launch_map(r, map_blocks, q.side))) return x;
+                if ((x = cudaEventRecord(q.join, q.side))) return x;
+            }
             if ((x = bounce ? launch_bounce(r, sh_blocks, threads, stream, by_planes)
-                            : launch_shade(r, sh_blocks, threads, stream, fused, map, wide)))
+                            : launch_shade(r, sh_blocks, threads, stream, fused, wide)))
                 return x;
+            if (beside) x = cudaStreamWaitEvent(stream, q.join, 0);
+            else if (map) x = launch_map(r, map_blocks, stream);
+            if (x) return x;
             if (timing && (x = cudaEventRecord(kev[6 * k + 5], stream))) return x;
             return cudaSuccess;
         };
@@ -933,6 +947,11 @@ void run_worker_body(pach_run *run) {
                 if (k == 0) q.stream = stream;
                 else if (!q.stream && (x = cudaStreamCreateWithFlags(&q.stream, cudaStreamNonBlocking))) return x;
                 if (!q.end && (x = cudaEventCreate(&q.end))) return x;
+                if (map && !q.side) {
+                    if ((x = cudaStreamCreateWithFlags(&q.side, cudaStreamNonBlocking))) return x;
+                    for (cudaEvent_t *ev : {&q.fork, &q.join})
+                        if ((x = cudaEventCreateWithFlags(ev, cudaEventDisableTiming))) return x;
+                }
                 q.r = r;
                 if (q.r.mirror) q.r.mirror += k;
                 q.r.ring = run->qa.as<ORayItem>() + k * ring_cap;
@@ -1046,7 +1065,7 @@ void run_worker_body(pach_run *run) {
                     }
                     for (int k = 0; k < batch; ++k, ++it) {
                         RTRY(one_iteration(pipes[0], k));
-                        launches += (sorting ? 7 : 4) - (fused ? 1 : 0);
+                        launches += (sorting ? 7 : 4) - (fused ? 1 : 0) + (map ? 1 : 0);
                     }
                     RTRY(cudaMemcpyAsync(h_ctl, run->qctl.p, sizeof(WaveCtl), cudaMemcpyDeviceToHost, stream));
                     RTRY(cudaMemcpyAsync(h_cnt, run->cnt.p, sizeof(DevCounters), cudaMemcpyDeviceToHost, stream));
@@ -1217,7 +1236,7 @@ void run_worker_body(pach_run *run) {
         s.broadband_ms = t_bb;
         s.sort_ms = t_sort;
         s.waves = (int64_t)all.waves;
-        s.kernel_launches = timing ? launches : P + (long long)all.iters * ((sorting ? 7 : 4) - (fused ? 1 : 0));
+        s.kernel_launches = timing ? launches : P + (long long)all.iters * ((sorting ? 7 : 4) - (fused ? 1 : 0) + (map ? 1 : 0));
         s.peak_live_rays = (int64_t)all.peak_live;
         s.bvh_nodes_visited = (int64_t)h_cnt->bvh_nodes;
         s.tri_tests = (int64_t)h_cnt->tri_tests;
@@ -1257,7 +1276,9 @@ void run_worker_body(pach_run *run) {
         if (q.stream) cudaStreamSynchronize(q.stream);
         if (q.exec) cudaGraphExecDestroy(q.exec);
         if (q.graph) cudaGraphDestroy(q.graph);
-        if (q.end) cudaEventDestroy(q.end);
+        for (cudaEvent_t ev : {q.end, q.fork, q.join})
+            if (ev) cudaEventDestroy(ev);
+        if (q.side) cudaStreamDestroy(q.side);
         if (q.stream && q.stream != stream) cudaStreamDestroy(q.stream);
     }
     for (cudaEvent_t ev : kev) cudaEventDestroy(ev);

@@ -647,10 +647,11 @@ __device__ __forceinline__ int map_cell_index(float p, float lo, float vd) {
 // increments from the ray's POSITION (R.x where R.dx is meant) and stops as soon as ANY cell index
 // equals the end cell's; the octave walk starts at the grid entry point and stops on reaching the
 // end cell without visiting it (after a segment that starts and ends in one cell it runs on to the
-// grid's edge).  walk 1 visits every cell the segment crosses, the end cell included.
+// grid's edge).  walk 1 visits every cell the segment crosses, the end cell included.  This is the broadband ray's; the
+// octave rays' walk is MapCursor.
 template <typename Visit>
-__device__ __forceinline__ void map_walk(const MapDev &M, float3 o, float3 d, float3 end, bool broadband, Visit visit) {
-    const bool quirk = broadband && M.walk == 0;
+__device__ __forceinline__ void map_walk(const MapDev &M, float3 o, float3 d, float3 end, Visit visit) {
+    const bool quirk = M.walk == 0;
     float3 s = o;
     const bool inside = o.x >= M.lo[0] && o.x <= M.hi[0] && o.y >= M.lo[1] && o.y <= M.hi[1] && o.z >= M.lo[2] &&
                         o.z <= M.hi[2];
@@ -719,26 +720,90 @@ __device__ __forceinline__ void map_walk(const MapDev &M, float3 o, float3 d, fl
         }
         if (quirk) {
             if (!(c[0] != ce[0] && c[1] != ce[1] && c[2] != ce[2])) return;
-        } else if (M.walk == 0) {
-            if (c[0] == ce[0] && c[1] == ce[1] && c[2] == ce[2]) return;
         }
     }
 }
 
-// Map_Receiver.CheckRay (Pach_Map_Receiver.cs:1810-1826) over the grid: energy
-// I 10^(-0.1 m t) / (pi r^2), t = arrival time after the receiver's direct arrival (s).
-__device__ __forceinline__ uint32_t map_detect_octave(const MapDev &M, const RoomParams &P, float3 o, float3 d,
-                                                      float tseg, double t_sum, float Iabs, int oct) {
-    uint32_t n = 0;
-    map_walk(M, o, d, o + d * tseg, false, [&](int k) {
-        float t, half;
-        if (!sphere_hit(__ldg(M.rec + k), o, d, tseg, t, half)) return;
-        ++n;
-        const double time = t_sum + (double)(t * P.inv_c) - __ldg(M.direct + k);
-        map_add(M, k, oct, time, Iabs * exp2f(M.atten_k[oct] * (float)time) * M.size_mod, d);
-    });
-    return n;
-}
+// An octave ray's walk over the receiver grid (the octave walk of map_walk's comment), as a state that advances one
+// cell at a time, so that lanes at different cells of different segments run the same instructions.
+struct MapCursor {
+    int ci;                // cell
+    int e, e1;             // its entries still to visit
+    uint32_t seen;         // neighbour mask of the last three cells visited
+    int stride[3];         // change of ci for a move along an axis
+    int left[3];           // moves left before the grid's edge
+    int to_end[3];         // moves to the end cell's index
+    float tmax[3], tdel[3];
+    int a1, a2, w1, w2;    // axes of the last two moves (3: none) and their weights in a neighbour mask's bit
+
+    __device__ __forceinline__ void enter(const MapDev &M) {
+        e = __ldg(M.cell + ci);
+        e1 = __ldg(M.cell + ci + 1);
+    }
+
+    // Whether the segment o + t d, t in [0, tseg], walks the grid; if so the cursor is at its first cell.
+    __device__ __forceinline__ bool start(const MapDev &M, float3 o, float3 d, float tseg) {
+        const float3 end = o + d * tseg;
+        float3 s = o;
+        const bool inside = o.x >= M.lo[0] && o.x <= M.hi[0] && o.y >= M.lo[1] && o.y <= M.hi[1] && o.z >= M.lo[2] &&
+                            o.z <= M.hi[2];
+        if (!inside) {
+            float t0;
+            if (!map_box_entry(M, o, d, t0)) return false;
+            s = o + d * t0;
+        }
+        const float sp[3] = {s.x, s.y, s.z}, ep[3] = {end.x, end.y, end.z};
+        float g[3] = {d.x, d.y, d.z};
+        const int pitch[3] = {M.n[1] * M.n[2], M.n[2], 1};
+        ci = 0;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            g[a] = g[a] == 0.f ? 0.f : g[a];  // -0 walks as +0: its crossing time is +inf, never -inf
+            int c = map_cell_index(sp[a], M.lo[a], M.vd[a]);
+            const int ce = map_cell_index(ep[a], M.lo[a], M.vd[a]);
+            c = c < 0 ? 0 : (c >= M.n[a] ? M.n[a] - 1 : c);
+            const bool neg = g[a] < 0.f;
+            if ((neg && c < ce) || (g[a] >= 0.f && c > ce)) return false;
+            const int step = neg ? -1 : 1;
+            const float bound = (float)(neg ? c : c + 1) * M.vd[a] + M.lo[a];
+            tmax[a] = (bound - sp[a]) / g[a];
+            tdel[a] = M.vd[a] / g[a] * (float)step;
+            stride[a] = step * pitch[a];
+            left[a] = neg ? c : M.n[a] - 1 - c;
+            to_end[a] = neg ? c - ce : ce - c;
+            ci += c * pitch[a];
+        }
+        seen = 0;
+        a1 = a2 = 3;
+        w1 = w2 = 0;
+        return true;
+    }
+
+    // To the next cell; false at the walk's end.  At most the sum of the grid's sizes moves, as each uses up one of
+    // an axis's `left`.  A cell before the last one is a neighbour of this one if the two moves went along different
+    // axes, the one before that if all three did (an axis's moves go one way).
+    __device__ __forceinline__ bool advance(const MapDev &M) {
+        if (M.walk && (to_end[0] | to_end[1] | to_end[2]) == 0) return false;
+        // the reference's comparison order (ties go to z, then y)
+        const bool sx = tmax[0] < tmax[1] && tmax[0] < tmax[2];
+        const bool sy = !(tmax[0] < tmax[1]) && tmax[1] < tmax[2];
+        int axis, w, ahead;
+        if (sx) {
+            axis = 0; ahead = --left[0]; --to_end[0]; tmax[0] += tdel[0]; ci += stride[0]; w = stride[0] < 0 ? -9 : 9;
+        } else if (sy) {
+            axis = 1; ahead = --left[1]; --to_end[1]; tmax[1] += tdel[1]; ci += stride[1]; w = stride[1] < 0 ? -3 : 3;
+        } else {
+            axis = 2; ahead = --left[2]; --to_end[2]; tmax[2] += tdel[2]; ci += stride[2]; w = stride[2] < 0 ? -1 : 1;
+        }
+        if (ahead < 0) return false;  // outside the grid
+        if (!M.walk && (to_end[0] | to_end[1] | to_end[2]) == 0) return false;
+        const int b0 = 13 - w, b1 = b0 - w1, b2 = b1 - w2;
+        const bool near1 = a1 != 3 && a1 != axis, near2 = near1 && a2 != 3 && a2 != axis && a2 != a1;
+        seen = (1u << b0) | (near1 ? 1u << (b1 & 31) : 0u) | (near2 ? 1u << (b2 & 31) : 0u);
+        a2 = a1; w2 = w1; a1 = axis; w1 = w;
+        return true;
+    }
+};
 
 // Map_Receiver.CheckBroadbandRay (Pach_Map_Receiver.cs:1780-1808): all eight bands, whatever the
 // octave range.
@@ -746,7 +811,7 @@ __device__ __forceinline__ uint32_t map_detect_broad(const MapDev &M, const Room
                                                      float tseg, double t_sum, const float (&E)[kBands],
                                                      const float (&sc)[kBands]) {
     uint32_t n = 0;
-    map_walk(M, o, d, o + d * tseg, true, [&](int k) {
+    map_walk(M, o, d, o + d * tseg, [&](int k) {
         float t, half;
         if (!sphere_hit(__ldg(M.rec + k), o, d, tseg, t, half)) return;
         ++n;

@@ -161,6 +161,7 @@ struct WaveCtl {
     long long prim_first;           // first primary of the run
     unsigned long long per_prim;    // planned ring footprint per primary: 3x the pilots' largest peak (0 = none yet)
     unsigned long long trace_next;  // next wave item a trace thread takes (dynamic fetch)
+    unsigned long long map_next;    // the same for the map's kernel
     unsigned long long last_live;   // live count at the previous feed decision
     unsigned long long iters;       // loop iterations run (graph mode)
     unsigned long long idle;        // consecutive iterations that neither traced nor fed
@@ -392,8 +393,11 @@ cudaError_t launch_trace(const DevRun &r, int variant, int blocks, int threads, 
 // map: also detect the run's mapping receivers (kernel variants compiled with the grid walk)
 // wide: the shading variant with 4 blocks per SM, for rooms of at least kShadeWideReceivers receivers
 constexpr int kShadeWideReceivers = 48;
-cudaError_t launch_shade(const DevRun &r, int blocks, int threads, cudaStream_t s, bool fused = false, bool map = false,
-                         bool wide = false);
+cudaError_t launch_shade(const DevRun &r, int blocks, int threads, cudaStream_t s, bool fused = false, bool wide = false);
+cudaError_t launch_map(const DevRun &r, int blocks, cudaStream_t s);
+// Blocks of the map's kernel per SM: it runs beside the shading kernel (two 36.9 ms, the three that fit 37.5 on the
+// hall with 2500 primaries).
+constexpr int kMapBlocks = 2;
 // Room-acoustic parameters of n energy-time curves etc [n][T] x scale at fs Hz on the device (map_params.cu).
 cudaError_t launch_map_params(const double *etc, int n, int T, double fs, double scale, int decay_depth,
                               double clarity_s, double *t_x, double *edt, double *clarity, double *definition,

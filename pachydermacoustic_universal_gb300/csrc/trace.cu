@@ -232,6 +232,7 @@ __device__ void size_wave(const DevRun &r) {
     const unsigned long long most = (unsigned long long)(m < r.full_wave ? min(r.max_bounces, kSmallBounces) : r.max_bounces);
     c->bounces = (int)(per < most ? per : most);
     c->trace_next = 0;
+    c->map_next = 0;
     if (m) ++c->waves;
     if (live == 0 && c->next_prim >= c->prim_end) c->done = 1;
     if (live > 0 && m == 0) { ++c->overflow; c->done = 1; }  // ring full: cannot make progress
@@ -774,7 +775,7 @@ __device__ __forceinline__ bool surface(const DevRun &r, const DevScene &S, cons
 // block, -28 % more from the grouped detection; on the 16-receiver hall +17 % and +12 %, so it keeps
 // three blocks and the plain loop.
 constexpr int kShadeMinBlocks = 3;
-template <bool FUSED, bool MAP, bool WIDE = false>
+template <bool FUSED, bool WIDE>
 __global__ void __launch_bounds__(256, FUSED ? 2 : (WIDE ? 4 : kShadeMinBlocks)) k_shade(DevRun r) {
     extern __shared__ float4 s_rec_buf[];
     const int *s_rid;
@@ -807,6 +808,7 @@ __global__ void __launch_bounds__(256, FUSED ? 2 : (WIDE ? 4 : kShadeMinBlocks))
                     h = make_int4(tri, __float_as_int(tt), __float_as_int(B.w), __float_as_int(A.w));
                 }
                 L.v[C_RET] += tw.retests;
+                r.hits[j] = h;  // for the map's kernel
             } else {
                 h = r.hits[j];
             }
@@ -816,8 +818,6 @@ __global__ void __launch_bounds__(256, FUSED ? 2 : (WIDE ? 4 : kShadeMinBlocks))
             const RoomParams &P = r.rooms[R.room];
             L.v[C_DET] += detect_octave<WIDE>(r, P, s_rec, s_rid, R.p, R.d, hit ? t : 1e6f, R.t_sum, R.I * R.scale, R.oct,
                                         R.mask, R.prim);
-            if constexpr (MAP)
-                L.v[C_DET] += map_detect_octave(r.map, P, R.p, R.d, hit ? t : 1e6f, R.t_sum, R.I * R.scale, R.oct);
             if (!hit) {
                 // lost: no End_Trace after a miss in phase B (TaskAll:437-443), loop exit in phase C (500-505)
                 L.lost += (double)(R.I * R.scale);
@@ -841,6 +841,142 @@ __global__ void __launch_bounds__(256, FUSED ? 2 : (WIDE ? 4 : kShadeMinBlocks))
         if (nout == 2) ring_store(r, slot + 1, to_item(C));
     }
     flush_counters(r, L);
+}
+
+// The map's detections of the wave's octave rays (Map_Receiver.CheckRay, Pach_Map_Receiver.cs:1810-1826): energy
+// I 10^(-0.1 m t) / (pi r^2), t = arrival time after the receiver's direct arrival (s).
+// Inside the shading kernel each lane walked its segment's cells and their receivers to the end: 8.2 of 32 lanes
+// active.  Here a warp takes 32 segments at a time, keeps those that walk the grid, and a lane whose walk is over
+// takes the next of them; each step moves every lane by one cell or two receivers, and detections wait in a queue
+// until 32 are there.  Bound: latency of the chain cell - entry - receiver (42 % of the issue slots, 20 lanes active;
+// one receiver a step 162 us where two take 131 on a wave of 1.7M segments; four blocks an SM no faster), so it runs
+// beside the shading kernel, which reads the same wave: 20k-triangle hall, 608 receivers, 2500 primaries 42.2 ->
+// 38.7 ms, beside it 36.9.  Any number of idle lanes from 4 to 20 may wait for the next take: the same time.
+struct MapHit {
+    double t_sum;
+    float t, I;       // chord midpoint, absolute energy
+    float dx, dy, dz;
+    unsigned at;      // receiver << 3 | band
+};
+constexpr int kMapQueue = 64;
+constexpr int kMapHits = 96;   // 31 waiting and two of every lane
+constexpr int kMapRefill = 12;
+
+__global__ void __launch_bounds__(256, 3) k_map(DevRun r) {
+    __shared__ unsigned s_job[8][kMapQueue];
+    __shared__ MapHit s_hit[8][kMapHits];
+    WaveCtl *c = r.ctl;
+    const MapDev &M = r.map;
+    const unsigned long long m = c->m, head = c->head;
+    const int lane = threadIdx.x & 31;
+    const unsigned below = (1u << lane) - 1u;
+    unsigned *jobs = s_job[threadIdx.x >> 5];
+    MapHit *queue = s_hit[threadIdx.x >> 5];
+    int njobs = 0, queued = 0;
+    unsigned long long found = 0;
+    bool more = true, walking = false;
+    MapCursor K;
+    K.e = K.e1 = 0;
+    float3 o = make_float3(0.f, 0.f, 0.f), d = o;
+    float tseg = 0.f;
+    double t_sum = 0;
+    float I = 0.f;
+    unsigned oct = 0;
+    auto segment = [&](unsigned i, float3 &so, float3 &sd, float &st) {
+        const float4 *q = reinterpret_cast<const float4 *>(wave_item(r, head, i));
+        so = f3(q[0]);
+        sd = f3(q[1]);
+        const int4 h = r.hits[i];
+        st = h.x >= 0 ? __int_as_float(h.y) : 1e6f;
+    };
+    auto add = [&](int i) {
+        const MapHit x = queue[i];
+        const int k = (int)(x.at >> 3), oct = (int)(x.at & 7u);
+        const double time = x.t_sum + (double)(x.t * r.rooms[0].inv_c) - __ldg(M.direct + k);
+        map_add(M, k, oct, time, x.I * exp2f(M.atten_k[oct] * (float)time) * M.size_mod,
+                make_float3(x.dx, x.dy, x.dz));
+    };
+    for (;;) {
+        const unsigned idle = __ballot_sync(FULL, !walking);
+        if (__popc(idle) >= kMapRefill) {
+            const int want = __popc(idle);
+            while (more && njobs < want) {
+                unsigned long long base = 0;
+                if (lane == 0) base = atomicAdd(&c->map_next, 32ull);
+                base = __shfl_sync(FULL, base, 0);
+                if (base >= m) { more = false; break; }
+                bool cross = false;
+                const unsigned long long i = base + lane;
+                if (i < m) {
+                    float3 so, sd;
+                    float st;
+                    segment((unsigned)i, so, sd, st);
+                    MapCursor X;
+                    cross = X.start(M, so, sd, st);
+                }
+                const unsigned who = __ballot_sync(FULL, cross);
+                if (cross) jobs[njobs + __popc(who & below)] = (unsigned)i;
+                njobs += __popc(who);
+            }
+            __syncwarp();
+            if (njobs == 0 && idle == FULL) break;
+            const int rank = __popc(idle & below);
+            if (!walking && rank < njobs) {
+                const unsigned j = jobs[njobs - 1 - rank];
+                segment(j, o, d, tseg);
+                const Ray R = to_ray(load_item(wave_item(r, head, j), 0));
+                t_sum = R.t_sum;
+                I = R.I * R.scale;
+                oct = (unsigned)R.oct;
+                walking = K.start(M, o, d, tseg);
+                if (walking) K.enter(M);
+            }
+            njobs = max(njobs - want, 0);
+            __syncwarp();
+        }
+        if (walking && K.e == K.e1) {
+            walking = K.advance(M);
+            if (walking) K.enter(M);
+        }
+        bool hit[2] = {false, false};
+        float t[2] = {0.f, 0.f};
+        int k[2] = {0, 0};
+        if (walking && K.e < K.e1) {
+            float half;
+            const bool two = K.e + 1 < K.e1;
+            const uint2 en = __ldg(M.entry + K.e), en1 = __ldg(M.entry + K.e + two);
+            K.e += 1 + two;
+            k[0] = (int)en.x;
+            k[1] = (int)en1.x;
+            const float4 c0 = __ldg(M.rec + k[0]), c1 = __ldg(M.rec + k[1]);
+            hit[0] = !(en.y & K.seen) && sphere_hit(c0, o, d, tseg, t[0], half);
+            hit[1] = two && !(en1.y & K.seen) && sphere_hit(c1, o, d, tseg, t[1], half);
+        }
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const unsigned who = __ballot_sync(FULL, hit[q]);
+            if (hit[q]) {
+                MapHit x;
+                x.t_sum = t_sum;
+                x.t = t[q];
+                x.I = I;
+                x.dx = d.x; x.dy = d.y; x.dz = d.z;
+                x.at = (unsigned)k[q] << 3 | oct;
+                queue[queued + __popc(who & below)] = x;
+            }
+            queued += __popc(who);
+            found += __popc(who);
+        }
+        while (queued >= 32) {
+            __syncwarp();
+            queued -= 32;
+            add(queued + lane);
+            __syncwarp();
+        }
+    }
+    __syncwarp();
+    if (lane < queued) add(lane);
+    if (lane == 0 && found) atomicAdd(&r.cnt->detections, found);
 }
 
 // Small scenes: walk and shade, each lane keeping its ray in registers over up to ctl->bounces interactions, then
@@ -1163,14 +1299,15 @@ cudaError_t launch_trace(const DevRun &r, int variant, int blocks, int threads, 
     return cudaGetLastError();
 }
 
-cudaError_t launch_shade(const DevRun &r, int blocks, int threads, cudaStream_t s, bool fused, bool map, bool wide) {
-    if (map) {
-        if (fused) k_shade<true, true><<<blocks, threads, rec_smem(r), s>>>(r);
-        else k_shade<false, true><<<blocks, threads, rec_smem(r), s>>>(r);
-    } else {
-        if (wide) k_shade<false, false, true><<<blocks, threads, rec_smem(r), s>>>(r);
-        else k_shade<false, false><<<blocks, threads, rec_smem(r), s>>>(r);
-    }
+cudaError_t launch_shade(const DevRun &r, int blocks, int threads, cudaStream_t s, bool fused, bool wide) {
+    if (fused) k_shade<true, false><<<blocks, threads, rec_smem(r), s>>>(r);
+    else if (wide) k_shade<false, true><<<blocks, threads, rec_smem(r), s>>>(r);
+    else k_shade<false, false><<<blocks, threads, rec_smem(r), s>>>(r);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_map(const DevRun &r, int blocks, cudaStream_t s) {
+    k_map<<<blocks, 256, 0, s>>>(r);
     return cudaGetLastError();
 }
 
@@ -1198,8 +1335,8 @@ cudaError_t wave_kernel_occupancy(int variant, int threads, int smem_shade, int 
         default: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(bpsm_trace, k_trace<4, false, false>, threads, 0); break;
     }
     if (e != cudaSuccess) return e;
-    if (fused) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(bpsm_shade, k_shade<true, true>, threads, smem_shade);
-    if (wide) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(bpsm_shade, k_shade<false, false, true>, threads, smem_shade);
+    if (fused) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(bpsm_shade, k_shade<true, false>, threads, smem_shade);
+    if (wide) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(bpsm_shade, k_shade<false, true>, threads, smem_shade);
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(bpsm_shade, k_shade<false, false>, threads, smem_shade);
 }
 

@@ -248,3 +248,23 @@ def test_directional_map_matches_oracle():
         a, b = g[k].sum(axis=-1), ho[ko].sum(axis=-1)
         np.testing.assert_allclose(a, b, rtol=2e-3, atol=1e-6 * np.abs(b).max())
     assert (g["dir_pos"] >= 0).all() and (g["dir_neg"] <= 0).all()
+
+
+@pytest.mark.parametrize("walk", [0, 1])
+@pytest.mark.parametrize("layout", ["one", "row", "lattice"])
+@pytest.mark.parametrize("rays", [1, 33, 300])
+def test_map_walk_over_grid_shapes_matches_oracle(walk, layout, rays):
+    """The map's kernel from one segment to many (its takes of 32, its queue of 32 detections) over grids of one cell
+    a side, one cell wide and several cells on every axis.  A detection is the same size whatever its chord, and a
+    sphere grazed within FP32 rounding (about 1e-6 of them) or a bin edge may differ: 1e-3 of the sums, 2 % of the
+    bins."""
+    x = {"one": [(5.0, 4.0, 1.5)], "row": [(1.5 + i, 4.0, 1.5) for i in range(7)],
+         "lattice": [(2.0 + 1.5 * i, 2.0 + 1.3 * j, 0.8 + 0.9 * k) for i in range(5) for j in range(4) for k in range(3)]}
+    w, org = _shifted(rooms.shoebox_c1(), np.array(x[layout]))
+    m = tracer.MapReceivers(org, 1.0, 1000.0, walk=walk)
+    hg, sg, ho, so = _both(w, m, rays, 9, pure_specular=True)
+    Eg, Eo = hg["map"]["energy"], ho["map_energy"]
+    assert Eo.sum() > 0 or rays == 1  # one ray may miss the one receiver
+    np.testing.assert_allclose(Eg.sum(axis=(0, 2)), Eo.sum(axis=(0, 2)), rtol=1e-3)
+    occ = Eo > 0
+    assert not occ.any() or np.mean(np.abs(Eg[occ] - Eo[occ]) < 1e-3 * Eo[occ]) >= 0.98
