@@ -257,19 +257,28 @@ static void rebase_codes(float *nodes, size_t count, int stride, int code_at, in
     });
 }
 
-// Rebases 48-byte quantised nodes (see quantize_bvh): the first inner child's node id and the first
-// leaf triangle, which keeps its 24 bits (append_scene drops the quantised copy of a batch beyond that).
-static void rebase_qnodes(float *nodes, size_t count, int node_off, int tri_off) {
+// The walk's form of 48-byte quantised nodes (see quantize_bvh), ids offset by the scene's place in the array:
+//   8 words  origin x, y, z; step / 256 along x; lo.x of children 0-3 as bytes, hi.x, lo.y, hi.y
+//   8 words  lo.z, hi.z; child codes 0-3 as in the float nodes; step / 256 along y, z
+static void expand_qnodes(const float *nodes, size_t count, float *out, int node_off, int tri_off) {
     parallel_chunks(count, 16384, [=](size_t q0, size_t q1) {
         for (size_t q = q0; q < q1; ++q) {
-            float *g = nodes + q * kBvhQNodeFloats;
-            uint32_t nb, tw;
-            std::memcpy(&nb, &g[10], 4);
-            std::memcpy(&tw, &g[11], 4);
-            nb += (uint32_t)node_off;
-            tw = (((tw & 0xFFFFFFu) + (uint32_t)tri_off) & 0xFFFFFFu) | (tw & 0xFF000000u);
-            std::memcpy(&g[10], &nb, 4);
-            std::memcpy(&g[11], &tw, 4);
+            uint32_t g[kBvhQNodeFloats], o[kBvhDevFloats];
+            std::memcpy(g, nodes + q * kBvhQNodeFloats, sizeof(g));
+            for (int k = 0; k < 3; ++k) o[k] = g[k];
+            const uint32_t slots = (g[3] >> 24) | ((g[11] >> 24) << 8);
+            o[3] = (g[3] & 255u) << 23;
+            o[14] = ((g[3] >> 8) & 255u) << 23;
+            o[15] = ((g[3] >> 16) & 255u) << 23;
+            for (int k = 0; k < 6; ++k) o[4 + k] = g[4 + k];
+            int inner = (int)g[10] + node_off, tri = (int)(g[11] & 0xFFFFFFu) + tri_off;
+            for (int k = 0; k < 4; ++k) {
+                const int v = (int)((slots >> (4 * k)) & 15u);
+                o[10 + k] = (uint32_t)(v == 0 ? inner : v <= 8 ? ~(tri * 16 + v - 1) : (int)0x80000000);
+                inner += v == 0;
+                tri += v <= 8 ? v : 0;
+            }
+            std::memcpy(out + q * kBvhDevFloats, o, sizeof(o));
         }
     });
 }
@@ -380,11 +389,13 @@ int append_scene(const HostScene &hs, SceneArrays &A, int *n_planes = nullptr) {
                        (long long)tri_off + hs.ntri <= (1ll << 24);
     if (!quant) A.bvhq.clear();
     const size_t q0 = A.bvhq.size();
-    if (quant) A.bvhq.insert(A.bvhq.end(), hs.bvhq.begin(), hs.bvhq.end());
-    if (tri_off || node_off) {
-        rebase_codes(&A.bvh[b0], hs.bvh.size() / kBvhNodeFloats, kBvhNodeFloats, 24, node_off, tri_off);
-        if (quant) rebase_qnodes(&A.bvhq[q0], hs.bvhq.size() / kBvhQNodeFloats, node_off, tri_off);
+    if (quant) {
+        const size_t nodes = hs.bvhq.size() / kBvhQNodeFloats;
+        A.bvhq.resize(q0 + nodes * kBvhDevFloats);
+        expand_qnodes(hs.bvhq.data(), nodes, &A.bvhq[q0], node_off, tri_off);
     }
+    if (tri_off || node_off)
+        rebase_codes(&A.bvh[b0], hs.bvh.size() / kBvhNodeFloats, kBvhNodeFloats, 24, node_off, tri_off);
     A.t_eps = std::max(A.t_eps, (float)(2e-7 * hs.scale));
     A.has_trans = A.has_trans || hs.has_trans;
     return node_off;
@@ -409,7 +420,7 @@ cudaError_t upload_scene(const SceneArrays &A, DevMem &tri, DevMem &tri64, DevMe
         (e = upload(bvh, A.bvh.data(), A.bvh.size() * sizeof(float))) ||
         (e = upload(bvhq, A.bvhq.data(), A.bvhq.size() * sizeof(float))))
         return e;
-    d.bvhq = bvhq.as<float4>();
+    d.bvhq = bvhq.as<float>();
     d.tri = tri.as<float4>();
     d.tri64 = tri64.as<double>();
     d.pnormal = norm.as<float4>();
@@ -1243,7 +1254,7 @@ void run_worker_body(pach_run *run) {
         s.accel[0] = (int32_t)(n_rooms > 1 ? run->bbvh.bytes / (kBvhNodeFloats * sizeof(float)) : hs.bvh_nodes);
         s.accel[1] = hs.bvh_leaves;
         s.accel[2] = hs.bvh_depth;
-        s.walk = (quant ? 4 * kBvhQNodeFloats : 4 * kBvhNodeFloats) + 1000 * (fused ? 3 : ((tr_variant & 16) ? 2 : 1));
+        s.walk = (quant ? 4 * kBvhDevFloats : 4 * kBvhNodeFloats) + 1000 * (fused ? 3 : ((tr_variant & 16) ? 2 : 1));
         s.revolutions = conv_mode ? run->conv_revs : 0;
         s.converged = conv_mode && run->conv_converged ? 1 : 0;
         s.check_receivers[0] = conv_mode ? run->conv_rows[0] : -1;

@@ -107,6 +107,7 @@ struct HostScene {
 constexpr int kBvhStack = 64;
 constexpr int kBvhNodeFloats = 32;
 constexpr int kBvhQNodeFloats = 12;  // 48-byte quantised nodes
+constexpr int kBvhDevFloats = 16;    // the walk's 64-byte form of them (expand_qnodes)
 constexpr int kLeafMax = 8;      // largest leaf the node encoding holds
 constexpr int kLeafDefault = 3;  // leaf size used when the scene does not ask for one (measured best of 2..8)
 
@@ -124,7 +125,7 @@ struct DevScene {
     const float4 *mat;          // [npoly*8]: (1-alpha, s_lo, s_mid, s_hi)
     const float *trans;         // [npoly*8]
     const float4 *bvh;          // [nodes*8] 128-byte nodes
-    const float4 *bvhq;         // [nodes*3] 48-byte quantised nodes (null: walk the 128-byte ones)
+    const float *bvhq;          // [nodes*16] 64-byte quantised nodes (null: walk the 128-byte ones)
     const float4 *plane;        // [planes*2] every room's planes (RoomParams::plane_begin)
     const int *plane_tri;       // the planes' triangles
     int ntri;
@@ -369,7 +370,7 @@ cudaError_t launch_sort(const DevRun &r, int blocks, cudaStream_t s);  // count 
 // scenes of more than kSpecMinTris triangles: measured on a 20k-triangle hall it walks 1.5x faster than
 // one leaf at a time, while on a 12-triangle shoebox (a two-level tree) it is 10 % slower.
 constexpr int kSpecMinTris = 64;
-// quantised: walk the 48-byte nodes (variants for 4 and 6 blocks per SM), + 32.
+// quantised: walk the quantised nodes (variants for 4 and 6 blocks per SM), + 32.
 inline int trace_variant(int blocks_per_sm, int traversal, int ntri, bool quantised = false) {
     // default: 6 blocks of 256 (40 registers) on the smaller quantised nodes (+2.5 % on a 20k-triangle
     // hall), 4 (64 registers) on 128-byte nodes (+23 %)
@@ -379,10 +380,10 @@ inline int trace_variant(int blocks_per_sm, int traversal, int ntri, bool quanti
     if (spec) return 16 + (minb >= 6 ? 6 : 4);
     return minb;
 }
-// bvh_format of pach_trace_params: 0 default, 1 128-byte float nodes, 2 48-byte quantised nodes.
-// The default walks quantised nodes above kQuantMinTris triangles: measured +6 % walk rate on a
-// 20k-triangle hall and +8 % on a 500k-triangle arena (L1-bound walks), -37 % on a 12-triangle
-// shoebox (a two-node tree: the decode costs, the smaller nodes save nothing).
+// bvh_format of pach_trace_params: 0 default, 1 128-byte float nodes, 2 quantised nodes (48 bytes on the host, 64
+// in the walk's form).  The default walks quantised nodes above kQuantMinTris triangles.  They are the faster ones
+// from 84 triangles on (a room of 532: 51.5 ms against 77.5), but of two triangles at the very same distance the
+// first one walked wins and the two formats' orders differ, so the line stays where it was.
 constexpr int kQuantMinTris = 1024;
 inline bool use_quantised_nodes(int bvh_format, int ntri) {
     return bvh_format == 2 || (bvh_format == 0 && ntri > kQuantMinTris);
