@@ -537,11 +537,17 @@ __device__ __forceinline__ void write_hit(const DevRun &r, const DevScene &S, un
 // shrink the best hit sooner (fewer nodes and triangles per ray) and the warp idles less.  Measured
 // on the arena (500k triangles) for 0 / 2 / 8 / 10 / 12 / 16 / 24 / 31: 1.65 / 1.73 / 1.78 / 1.80 /
 // 1.79 / 1.76 / 1.58 / 1.23 G segments/s; on the 20k-triangle hall 0 / 8 / 12: 1.82 / 1.99 / 1.97.
-constexpr int kSpecSlack = 10;
+// Lanes whose walk has ended write their hits and take new rays once kTraceRefill of them are there: one at a time
+// each cost the warp the loads and three divisions of a ray start.  Device ms of the hall and the arena, refill at
+// 1 / 4 / 6 / 8 / 12 / 16 / 20 with slack 10: 140.2 / 136.8 / 135.2 / 134.0 / 133.5 / 135.6 / 140.4 and 87.9 / 87.0 /
+// 86.1 / 85.1 / 84.8 / 86.7 / 87.2; at 12 with slack 8 131.8 and 84.7, with 6 131.4 and 85.4.
+constexpr int kSpecSlack = 8;
+constexpr int kTraceRefill = 12;
 
 // Persistent BVH walk with dynamic ray fetch: every loop iteration a lane descends inner nodes to
 // its next leaf and tests it; a lane whose walk has ended writes its hit and takes the next wave
-// item at once (one ticket atomic per warp), so a warp does not idle on its slowest lane.
+// item (one ticket atomic per warp; the speculative walk: once kTraceRefill lanes wait), so a warp does not idle on
+// its slowest lane.
 // Values the walk needs only when a ray starts or ends, once per leaf or once per warp iteration live
 // in shared memory (each lane's wave index, the plane it leaves and its hit tolerance; each warp's node
 // and triangle counts), not in registers: the walk's 40 registers already spill.  The counts are taken
@@ -559,7 +565,7 @@ __global__ void __launch_bounds__(256, MINB) k_trace(DevRun r) {
     if (lane == 0) s_cnt[wid][0] = s_cnt[wid][1] = 0;
     __syncwarp();
     TraceWork w;
-    bool have = false, exhausted = false;
+    bool have = false, exhausted = false, done = false;
     unsigned j = 0;  // index in the wave (a wave holds at most half the ring: < 2^31 items)
     float3 o = make_float3(0.f, 0.f, 0.f), d = o;
     float ix = 0.f, iy = 0.f, iz = 0.f, ox = 0.f, oy = 0.f, oz = 0.f, best = FLT_MAX;
@@ -568,7 +574,11 @@ __global__ void __launch_bounds__(256, MINB) k_trace(DevRun r) {
     int2 stack[kBvhStack];
     for (;;) {
         const unsigned need = __ballot_sync(FULL, !have && !exhausted);
-        if (need) {
+        if (need && (!SPEC || __popc(need) >= kTraceRefill || !__any_sync(FULL, have))) {
+            if constexpr (SPEC) {
+                if (done) write_hit(r, S, s_item[threadIdx.x], bi, best);
+                done = false;
+            }
             const int leader = __ffs(need) - 1;
             unsigned long long base = 0;
             if (lane == leader) base = atomicAdd(&c->trace_next, (unsigned long long)__popc(need));
@@ -602,7 +612,7 @@ __global__ void __launch_bounds__(256, MINB) k_trace(DevRun r) {
                 }
             }
         }
-        if (!__any_sync(FULL, have)) break;
+        if (!__any_sync(FULL, have)) break;  // every lane is exhausted
         if constexpr (SPEC) {
             // Speculative walk: a lane that has found a leaf keeps descending inner nodes while any
             // lane of the warp is still looking for its first leaf; then the warp tests its leaves
@@ -657,7 +667,7 @@ __global__ void __launch_bounds__(256, MINB) k_trace(DevRun r) {
                 leaf = 0;
             }
             if (have && node == kEmptyChild) {
-                write_hit(r, S, s_item[threadIdx.x], bi, best);
+                done = true;
                 have = false;
             }
         } else {
@@ -683,6 +693,9 @@ __global__ void __launch_bounds__(256, MINB) k_trace(DevRun r) {
                 have = false;
             }
         }
+    }
+    if constexpr (SPEC) {
+        if (done) write_hit(r, S, s_item[threadIdx.x], bi, best);
     }
     // one atomic per warp for each counter
     unsigned long long a = w.retests, b = w.nodes, c2 = w.tris;
