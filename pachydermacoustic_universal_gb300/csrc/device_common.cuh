@@ -207,6 +207,18 @@ __device__ __forceinline__ void cswap(float &ka, int &va, float &kb, int &vb) {
     }
 }
 
+// 32 bytes in one load.  A large scene's walk is bound by its L1 requests (each lane's goes to a line of its own) and
+// by issue: three 16-byte loads of a 48-byte node and 40 instructions for its child codes and steps against two
+// loads of a node that holds them ready: 10 % fewer instructions; 20k-triangle hall 142.5 -> 140.5 ms, 500k-triangle
+// arena 91.3 -> 88.4.  (Triangles padded to 64 bytes for the same: 142.7 and 89.2, a third more lines.)  Nodes evicted
+// last: arena 84.7 -> 84.0, hall unchanged.  128-byte nodes by four loads instead of seven: a room of 1004 triangles
+// 85.1 -> 69.2 ms, of 84 triangles 49.4 -> 45.0.
+__device__ __forceinline__ void load8(const float *p, uint32_t (&w)[8]) {
+    asm("ld.global.nc.L1::evict_last.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
+        : "l"(p));
+}
+
 // One 4-wide node: slab-test the children against [0, best], order the hit ones by entry distance
 // (5-exchange sorting network), push all but the nearest (farthest first), return the nearest in
 // `next`.  Returns false when no child is hit.
@@ -216,15 +228,21 @@ __device__ __forceinline__ bool bvh4_step(const float4 *__restrict__ bvh, int no
     const float4 *N = bvh + (kBvhNodeFloats / 4) * node;
     // the near plane of each axis is the low bound for a positive direction, the high one otherwise:
     // choosing it per node leaves one max and one min per axis and child
-    const float4 lx = __ldg(N), hx = __ldg(N + 1), ly = __ldg(N + 2), hy = __ldg(N + 3);
-    const float4 lz = __ldg(N + 4), hz = __ldg(N + 5);
+    uint32_t X[8], Y[8], Z[8];  // low bounds of children 0-3, high bounds
+    load8(reinterpret_cast<const float *>(N), X);
+    load8(reinterpret_cast<const float *>(N + 2), Y);
+    load8(reinterpret_cast<const float *>(N + 4), Z);
     const int4 ch = __ldg(reinterpret_cast<const int4 *>(N + 6));
-    const float4 nx = ix < 0.f ? hx : lx, fx = ix < 0.f ? lx : hx;
-    const float4 ny = iy < 0.f ? hy : ly, fy = iy < 0.f ? ly : hy;
-    const float4 nz = iz < 0.f ? hz : lz, fz = iz < 0.f ? lz : hz;
-    const float anx[4] = {nx.x, nx.y, nx.z, nx.w}, afx[4] = {fx.x, fx.y, fx.z, fx.w};
-    const float any_[4] = {ny.x, ny.y, ny.z, ny.w}, afy[4] = {fy.x, fy.y, fy.z, fy.w};
-    const float anz[4] = {nz.x, nz.y, nz.z, nz.w}, afz[4] = {fz.x, fz.y, fz.z, fz.w};
+    float anx[4], afx[4], any_[4], afy[4], anz[4], afz[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        anx[k] = __uint_as_float(ix < 0.f ? X[4 + k] : X[k]);
+        afx[k] = __uint_as_float(ix < 0.f ? X[k] : X[4 + k]);
+        any_[k] = __uint_as_float(iy < 0.f ? Y[4 + k] : Y[k]);
+        afy[k] = __uint_as_float(iy < 0.f ? Y[k] : Y[4 + k]);
+        anz[k] = __uint_as_float(iz < 0.f ? Z[4 + k] : Z[k]);
+        afz[k] = __uint_as_float(iz < 0.f ? Z[k] : Z[4 + k]);
+    }
     int id[4] = {ch.x, ch.y, ch.z, ch.w};
     float tk[4];
 #pragma unroll
@@ -253,16 +271,6 @@ __device__ __forceinline__ bool bvh4_step(const float4 *__restrict__ bvh, int no
 // 2^23 + 256 q; with the node's scale s / 256 the 2^15 steps it carries are taken off the slab offset
 // once per node and axis (one rounding, at most 2^-9 of a step, inside the builder's s / 256 margin)
 // instead of a subtraction per bound.
-// 32 bytes in one load.  A large scene's walk is bound by its L1 requests (each lane's goes to a line of its own) and
-// by issue: three 16-byte loads of a 48-byte node and 40 instructions for its child codes and steps against two
-// loads of a node that holds them ready: 10 % fewer instructions; 20k-triangle hall 142.5 -> 140.5 ms, 500k-triangle
-// arena 91.3 -> 88.4.  (Triangles padded to 64 bytes for the same: 142.7 and 89.2, a third more lines.)
-__device__ __forceinline__ void load8(const float *p, uint32_t (&w)[8]) {
-    asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-        : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
-        : "l"(p));
-}
-
 template <typename E>
 __device__ __forceinline__ bool bvh4q_step(const float *__restrict__ bvhq, int node, float ix, float iy, float iz,
                                            float px, float py, float pz, float best, E *stack, int &sp, int &next) {

@@ -382,7 +382,7 @@ inline int trace_variant(int blocks_per_sm, int traversal, int ntri, bool quanti
 }
 // bvh_format of pach_trace_params: 0 default, 1 128-byte float nodes, 2 quantised nodes (48 bytes on the host, 64
 // in the walk's form).  The default walks quantised nodes above kQuantMinTris triangles.  They are the faster ones
-// from 84 triangles on (a room of 532: 51.5 ms against 77.5), but of two triangles at the very same distance the
+// from 84 triangles on (a room of 532: 51.5 ms against 63.8), but of two triangles at the very same distance the
 // first one walked wins and the two formats' orders differ, so the line stays where it was.
 constexpr int kQuantMinTris = 1024;
 inline bool use_quantised_nodes(int bvh_format, int ntri) {

@@ -229,3 +229,21 @@ def test_primaries_shared_out_to_several_loops_equal_one_loop(kind, rays):
             if isinstance(x, np.ndarray):
                 rtol = 1.2e-4 if name == "capture" else 1e-9
                 np.testing.assert_allclose(x, b[name], rtol=rtol, atol=1e-30, err_msg=name)
+
+
+@pytest.mark.parametrize("bvh_format", [1, 2])
+@pytest.mark.parametrize("tris,rays", [(84, 1), (84, 300), (2000, 5), (2000, 260), (5000, 40)])
+def test_speculative_walk_finds_the_hits_of_the_plain_one(bvh_format, tris, rays):
+    """Lanes that take rays together, from fewer rays than a warp to many, and both node forms: the same nearest hits
+    as one leaf at a time, up to exact ties between triangles (a few rays in a million, as between the formats)."""
+    w = rooms.irregular_hall_c2(target_tris=tris) if tris > 1000 else rooms.shoebox_c1()
+    if tris <= 1000:
+        w.scene = rooms._jittered_room(np.random.default_rng(2), (10.0, 8.0, 4.0), tris, 3, 0.0, (0.1, 0.4), (0.1, 0.5))
+        assert w.scene.n_triangles > 64
+    w.cutoff_s = 0.4
+    ds = tracer.DeviceScene(w.scene)
+    ha, sa = tracer.trace(w, dscene=ds, rays=rays, seed=3, bvh_format=bvh_format, traversal=1)
+    hb, sb = tracer.trace(w, dscene=ds, rays=rays, seed=3, bvh_format=bvh_format, traversal=2)
+    assert sb["primaries"] == rays and sb["queue_overflows"] == 0
+    assert abs(sa["segments"] - sb["segments"]) <= 1e-4 * sa["segments"]
+    assert hb["energy"].sum() == pytest.approx(ha["energy"].sum(), rel=1e-3)
