@@ -540,9 +540,10 @@ __device__ __forceinline__ void write_hit(const DevRun &r, const DevScene &S, un
 // Lanes whose walk has ended write their hits and take new rays once kTraceRefill of them are there: one at a time
 // each cost the warp the loads and three divisions of a ray start.  Device ms of the hall and the arena, refill at
 // 1 / 4 / 6 / 8 / 12 / 16 / 20 with slack 10: 140.2 / 136.8 / 135.2 / 134.0 / 133.5 / 135.6 / 140.4 and 87.9 / 87.0 /
-// 86.1 / 85.1 / 84.8 / 86.7 / 87.2; at 12 with slack 8 131.8 and 84.7, with 6 131.4 and 85.4.
-constexpr int kSpecSlack = 8;
-constexpr int kTraceRefill = 12;
+// 86.1 / 85.1 / 84.8 / 86.7 / 87.2; at 12 with slack 8 131.8 and 84.7, with 6 131.4 and 85.4.  With the stack of
+// 4-byte entries: 12 and 10 127.0 and 79.9, 12 and 8 125.2 and 80.2, 10 and 8 125.3 and 79.6, 10 and 6 124.1 and 79.9.
+constexpr int kSpecSlack = 6;
+constexpr int kTraceRefill = 10;
 
 // Persistent BVH walk with dynamic ray fetch: every loop iteration a lane descends inner nodes to
 // its next leaf and tests it; a lane whose walk has ended writes its hit and takes the next wave
@@ -571,7 +572,11 @@ __global__ void __launch_bounds__(256, MINB) k_trace(DevRun r) {
     float ix = 0.f, iy = 0.f, iz = 0.f, ox = 0.f, oy = 0.f, oz = 0.f, best = FLT_MAX;
     int skip = -1, node = 0, sp = 0, bi = -1, leaf = 0;
     float teps = S.t_eps;
-    int2 stack[kBvhStack];
+    // 4-byte entries: a box beyond the best hit is then entered once more and rejected by its children's test, yet the
+    // stack is what the walk reads most, and its lines that miss L1: hall 131.8 -> 125.2 ms, arena 83.8 -> 80.2
+    // against (id, distance) entries.  (The first 4 to 16 in shared memory 128 and 82, the top in a register 130.5 and
+    // 81.8; 5 or 7 blocks an SM 135 and 133.)
+    int stack[kBvhStack];
     for (;;) {
         const unsigned need = __ballot_sync(FULL, !have && !exhausted);
         if (need && (!SPEC || __popc(need) >= kTraceRefill || !__any_sync(FULL, have))) {
@@ -645,11 +650,9 @@ __global__ void __launch_bounds__(256, MINB) k_trace(DevRun r) {
                     // two thirds of the walk's L1 requests (hall 140.5 -> 137.7 ms, arena 88.4 -> 86.9 against a
                     // loop for each; the top entry in registers 138.8 and 87.8)
                     while (node == kEmptyChild && sp > 0) {
-                        const int2 e = stack[--sp];
-                        if (__int_as_float(e.y) <= best) {
-                            if (e.x < 0 && leaf == 0) leaf = e.x;
-                            else node = e.x;
-                        }
+                        const int e = stack[--sp];
+                        if (e < 0 && leaf == 0) leaf = e;
+                        else node = e;
                     }
                 }
             }
