@@ -468,21 +468,22 @@ def filters_measure(h0, fs, reps, flush, device):
             fp = json.load(f).get("filters", {})
     except (OSError, ValueError):
         fp = {}
-    if fp.get("dp_inst_per_filter") and geo == 32768:
-        # FP64 issue: DP lane-instructions per second against SMs x 2 FP64 lanes x the SM clock
+    if fp.get("thread_inst_per_filter") and geo == 32768:
+        # instruction issue: lane-instructions per second against SMs x 4 schedulers x 32 lanes x the SM clock
         props = torch.cuda.get_device_properties(device)
         mhz = (_peaks()[0] or {}).get("sm_max_mhz", 2070.0)
-        peak = props.multi_processor_count * fp["fp64_lanes_per_sm_cycle"] * mhz * 1e6
-        ach = fp["dp_inst_per_filter"] * n / (ms * 1e-3)
-        roof = {"bound": "fp64 issue", "achieved": ach / 1e9, "peak": peak / 1e9, "unit": "G DP lane-instructions/s",
-                "frac": ach / peak, "per_unit": f"{fp['dp_inst_per_filter'] / 1e6:.2f} M DP instructions per filter "
+        peak = props.multi_processor_count * 128 * mhz * 1e6
+        ach = fp["thread_inst_per_filter"] * n / (ms * 1e-3)
+        roof = {"bound": "instruction issue", "achieved": ach / 1e9, "peak": peak / 1e9, "unit": "G lane-instructions/s",
+                "frac": ach / peak, "per_unit": f"{fp['thread_inst_per_filter'] / 1e6:.2f} M lane-instructions per filter "
                                                 "of a 32768-point transform (ncu)",
-                "peak_source": f"{props.multi_processor_count} SMs x {fp['fp64_lanes_per_sm_cycle']} FP64 lanes x "
-                               f"{mhz:.0f} MHz", "source": fp.get("source")}
+                "peak_source": f"{props.multi_processor_count} SMs x 4 schedulers x 32 lanes x {mhz:.0f} MHz",
+                "source": fp.get("source")}
     return {"filters": n, "receivers": R, "bins": T, "transform_length": geo, "filter_samples": T + 12287,
             "device_ms": ms, "device_us_per_filter": ms * 1e3 / n, "e2e_ms": e2e_ms,
             "e2e_h2d_bytes": int(E.nbytes + P.nbytes + Dp.nbytes + Dn.nbytes), "e2e_d2h_bytes": int(n * (T + 12287) * 8),
-            "launches": 4 + 3 * -(-n // max(1, min(n, (512 << 20) // (5 * geo * 16)))),
+            # integer transforms: 5 kernels a call and 4 for every 96 MB of filters
+            "launches": 5 + 4 * -(-n // max(1, min(n, (96 << 20) // (252 * T + 20 * geo + 1024)))),
             "cpu_baseline": {"value": cpu_ms, "unit": "ms per filter", "cores": 1, "kind": "port",
                              "sample": "the 7 filters of receiver 0 (numpy FP64 FFT convolution)"},
             "roofline": roof,
@@ -703,6 +704,8 @@ def main():
     kern = "k_trace" if agg["trace_ms"] >= agg["shade_ms"] else "k_shade"
     k_ms = agg["trace_ms"] if kern == "k_trace" else agg["shade_ms"]
     k_bytes = trace_bytes if kern == "k_trace" else shade_bytes
+    if stats[0]["walk"] // 1000 == 3:  # small scenes: rays stay in registers over up to 32 interactions
+        kern, k_bytes = "k_bounce", 48.0 * agg["detections"]
     achieved_gbs = k_bytes / (k_ms * 1e-3) / 1e9 if k_ms > 0 else None
     oct_launch = agg["waves"]
     # the on-chip side of the walk: BVH node (128 B) and triangle (48 B) reads served by L1/L2
@@ -740,6 +743,7 @@ def main():
                      "frac": (achieved_gbs / peaks["hbm_gbs"]) if achieved_gbs else None,
                      "traffic": None, "peak_source": peak_kind,
                      "per_unit": ("56 B per octave segment" if kern == "k_trace" else
+                                  "48 B per detection" if kern == "k_bounce" else
                                   "72 B in + 64 B per output ray per octave segment + 48 B per detection"),
                      "bvh_reads_gbs": bvh_gbs,
                      "bvh_reads_note": f"BVH node ({node_bytes:.0f} B) and triangle (48 B) reads of the walk per "

@@ -114,9 +114,11 @@ typedef struct {
     int64_t feed_batch;            /* primaries handed to the device per phase-A launch (0 = default) */
     int32_t block_threads;         /* threads per block of the trace and shade kernels; 0 = default */
     int32_t blocks_per_sm;         /* resident blocks per SM to launch; 0 = occupancy maximum */
-    int32_t wave_kilo_items;       /* octave rays per wave, in units of 1024; 0 = default (8192) */
+    int32_t wave_kilo_items;       /* octave rays per wave, in units of 1024; 0 = default (8192; 4096
+                                      in each of the loops a run is shared out to) */
     int32_t ring_log2;             /* ring queue capacity 2^ring_log2 octave rays; 0 = default (2^22..2^28 by
-                                      the run's primaries, 2048 rays each) */
+                                      the run's primaries, 2048 rays each; runs of more than 256
+                                      primaries: three rings of a quarter, at least 2^22 each) */
     int32_t kernel_timing;         /* 1: CUDA events around every kernel (per-kernel times in pach_stats) */
     int32_t ray_sort;              /* 1: order each wave by (direction octant, origin cell) before tracing;
                                       0 = default (off: measured +6 % walk rate in the 20k-triangle
@@ -380,7 +382,8 @@ pach_status pach_trace_specular_paths(pach_scene *scene, int32_t n, const double
 pach_status pach_scene_shoot_host(const pach_scene_desc *desc, int32_t n, const double *origins, const double *dirs,
                                   int32_t *poly_out, double *t_out);
 
-/* Receiver filters (auralisation impulse responses), computed on the GPU in FP64.
+/* Receiver filters (auralisation impulse responses), computed on the GPU: T + 16383 <= 65536
+ * by exact integer transforms of values scaled to 62 bits, longer ones by FP64 transforms.
  * pach_etc_to_filter: Pach_SP.ETCToFilter (Pach_SP.cs:1584-1680) of n band-pressure envelope sets
  *   prms [n][8][T] at sample_rate Hz: out [n][T + 16383].  Each band's |P| 10^((120 - swl[b]) / 20) is
  *   convolved with a 16384-sample band-limited sinc carrier, plus a 16 kHz band from the 8 kHz

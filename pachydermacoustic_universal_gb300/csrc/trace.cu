@@ -17,6 +17,10 @@
 //                absorption, one Philox draw block, Scatter_Late (phase B, 4629-4701) or
 //                Scatter_VeryLate (phase C, 4572-4627), then the surviving ray and a split child are
 //                appended to the ring with one atomic per warp (TaskAll:429-536).
+//   k_map        with mapping receivers: the wave's receiver-grid walks, beside k_shade.
+//   k_bounce     small scenes without mapping receivers, instead of the last three: walk and shade, a ray staying
+//                in its lane over up to 32 interactions.
+// A run of more than 256 primaries is several such loops, each over a share of them (run_worker_body).
 // Random numbers are Philox4x32-10 streams keyed by (seed, primary, stream id, block): the streams
 // the CPU oracle draws, so a ray's decisions do not depend on scheduling.
 #include "device_common.cuh"
@@ -998,7 +1002,8 @@ __global__ void __launch_bounds__(256, 3) k_map(DevRun r) {
 // Bound: issue (61 % of slots, 19.6 of 32 lanes active: interactions differ) at three blocks an SM; two or four
 // blocks 848 and 834 ms where three take 753.  One interaction a
 // launch read and wrote every ray (128 bytes) and appended it each time, and a chain of 200 interactions was 200
-// waves: a 1003-primary shoebox took 228 waves and 19.1 ms, now 30 and 9.6 ms; 100k primaries 1180 ms, now 753.
+// waves: a 1003-primary shoebox took 228 waves and 19.1 ms, now 30 and 9.6 ms (in three loops 8.7); 100k primaries 1180
+// ms, then 753, now 733.
 //
 // Detections wait in a queue of the warp until 32 are there, so that a lane's detection (FP64 time and bin, six
 // atomics) does not hold the other 31: in a 3-receiver shoebox 3 % of the segments, two of three iterations.
