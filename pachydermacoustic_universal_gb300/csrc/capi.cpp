@@ -700,10 +700,7 @@ void run_worker_body(pach_run *run) {
         if (!quant) S.bvhq = nullptr;  // trace_ray walks whichever node array is set
         const int tr_variant = trace_variant(run->p.blocks_per_sm, run->p.traversal, ntri_max, quant);
         const bool fused = fused_walk(run->p.traversal, ntri_max) && run->p.ray_sort <= 0;
-        size_t rec_max = 0;
-        for (const RoomSpec &rm : run->rooms) rec_max = std::max(rec_max, rm.rec.size());
-        const bool wide = rec_max >= (size_t)kShadeWideReceivers;
-        TRY(wave_kernel_occupancy(tr_variant, threads, receiver_smem_bytes(R), &bps_tr, &bps_sh, fused, wide));
+        TRY(wave_kernel_occupancy(tr_variant, threads, receiver_smem_bytes(R), &bps_tr, &bps_sh, fused));
         const bool bounce = fused && !map;
         const bool by_planes = bounce && *std::min_element(planes.begin(), planes.end()) > 0;
         if (bounce) TRY(bounce_occupancy(threads, receiver_smem_bytes(R), &bps_sh, by_planes));
@@ -721,8 +718,9 @@ void run_worker_body(pach_run *run) {
         // Pipes: the primaries are shared out to independent device loops on streams of their own, so that the ends of
         // one's waves (60 us in which the last rays finish, of the 150 to 550 us of an iteration) and its launches
         // overlap the others' work.  Device time with 1 / 2 / 3 / 4 loops: hall of 20k triangles, 2500 primaries and
-        // an audience map 46.8 / 45.0 / 42.3 / 43.5 ms; 20k primaries 145 / 143.5 / 142.5 / 140.9; arena of 500k
-        // triangles, 60k primaries 95 / 91.5 / 91.3 / 91.1; 8 small rooms of 500 primaries 287 / - / 248 / -.  Below a
+        // an audience map 36.1 / 33.5 / 32.2 / 34.0 ms; 20k primaries 128.1 / 127.9 / 124.4 / 123.4; arena of 500k
+        // triangles, 60k primaries 82.5 / 82.5 / 79.9 / 80.2; 8 small rooms of 500 primaries 254 / 227 / 218 / 220;
+        // shoebox, 1003 primaries 8.7 with three, 8.3 with four.  Below a
         // pilot's size there is one wave front to share and more loops only split it (hall, 128 primaries: 8.7 ms with
         // one, 9.2 with two; 300: 13.6, 9.7, with three 9.3).  Runs that the caller shapes (ring, feed, sorted
         // waves, kernel times) and convergence runs, whose revolutions are smaller, keep one.
@@ -893,7 +891,7 @@ void run_worker_body(pach_run *run) {
                 if ((x = cudaEventRecord(q.join, q.side))) return x;
             }
             if ((x = bounce ? launch_bounce(r, sh_blocks, threads, stream, by_planes)
-                            : launch_shade(r, sh_blocks, threads, stream, fused, wide)))
+                            : launch_shade(r, sh_blocks, threads, stream, fused)))
                 return x;
             if (beside) x = cudaStreamWaitEvent(stream, q.join, 0);
             else if (map) x = launch_map(r, map_blocks, stream);

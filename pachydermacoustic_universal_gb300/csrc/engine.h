@@ -391,10 +391,7 @@ inline bool use_quantised_nodes(int bvh_format, int ntri) {
 cudaError_t launch_trace(const DevRun &r, int variant, int blocks, int threads, cudaStream_t s);
 // fused: k_shade walks the rays itself (no k_trace launch) -- the default for scenes of at most
 // kFuseMaxTris triangles, or traversal = 3
-// map: also detect the run's mapping receivers (kernel variants compiled with the grid walk)
-// wide: the shading variant with 4 blocks per SM, for rooms of at least kShadeWideReceivers receivers
-constexpr int kShadeWideReceivers = 48;
-cudaError_t launch_shade(const DevRun &r, int blocks, int threads, cudaStream_t s, bool fused = false, bool wide = false);
+cudaError_t launch_shade(const DevRun &r, int blocks, int threads, cudaStream_t s, bool fused = false);
 cudaError_t launch_map(const DevRun &r, int blocks, cudaStream_t s);
 // Blocks of the map's kernel per SM: it runs beside the shading kernel (two 36.9 ms, the three that fit 37.5 on the
 // hall with 2500 primaries).
@@ -423,7 +420,7 @@ cudaError_t launch_bounce(const DevRun &r, int blocks, int threads, cudaStream_t
 cudaError_t bounce_occupancy(int threads, int smem, int *blocks_per_sm, bool planes);
 inline bool fused_walk(int traversal, int ntri) { return traversal == 3 || (traversal == 0 && ntri <= kFuseMaxTris); }
 cudaError_t wave_kernel_occupancy(int variant, int threads, int smem_shade, int *bpsm_trace, int *bpsm_shade,
-                                  bool fused = false, bool wide = false);
+                                  bool fused = false);
 cudaError_t launch_paths(const DevScene &S, int n, const double *o, const double *d, int max_bounces, int *poly,
                          double *t, double *pts, cudaStream_t s);
 cudaError_t launch_emit(const DevRun &r, long long p0, int n, double *out, cudaStream_t s);

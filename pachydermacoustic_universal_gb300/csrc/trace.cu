@@ -785,15 +785,13 @@ __device__ __forceinline__ bool surface(const DevRun &r, const DevScene &S, cons
 
 // FUSED: walk the ray here instead of reading k_trace's hit (small scenes, whose walk is a few
 // cached nodes: the separate trace pass would only re-read the ray and round-trip its hit via HBM).
-// the shading pass alone fits three 256-thread blocks per SM (80 registers; +1.6 % on a 500k-triangle
-// arena, equal on a 20k-triangle hall); the fused walk, two (128 registers).  WIDE, for rooms of many
-// receivers: the grouped detection and four blocks per SM (64 registers, more spilled: the long
-// detection loop waits on its loads) -- on the 64-receiver arena -6 % shading time from the fourth
-// block, -28 % more from the grouped detection; on the 16-receiver hall +17 % and +12 %, so it keeps
-// three blocks and the plain loop.
-constexpr int kShadeMinBlocks = 3;
-template <bool FUSED, bool WIDE>
-__global__ void __launch_bounds__(256, FUSED ? 2 : (WIDE ? 4 : kShadeMinBlocks)) k_shade(DevRun r) {
+// The shading pass alone takes receivers four at a time through a cheap test, in four 256-thread blocks per SM (64
+// registers): on the 64-receiver arena -28 % and -6 % shading time against one at a time in three blocks.  Beside the
+// other loops' walks that holds from the fewest receivers on (hall, 10k primaries with 2 / 8 / 16 of them 66.1 / 67.0 /
+// 68.1 ms against 66.4 / 68.1 / 69.9; 20k primaries 121.0 against 124.4).  The fused walk: two blocks (128 registers),
+// one at a time.
+template <bool FUSED>
+__global__ void __launch_bounds__(256, FUSED ? 2 : 4) k_shade(DevRun r) {
     extern __shared__ float4 s_rec_buf[];
     const int *s_rid;
     const float4 *s_rec = stage_receivers(r, s_rec_buf, s_rid);
@@ -833,7 +831,7 @@ __global__ void __launch_bounds__(256, FUSED ? 2 : (WIDE ? 4 : kShadeMinBlocks))
             const float t = __int_as_float(h.y);
             ++L.v[R.phase == 0 ? C_SEGB : C_SEGC];
             const RoomParams &P = r.rooms[R.room];
-            L.v[C_DET] += detect_octave<WIDE>(r, P, s_rec, s_rid, R.p, R.d, hit ? t : 1e6f, R.t_sum, R.I * R.scale, R.oct,
+            L.v[C_DET] += detect_octave<!FUSED>(r, P, s_rec, s_rid, R.p, R.d, hit ? t : 1e6f, R.t_sum, R.I * R.scale, R.oct,
                                         R.mask, R.prim);
             if (!hit) {
                 // lost: no End_Trace after a miss in phase B (TaskAll:437-443), loop exit in phase C (500-505)
@@ -1317,10 +1315,9 @@ cudaError_t launch_trace(const DevRun &r, int variant, int blocks, int threads, 
     return cudaGetLastError();
 }
 
-cudaError_t launch_shade(const DevRun &r, int blocks, int threads, cudaStream_t s, bool fused, bool wide) {
-    if (fused) k_shade<true, false><<<blocks, threads, rec_smem(r), s>>>(r);
-    else if (wide) k_shade<false, true><<<blocks, threads, rec_smem(r), s>>>(r);
-    else k_shade<false, false><<<blocks, threads, rec_smem(r), s>>>(r);
+cudaError_t launch_shade(const DevRun &r, int blocks, int threads, cudaStream_t s, bool fused) {
+    if (fused) k_shade<true><<<blocks, threads, rec_smem(r), s>>>(r);
+    else k_shade<false><<<blocks, threads, rec_smem(r), s>>>(r);
     return cudaGetLastError();
 }
 
@@ -1341,7 +1338,7 @@ cudaError_t bounce_occupancy(int threads, int smem, int *blocks_per_sm, bool pla
 }
 
 cudaError_t wave_kernel_occupancy(int variant, int threads, int smem_shade, int *bpsm_trace, int *bpsm_shade,
-                                  bool fused, bool wide) {
+                                  bool fused) {
     cudaError_t e;
     switch (variant) {
 #define PACH_OCC(M, SP, Q)                                                                           \
@@ -1353,9 +1350,8 @@ cudaError_t wave_kernel_occupancy(int variant, int threads, int smem_shade, int 
         default: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(bpsm_trace, k_trace<4, false, false>, threads, 0); break;
     }
     if (e != cudaSuccess) return e;
-    if (fused) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(bpsm_shade, k_shade<true, false>, threads, smem_shade);
-    if (wide) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(bpsm_shade, k_shade<false, true>, threads, smem_shade);
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(bpsm_shade, k_shade<false, false>, threads, smem_shade);
+    return fused ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(bpsm_shade, k_shade<true>, threads, smem_shade)
+                 : cudaOccupancyMaxActiveBlocksPerMultiprocessor(bpsm_shade, k_shade<false>, threads, smem_shade);
 }
 
 cudaError_t launch_scale(double *dst, const double *src, size_t n, double f, const double *rows, size_t per_row,
