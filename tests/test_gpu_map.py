@@ -16,7 +16,8 @@ import numpy as np
 import pytest
 
 from oracle import oracle as O
-from pachydermacoustic_universal_gb300 import _capi, rooms, tracer
+from pachydermacoustic_universal_gb300 import rooms, tracer
+from pachydermacoustic_universal_gb300 import _capi
 from pachydermacoustic_universal_gb300.simulation import AcousticalMath
 
 pytestmark = pytest.mark.gpu
