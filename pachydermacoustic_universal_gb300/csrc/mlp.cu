@@ -31,6 +31,7 @@
 #include <vector>
 
 #include "engine.h"
+#include "mlp_plan.h"
 #include "../../include/pach_proposal.h"
 
 namespace pach {
@@ -50,7 +51,7 @@ constexpr int kOperandBytes = kTile * kChunk * 2;        // one 128 x 128 BF16 b
 // kernel's time is its epilogue and its latencies, not its MMAs: 32 columns give 80 CTAs for 1200 rows
 // where 256 gave 10, and the epilogue went from 50 us to 2-3 us with them.
 constexpr int kCols = 32;
-constexpr int kMaxSplits = 16;                           // row ranges of the weight-gradient products
+static_assert(kChunk == kRowChunk, "row ranges are whole chunks");
 __host__ __device__ constexpr int stage_bytes(int cols) { return kOperandBytes + cols * kChunk * 2; }
 __host__ __device__ constexpr int smem_bytes(int cols) { return kStages * stage_bytes(cols) + 256 + 1024; }
 constexpr int kTransStride = kTile + 8;                  // transposed BF16 tile: 272-byte rows, no bank conflicts
@@ -682,15 +683,6 @@ cudaError_t launch_gemm(const Gemm &g, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-// Row ranges of the weight gradients for Mp rows: at least 256 rows each (two chunks in flight), at most
-// kMaxSplits, whose sums the optimiser reads.  1200 rows: 7 us in five ranges and 1 us more in k_adam,
-// 14.5 us in one.
-int wgrad_rows_per(int Mp) {
-    const int s = std::max(1, std::min(kMaxSplits, Mp / 256));
-    return round_up((Mp + s - 1) / s, kChunk);
-}
-int wgrad_splits(int Mp) { return (Mp + wgrad_rows_per(Mp) - 1) / wgrad_rows_per(Mp); }
-
 struct Buf {
     void *p = nullptr;
     cudaError_t alloc(size_t bytes) {
@@ -1024,7 +1016,7 @@ pach_status pach_mlp_create(uint64_t seed, int32_t max_rows, pach_mlp **out) {
         MTRY(m->m1.alloc(m->n_dev * F));
         MTRY(m->m2.alloc(m->n_dev * F));
         MTRY(m->g.alloc(m->n_dev * F));
-        MTRY(m->part.alloc((size_t)wgrad_splits(Mp) * m->n_dev * F));
+        MTRY(m->part.alloc((size_t)wgrad_splits_max(Mp) * m->n_dev * F));  // training may set fewer rows
         MTRY(cudaMallocHost(&m->h_err, sizeof(int)));
         MTRY(m->decay.alloc(m->n_dev));
         MTRY(m->step.alloc(sizeof(int)));

@@ -71,6 +71,29 @@ def test_gradient_at_tile_and_range_edges(rows):
     assert loss2 == loss and np.linalg.norm(g2 - g) <= 1e-5 * np.linalg.norm(g)
 
 
+@pytest.mark.parametrize("max_rows,rows", [(1100, 1000), (2176, 2048), (4200, 4096)])
+def test_fewer_rows_than_the_network_holds(max_rows, rows):
+    """Fewer rows can take more row ranges than the most the network was made for (4 against 3, 8 against 6, 16
+    against 11): the gradient equals a network's made for just these rows (weights bit for bit, the ranges' sums
+    have a fixed order; biases are FP32 atomics over the rows: 1e-5), and training steps agree."""
+    nets = [proposal.ProposalNet(seed=5, max_rows=n) for n in (max_rows, rows)]
+    cond, target = _problem(rows, seed=rows)
+    got = []
+    for net in nets:
+        net.set_data(cond, target)
+        got.append(net.loss_grad())
+    (la, ga), (lb, gb) = got
+    assert la == lb
+    at = 0
+    for n, k in MO.LAYERS:
+        assert np.array_equal(ga[at:at + n * k], gb[at:at + n * k])
+        assert np.linalg.norm(ga[at + n * k:at + n * k + n] - gb[at + n * k:at + n * k + n]) <= \
+            1e-5 * np.linalg.norm(gb[at + n * k:at + n * k + n])
+        at += n * k + n
+    ca, cb = (net.train(3, lr=1e-3) for net in nets)
+    assert np.all(np.isfinite(ca)) and ca[0] == cb[0] and np.allclose(ca, cb, rtol=2e-3)
+
+
 def test_training_reduces_loss_and_forward_is_consistent():
     net = proposal.ProposalNet(seed=3, max_rows=512)
     rng = np.random.default_rng(9)
