@@ -233,7 +233,11 @@ __device__ __forceinline__ FitSums fit_products(const double *cum, const double 
 // 3000 bins: 160 us (FP64 pipe 64 % busy), where a logarithm a bin in two of three passes took 1155 us (85 %
 // busy).  A curve with a negative, infinite or undefined value or without energy goes to curve_general.
 constexpr int kSharedBins = 6000;  // 48 KB: four curves an SM still keep the FP64 pipe half busy
-__host__ __device__ inline int chunk_bins(int T) { return ((T + 63) / 64) | 1; }
+constexpr int kFourBytes = 27 * 1024;  // curves up to this size go four to a block
+// Most dynamic shared memory of a launch.  The kernel's limit is one value for the whole device and every call sets
+// it to this, whatever its own curves need: a call with longer curves on another thread launches in between.
+constexpr int kMaxSharedBytes = 4 * kFourBytes;
+__host__ __device__ constexpr int chunk_bins(int T) { return ((T + 63) / 64) | 1; }
 
 // what every curve of a launch shares
 struct Curves {
@@ -365,9 +369,10 @@ cudaError_t launch_map_params(const double *etc, int n, int T, double fs, double
     const Out o{t_x, edt, clarity, definition, sum};
     if (T <= kSharedBins) {
         const int per = 64 * chunk_bins(T) * (int)sizeof(double);
-        const int warps = per <= 27 * 1024 ? 4 : 1;
+        const int warps = per <= kFourBytes ? 4 : 1;
+        static_assert(64 * chunk_bins(kSharedBins) * sizeof(double) <= kMaxSharedBytes, "one curve a block");
         const cudaError_t e = cudaFuncSetAttribute(k_curve_params, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   warps * per);
+                                                   kMaxSharedBytes);
         if (e != cudaSuccess) return e;
         const double bw = 1.0 / fs;
         Curves k;

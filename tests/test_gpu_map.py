@@ -10,6 +10,7 @@ Tolerances, stated per test:
   JND (5 % T30/EDT, 1 dB C80, 5 points D50) where both sides are finite;
 * the device parameter kernel against the host AcousticalMath on the same histograms: 1e-9 relative.
 """
+import threading
 import types
 
 import numpy as np
@@ -175,6 +176,33 @@ def test_parameter_kernel_over_curve_lengths_and_kinds(T, depth, cms):
                    "definition": AcousticalMath.Definition(etc[i], 1000, 0.05, 0.0, False), "energy": etc[i].sum()}
             for k, v in ref.items():
                 np.testing.assert_allclose(out[k][i], v, rtol=1e-9, atol=1e-300, equal_nan=True, err_msg=f"{k} {i}")
+
+
+def test_parameters_of_different_lengths_on_two_threads():
+    """Calls on several host threads share the kernel's shared-memory limit: curves of 300 bins (10 KB a block) beside
+    curves of 3000 (96 KB) and of 6000 (48 KB for one), each call as if alone."""
+    L = _capi.lib()
+    rng = np.random.default_rng(2)
+    wrong = []
+
+    def work(T, reps):
+        etc = np.ascontiguousarray(np.exp(-np.arange(T) / (0.2 * T)) * rng.gamma(0.5, 1.0, (4, T)))
+        first = None
+        for _ in range(reps):
+            out = [np.zeros(4) for _ in range(5)]
+            s = L.pach_etc_parameters(_capi.dptr(etc), 4, T, 1000, 30, 0.08, *(_capi.dptr(v) for v in out))
+            first = out if first is None else first
+            if s != 0 or any(not np.array_equal(a, b, equal_nan=True) for a, b in zip(out, first)):
+                wrong.append((T, s))
+                return
+
+    work(300, 1)  # the context is there before the threads start
+    ts = [threading.Thread(target=work, args=(T, 1500)) for T in (300, 3000, 300, 6000)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not wrong, wrong
 
 
 def test_one_point_map_matches_oracle():
