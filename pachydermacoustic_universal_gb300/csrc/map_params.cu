@@ -231,7 +231,8 @@ __device__ __forceinline__ FitSums fit_products(const double *cum, const double 
 // running sums, a scan makes them the Schroeder curve, the fit limits are binary searches on it (energies are not negative, so it falls monotonically; the
 // limits in dB are compared as ratios) and the fits are products (fit_products).  608 receivers x 8 bands x
 // 3000 bins: 160 us (FP64 pipe 64 % busy), where a logarithm a bin in two of three passes took 1155 us (85 %
-// busy).  A curve with a negative, infinite or undefined value or without energy goes to curve_general.
+// busy).  A curve with a negative, infinite or undefined value, or whose total is not above zero or has no finite
+// reciprocal, goes to curve_general.
 constexpr int kSharedBins = 6000;  // 48 KB: four curves an SM still keep the FP64 pipe half busy
 constexpr int kFourBytes = 27 * 1024;  // curves up to this size go four to a block
 // Most dynamic shared memory of a launch.  The kernel's limit is one value for the whole device and every call sets
@@ -242,6 +243,7 @@ __host__ __device__ constexpr int chunk_bins(int T) { return ((T + 63) / 64) | 1
 // what every curve of a launch shares
 struct Curves {
     double limit[4];         // curve values at the fits' limits: T_X first and second, EDT first and second
+    double db[4];            // the limits themselves
     double split_c, split_d; // shares of the boundary bins ei_c, ei_d that are early
     double inv_fs;
     int ei_c, ei_d;
@@ -287,22 +289,33 @@ __global__ void __launch_bounds__(128) k_curve_params(const double *etc, int n, 
     base[lane] = lane ? before : 0.0;
     base[lane + 32] = half + (lane ? before2 : 0.0);
     const double tot = half + __shfl_sync(FULL, incl2, 31);
-    if (__any_sync(FULL, odd) || !(tot > 0.0) || isinf(tot)) {
+    const double rt = 1.0 / tot;
+    if (__any_sync(FULL, odd) || !(tot > 0.0) || isinf(tot) || isinf(rt)) {
         curve_general(x, w, T, fs, scale, depth, clar_s, o);
         return;
     }
     __syncwarp();
-    const double rt = 1.0 / tot;
     auto sum_to = [&](int i) { return base[i / c] + cum[i]; };  // bins 0 .. i
     // fit limits: first bin >= 1 below each level (lanes 0-3: T_X first and second, EDT first and second)
-    const double th = k.limit[lane & 3];
-    int lo = 1, hi = T;
-    if (lane < 4)
+    const double th = k.limit[lane & 3], db = k.db[lane & 3];
+    auto first_where = [&](auto below) {
+        int lo = 1, hi = T;
         while (lo < hi) {
             const int mid = (lo + hi) >> 1;
-            if (fma(-sum_to(mid), rt, 1.0) < th) hi = mid;
+            if (below(mid)) hi = mid;
             else lo = mid + 1;
         }
+        return lo;
+    };
+    auto curve = [&](int i) { return fma(-sum_to(i), rt, 1.0); };
+    int lo = T;
+    if (lane < 4) {
+        lo = first_where([&](int i) { return curve(i) < th; });
+        // A bin within rounding of the limit (steps of equal bins: 1 - 99 / 100 at -20 dB) is decided by the quotient
+        // and the logarithm, as curve_general does.
+        if ((lo < T && fabs(curve(lo) - th) < 1e-14) || (lo > 1 && fabs(curve(lo - 1) - th) < 1e-14))
+            lo = first_where([&](int i) { return level(1.0 - sum_to(i) / tot, i) < db; });
+    }
     // not found: index 0, as the reference's loops leave them; a fit of one bin or less has no slope
     const int f0 = __shfl_sync(FULL, lo, 0), f1 = __shfl_sync(FULL, lo, 1), f2 = __shfl_sync(FULL, lo, 2),
               f3 = __shfl_sync(FULL, lo, 3);
@@ -376,10 +389,11 @@ cudaError_t launch_map_params(const double *etc, int n, int T, double fs, double
         if (e != cudaSuccess) return e;
         const double bw = 1.0 / fs;
         Curves k;
-        k.limit[0] = level_ratio(-5.0);
-        k.limit[1] = level_ratio(-5.0 - std::fabs((double)decay_depth));
-        k.limit[2] = level_ratio(-1.0);
-        k.limit[3] = level_ratio(-10.0001);
+        k.db[0] = -5.0;
+        k.db[1] = -5.0 - std::fabs((double)decay_depth);
+        k.db[2] = -1.0;
+        k.db[3] = -10.0001;
+        for (int i = 0; i < 4; ++i) k.limit[i] = level_ratio(k.db[i]);
         k.ei_c = (int)std::floor((clarity_s + 0.0) * fs);
         k.ei_d = (int)std::floor(0.05 * fs);
         k.split_c = (clarity_s + 0.0 - k.ei_c * bw) / bw;

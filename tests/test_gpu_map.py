@@ -178,6 +178,31 @@ def test_parameter_kernel_over_curve_lengths_and_kinds(T, depth, cms):
                 np.testing.assert_allclose(out[k][i], v, rtol=1e-9, atol=1e-300, equal_nan=True, err_msg=f"{k} {i}")
 
 
+@pytest.mark.parametrize("T,depth", [(10, 5), (100, 15), (200, 15), (1000, 15), (1000, 25), (400, 30), (6000, 55)])
+@pytest.mark.parametrize("scale", [1.0, 2.0**-1060])
+def test_fit_limits_at_steps_that_meet_them(T, depth, scale):
+    """Equal bins, whose Schroeder curve 1 - k / T meets round limits within rounding (100 bins: 1 - 99 / 100 is
+    above -20 dB), a plateau at such a step, and the same curves with subnormal totals: the limits are those of
+    AcousticalMath's own quotient and logarithm, and with the limits the slopes.  Sums of whole numbers are exact,
+    so 1e-9 as in the other comparisons.  A step whose level equals the limit in the last bit of the logarithm
+    (10 bins at -10 dB) may fall on either side: those curves are left out where the host's level is the limit."""
+    curves = [np.ones(T), np.concatenate([np.ones(T - 10), np.zeros(50), np.ones(10)])[:T + 50]]
+    L = _capi.lib()
+    for c in curves:
+        n = c.size
+        etc = np.ascontiguousarray(c * scale)[None]
+        sch = AcousticalMath.Schroeder_Integral(etc[0])
+        with np.errstate(all="ignore"):
+            lev = 10.0 * np.log10(sch)
+        if np.any(lev == -5.0 - depth):
+            continue
+        out = {k: np.zeros(1) for k in ("t_x", "edt", "clarity", "definition", "energy")}
+        _capi.check(L.pach_etc_parameters(_capi.dptr(etc), 1, n, 1000, depth, 0.08, *(_capi.dptr(v) for v in out.values())))
+        np.testing.assert_allclose(out["t_x"][0], AcousticalMath.T_X(sch, depth, 1000), rtol=1e-9, equal_nan=True)
+        np.testing.assert_allclose(out["edt"][0], AcousticalMath.EarlyDecayTime(sch, 1000), rtol=1e-9, equal_nan=True)
+        assert out["energy"][0] == etc.sum()
+
+
 def test_parameters_of_different_lengths_on_two_threads():
     """Calls on several host threads share the kernel's shared-memory limit: curves of 300 bins (10 KB a block) beside
     curves of 3000 (96 KB) and of 6000 (48 KB for one), each call as if alone."""
