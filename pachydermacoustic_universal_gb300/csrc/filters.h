@@ -19,7 +19,6 @@ struct FilterJob {
 // than the 8 kHz one.
 bool ntt_supported(int T);
 size_t ntt_workspace_bytes(int n_filters, int T);
-size_t ntt_workspace_min(int T);
 cudaError_t ntt_filters(FilterJob J, int n, int fs, double add, int L, double *out, void *ws, size_t ws_bytes,
                         cudaStream_t st);
 

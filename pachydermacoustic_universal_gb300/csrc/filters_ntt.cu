@@ -629,6 +629,10 @@ size_t fixed_layout(char *base, Bufs &B, int T, int W) {
     return off;
 }
 
+// Filters at a time, however much workspace there is: their buffers stay within L2, and k_ntt_env's grid (eight rows a
+// receiver) within 65535.
+size_t chunk_max(size_t job) { return std::max<size_t>(1, std::min<size_t>(kChunkBytes / job, 65535 / 8 - 1)); }
+
 size_t job_bytes(int T, int W) {
     return align_up((size_t)9 * T * 8 + (size_t)kPrimes * 9 * T * 4 + (size_t)kPrimes * W * 4 + 4) + 1024;
 }
@@ -641,11 +645,8 @@ size_t ntt_workspace_bytes(int n_filters, int T) {
     Bufs B{};
     const int W = transform_len(T);
     const size_t pj = job_bytes(T, W);
-    const size_t chunk = std::max<size_t>(1, std::min<size_t>((size_t)n_filters, kChunkBytes / pj));
-    return fixed_layout(nullptr, B, T, W) + chunk * pj;
+    return fixed_layout(nullptr, B, T, W) + std::min<size_t>((size_t)n_filters, chunk_max(pj)) * pj;
 }
-
-size_t ntt_workspace_min(int T) { return ntt_workspace_bytes(1, T); }
 
 cudaError_t ntt_filters(FilterJob J, int n, int fs, double add, int L, double *out, void *ws, size_t ws_bytes,
                         cudaStream_t st) {
@@ -654,7 +655,7 @@ cudaError_t ntt_filters(FilterJob J, int n, int fs, double add, int L, double *o
     char *base = static_cast<char *>(ws);
     size_t off = fixed_layout(base, B, T, W);
     const size_t pj = job_bytes(T, W);
-    const int chunk = (int)std::min<size_t>((size_t)n, std::min<size_t>((ws_bytes - off) / pj, 16384));
+    const int chunk = (int)std::min<size_t>(std::min<size_t>((size_t)n, (ws_bytes - off) / pj), chunk_max(pj));
     lay(base, off, B.env, (size_t)chunk * 9 * T);
     lay(base, off, B.res, (size_t)chunk * kPrimes * 9 * T);
     lay(base, off, B.y, (size_t)chunk * kPrimes * W);

@@ -142,6 +142,29 @@ def test_device_form_in_several_passes_equals_one_pass():
     _close(outs[0], ref)
 
 
+def _device_filters(P, wsb):
+    torch = pytest.importorskip("torch")
+    dev = torch.device("cuda:0")
+    n, _, T = P.shape
+    p, ws = torch.from_numpy(P).to(dev), torch.empty(wsb, dtype=torch.uint8, device=dev)
+    out = torch.full((n, T + 16383), np.nan, dtype=torch.float64, device=dev)
+    _capi.check(_capi.lib().pach_filters_device(None, p.data_ptr(), None, None, None, n, T, 1, 1000, None, 0, out.data_ptr(),
+                                                ws.data_ptr(), wsb, C.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    torch.cuda.synchronize()
+    return out
+
+
+def test_a_workspace_for_thousands_of_filters_equals_the_recommended_one():
+    """More single filters than a launch's grid has rows for, with room for all of them at once (2.7 GB)."""
+    n = 8200
+    P = np.random.default_rng(5).random((n, 8, 1))
+    recommended = _capi.lib().pach_filters_workspace_bytes(n, 1)
+    one = _capi.lib().pach_filters_workspace_bytes(1, 1)
+    a, b = _device_filters(P, recommended), _device_filters(P, one + n * 330_000)
+    assert bool((a == b).all())
+    _close(b[n - 1].cpu().numpy(), F.etc_to_filter(P[n - 1], [120] * 8, 1000))
+
+
 def test_receiver_bank_create_filter_after_a_split_ray_tracer_run():
     w = rooms.shoebox_c1()
     room = Polygon_Scene.from_arrays(w.scene)
