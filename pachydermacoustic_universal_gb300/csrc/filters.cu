@@ -402,7 +402,10 @@ pach_status filters_device(const double *E, const double *P, const double *Dp, c
     }
     const Geom g = make_geom(T);
     const size_t fixed = fixed_bytes(g, T), pj = per_job_bytes(g);
-    if (ws_bytes < filters_workspace_bytes(1, T))
+    // one filter's integer transforms take two to three times the FP64 ones' workspace: less than theirs, but enough
+    // for the FP64 ones, goes to those
+    const bool ntt = ntt_supported(T) && ws_bytes >= ntt_workspace_bytes(1, T);
+    if (!ntt && ws_bytes < fixed + pj)
         return ffail(PACH_ERR_INVALID_ARGUMENT, "workspace smaller than one filter needs");
     const int n = R * kinds;
     Work w{};
@@ -420,7 +423,7 @@ pach_status filters_device(const double *E, const double *P, const double *Dp, c
     J.kinds = kinds;
     // up to 65536 points the integer transforms are the faster ones (448 filters of 32768 points: 2.4 against
     // 11.2 ms; one filter 0.12 against 0.45 ms) and no less exact; the FP64 transforms take any length
-    if (ntt_supported(T)) {
+    if (ntt) {
         const cudaError_t e = ntt_filters(J, n, fs, hf_extra_attenuation(), L, out, ws, ws_bytes, st);
         return e == cudaSuccess ? PACH_OK : cuda_fail(e, "filter kernels");
     }

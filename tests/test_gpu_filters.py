@@ -165,6 +165,20 @@ def test_a_workspace_for_thousands_of_filters_equals_the_recommended_one():
     _close(b[n - 1].cpu().numpy(), F.etc_to_filter(P[n - 1], [120] * 8, 1000))
 
 
+@pytest.mark.parametrize("T,least", [(1, 5112064), (500, 9048064), (3500, 9072128), (16386, 17039616), (49153, 17301760)])
+def test_workspaces_of_the_fp64_transforms_are_still_taken(T, least):
+    """A workspace too small for one filter's integer transforms but large enough for its FP64 ones (`least` bytes, by
+    their layout) is taken, a byte less refused; the longest length with integer transforms and the first of each
+    transform length."""
+    assert _capi.lib().pach_filters_workspace_bytes(1, T) > least
+    P = np.random.default_rng(T).random((2, 8, T))
+    got = _device_filters(P, least).cpu().numpy()
+    for i in range(2):
+        _close(got[i], F.etc_to_filter(P[i], [120] * 8, 1000))
+    with pytest.raises(_capi.PachError):
+        _device_filters(P, least - 1)
+
+
 def test_receiver_bank_create_filter_after_a_split_ray_tracer_run():
     w = rooms.shoebox_c1()
     room = Polygon_Scene.from_arrays(w.scene)
