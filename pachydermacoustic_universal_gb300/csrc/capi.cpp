@@ -18,35 +18,9 @@
 #include <tuple>
 #include <vector>
 
-#include <unistd.h>
-
 #include "engine.h"
 
 using namespace pach;
-
-void pach::touch_pages(const std::vector<std::pair<void *, size_t>> &ranges) {
-    const size_t page = (size_t)std::max(4096l, sysconf(_SC_PAGESIZE));
-    std::vector<std::pair<char *, size_t>> runs;  // first byte to write, pages
-    size_t total = 0;
-    for (const auto &r : ranges) {
-        if (!r.first || r.second < page) continue;  // too small to matter
-        runs.emplace_back(static_cast<char *>(r.first), (r.second + page - 1) / page);
-        total += runs.back().second;
-    }
-    auto touch = [&](size_t a, size_t b) {
-        size_t first = 0;
-        for (const auto &r : runs) {
-            for (size_t i = std::max(a, first); i < std::min(b, first + r.second); ++i)
-                *const_cast<volatile char *>(r.first + (i - first) * page) = 0;
-            first += r.second;
-        }
-    };
-    try {
-        parallel_chunks(total, std::max<size_t>(1, (size_t(2) << 20) / page), touch);
-    } catch (const std::exception &) {
-        // no thread to be had: the copy faults the pages in
-    }
-}
 
 namespace {
 

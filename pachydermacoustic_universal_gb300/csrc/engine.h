@@ -76,9 +76,11 @@ void parallel_chunks(size_t n, size_t grain, F &&f) {
     for (auto &p : parts) p.get();
 }
 
-// Writes one byte of every page of the given host ranges, on several threads when there are many: memory
-// that the caller has just allocated gets its pages here.  Left to the copy they are faulted in by the
-// GPU one after another, 55 us each (34 MB of fresh histogram arrays: 30 ms, against 3 ms touched).
+// Gives every page of the given host ranges its memory, on several threads when there are many, and changes
+// nothing in them: what is there stays when the copy then fails, when a range is an input of a copy still on its
+// way, and beside another thread's writes.  Memory that the caller has just allocated gets its pages here; left
+// to the copy they are faulted in by the GPU one after another, 55 us each (34 MB of fresh histogram arrays: 30 ms,
+// against 3 ms).
 void touch_pages(const std::vector<std::pair<void *, size_t>> &ranges);
 
 // Host-side prepared scene (FP64 master copy + FP32 device layout sources).
