@@ -104,7 +104,7 @@ struct pach_run {
     bool conv_converged = false;
     std::vector<ConvCheck> conv_checks;
     DevMem conv, bak[6];
-    // scaled copies on their way to the host (one caller at a time)
+    // scaled copies and parameter maps on their way to the host (one caller at a time), at most kStageBytes
     DevMem stage;
     std::mutex stage_mu;
     // independent device loops the run's primaries were shared out to, and the feed positions each has finished
@@ -169,25 +169,33 @@ long long room_done(const pach_run *run, int i, long long done) {
     return sum;
 }
 
-// Copies n doubles to the host scaled by f, or by rows[i / per_row] (device): scaled on the device into
-// the run's staging buffer, or on the host when that cannot be had.
+// Copies n doubles to the host scaled by f, or by rows[i / per_row] (device): scaled on the device in pieces of a
+// staging buffer, or on the host when that cannot be had.
+constexpr size_t kStageBytes = size_t(64) << 20;
 cudaError_t download_scaled(pach_run *run, double *dst, const double *src, size_t n, double f,
                             const std::vector<double> &rows, size_t per_row) {
     std::lock_guard<std::mutex> lk(run->stage_mu);
-    const size_t need = (n + rows.size()) * sizeof(double);
-    if (run->stage.bytes < need && run->stage.alloc(need) != cudaSuccess) {
-        cudaGetLastError();
-        run->stage.bytes = 0;
+    const size_t all = kStageBytes / sizeof(double);
+    const bool fits = rows.size() < all / 2;
+    const size_t piece = std::min(n, all - (fits ? rows.size() : 0)), need = (piece + rows.size()) * sizeof(double);
+    if (!fits || (run->stage.bytes < need && run->stage.alloc(need) != cudaSuccess)) {
+        if (fits) {
+            cudaGetLastError();
+            run->stage.bytes = 0;
+        }
         const cudaError_t e = cudaMemcpy(dst, src, n * sizeof(double), cudaMemcpyDeviceToHost);
         if (e == cudaSuccess)
             for (size_t i = 0; i < n; ++i) dst[i] *= rows.empty() ? f : rows[i / per_row];
         return e;
     }
-    double *st = run->stage.as<double>(), *dr = rows.empty() ? nullptr : st + n;
+    double *dr = rows.empty() ? nullptr : run->stage.as<double>(), *st = run->stage.as<double>() + rows.size();
     cudaError_t e = cudaSuccess;
     if (dr) e = cudaMemcpy(dr, rows.data(), rows.size() * sizeof(double), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = launch_scale(st, src, n, f, dr, per_row, nullptr);
-    if (e == cudaSuccess) e = cudaMemcpy(dst, st, n * sizeof(double), cudaMemcpyDeviceToHost);
+    for (size_t i = 0; i < n && e == cudaSuccess; i += piece) {
+        const size_t m = std::min(piece, n - i);
+        e = launch_scale(st, src + i, m, f, dr, i, per_row, nullptr);
+        if (e == cudaSuccess) e = cudaMemcpy(dst + i, st, m * sizeof(double), cudaMemcpyDeviceToHost);
+    }
     return e;
 }
 
@@ -1822,10 +1830,10 @@ pach_status pach_map_parameters(pach_run *run, int32_t decay_depth, int32_t clar
         const int n = g.M * kBands;
         cudaSetDevice(run->scene->device);
         std::lock_guard<std::mutex> lk(run->stage_mu);
-        const size_t bytes = (size_t)5 * n * sizeof(double);
-        cudaError_t e = cudaSuccess;
-        if (run->stage.bytes < bytes) {
-            e = run->stage.alloc(bytes);
+        // curves at a time: their five results fit the staging buffer
+        const int piece = (int)std::min<size_t>((size_t)n, kStageBytes / (5 * sizeof(double)));
+        if (run->stage.bytes < (size_t)5 * piece * sizeof(double)) {
+            const cudaError_t e = run->stage.alloc((size_t)5 * piece * sizeof(double));
             if (e != cudaSuccess) {
                 run->stage.bytes = 0;
                 return fail(PACH_ERR_OUT_OF_MEMORY, cuda_msg(e, "parameter map buffers"));
@@ -1833,15 +1841,18 @@ pach_status pach_map_parameters(pach_run *run, int32_t decay_depth, int32_t clar
         }
         double *d = run->stage.as<double>();
         const double scale = (double)run->nsrc / (double)std::max(1ll, run->rays_done.load());
-        e = launch_map_params(run->mE.as<double>(), n, g.T, 1000.0, scale, decay_depth, clarity_ms / 1000.0, d, d + n,
-                              d + 2 * (size_t)n, d + 3 * (size_t)n, d + 4 * (size_t)n, nullptr);
-        if (e != cudaSuccess) return fail(PACH_ERR_CUDA, cuda_msg(e, "parameter map kernel"));
-        hvec<double> host((size_t)5 * n);  // the five maps in one copy
-        e = cudaMemcpy(host.data(), d, bytes, cudaMemcpyDeviceToHost);
-        if (e != cudaSuccess) return fail(PACH_ERR_CUDA, cuda_msg(e, "parameter map copy"));
         double *dst[5] = {t_x, edt, clarity, definition, energy_sum};
-        for (int i = 0; i < 5; ++i)
-            if (dst[i]) std::memcpy(dst[i], host.data() + (size_t)i * n, (size_t)n * sizeof(double));
+        hvec<double> host((size_t)5 * piece);  // the five maps in one copy
+        for (int c = 0; c < n; c += piece) {
+            const size_t m = (size_t)std::min(piece, n - c);
+            cudaError_t e = launch_map_params(run->mE.as<double>() + (size_t)c * g.T, (int)m, g.T, 1000.0, scale, decay_depth,
+                                              clarity_ms / 1000.0, d, d + m, d + 2 * m, d + 3 * m, d + 4 * m, nullptr);
+            if (e != cudaSuccess) return fail(PACH_ERR_CUDA, cuda_msg(e, "parameter map kernel"));
+            e = cudaMemcpy(host.data(), d, 5 * m * sizeof(double), cudaMemcpyDeviceToHost);
+            if (e != cudaSuccess) return fail(PACH_ERR_CUDA, cuda_msg(e, "parameter map copy"));
+            for (int i = 0; i < 5; ++i)
+                if (dst[i]) std::memcpy(dst[i] + c, host.data() + (size_t)i * m, m * sizeof(double));
+        }
         return PACH_OK;
     }, fail);
 }

@@ -402,9 +402,9 @@ constexpr int kMapBlocks = 2;
 cudaError_t launch_map_params(const double *etc, int n, int T, double fs, double scale, int decay_depth,
                               double clarity_s, double *t_x, double *edt, double *clarity, double *definition,
                               double *sum, cudaStream_t s);
-// dst = src x f, or x rows[i / per_row] when rows is not null, for n doubles (trace.cu)
-cudaError_t launch_scale(double *dst, const double *src, size_t n, double f, const double *rows, size_t per_row,
-                         cudaStream_t s);
+// dst = src x f, or x rows[(first + i) / per_row] when rows is not null, for n doubles (trace.cu)
+cudaError_t launch_scale(double *dst, const double *src, size_t n, double f, const double *rows, size_t first,
+                         size_t per_row, cudaStream_t s);
 constexpr int kFuseMaxTris = 64;
 // k_bounce: walk and shade in one kernel, rays staying in registers over up to kMaxBounces interactions; planes:
 // every room has its planes.  Used for fused scenes without mapping receivers.

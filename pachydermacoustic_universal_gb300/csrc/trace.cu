@@ -1258,10 +1258,10 @@ __global__ void k_prop_sample(DevRun r, long long p0, int n, float *dirs, float 
 // Histogram scaling on the way to the host: HBM-bound, n x 16 bytes (the 20 M doubles of the arena's
 // histograms in 0.06 ms; the host loop it replaces took 20 ms on one core).
 __global__ void __launch_bounds__(256) k_scale(double *dst, const double *src, size_t n, double f, const double *rows,
-                                               size_t per_row) {
+                                               size_t first, size_t per_row) {
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
-        dst[i] = src[i] * (rows ? __ldg(rows + i / per_row) : f);
+        dst[i] = src[i] * (rows ? __ldg(rows + (first + i) / per_row) : f);
 }
 
 }  // namespace
@@ -1354,11 +1354,11 @@ cudaError_t wave_kernel_occupancy(int variant, int threads, int smem_shade, int 
                  : cudaOccupancyMaxActiveBlocksPerMultiprocessor(bpsm_shade, k_shade<false>, threads, smem_shade);
 }
 
-cudaError_t launch_scale(double *dst, const double *src, size_t n, double f, const double *rows, size_t per_row,
-                         cudaStream_t s) {
+cudaError_t launch_scale(double *dst, const double *src, size_t n, double f, const double *rows, size_t first,
+                         size_t per_row, cudaStream_t s) {
     if (n == 0) return cudaSuccess;
     const int blocks = (int)std::min<size_t>((n + 255) / 256, 8192);
-    k_scale<<<blocks, 256, 0, s>>>(dst, src, n, f, rows, per_row);
+    k_scale<<<blocks, 256, 0, s>>>(dst, src, n, f, rows, first, per_row);
     return cudaGetLastError();
 }
 

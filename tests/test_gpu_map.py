@@ -304,6 +304,41 @@ def test_directional_map_matches_oracle():
     assert (g["dir_pos"] >= 0).all() and (g["dir_neg"] <= 0).all()
 
 
+def test_scaled_downloads_keep_a_bounded_buffer():
+    """A scaled download leaves at most 64 MB on the device with the run, whatever the arrays' size (here 147 MB), and
+    its pieces meet: scaled arrays equal the raw ones times the run's factor, one product each, to the last element.
+    A batch's factors go by receiver across the pieces."""
+    torch = pytest.importorskip("torch")
+    w = rooms.shoebox_c1()
+    w.cutoff_s = 0.4
+    org = rooms.audience_plane((1.0, 1.0), (9.0, 7.0), 1.2, 0.25)
+    m = tracer.MapReceivers(org[:766], 0.25, 1000.0, directional=True)
+    ds = tracer.DeviceScene(w.scene)
+    run = tracer.Run(ds, w.sources, w.receivers, tracer.make_params(
+        rays=40, cutoff_length_m=w.cutoff_length_m, hist_cotime_ms=400.0, seed=3, map_receivers=m))
+    run.wait()
+    raw = run.map_histograms()
+    before = torch.cuda.mem_get_info(0)[0]
+    got = run.map_histograms(scaled=True)
+    assert before - torch.cuda.mem_get_info(0)[0] <= 66 << 20
+    assert got["dir_pos"].nbytes > 140 << 20 and raw["dir_pos"].any()
+    for k, f in (("energy", 1 / 40), ("pressure", np.sqrt(1 / 40)), ("dir_pos", 1 / 40), ("dir_neg", 1 / 40)):
+        assert np.array_equal(got[k], raw[k] * f), k
+    run.close()
+    ws = [rooms.proposal_room_c4(30 + i) for i in range(2)]
+    n = [30, 50]
+    p = tracer._batch_params(ws, n, 3)
+    p.hist_cotime_ms = 300_000.0  # 3 receivers x 3 x 8 x 300000 bins
+    b = tracer.BatchRun([tracer.DeviceScene(x.scene) for x in ws], ws, n, p)
+    b.wait()
+    raw, got = b.histograms(), b.histograms(scaled=True)
+    assert got["dir_pos"].nbytes > 2 * (64 << 20)
+    f = np.repeat([len(x.sources) / c for x, c in zip(ws, n)], b.room_receivers)
+    for k in ("energy", "dir_pos", "dir_neg", "analysis"):
+        assert np.array_equal(got[k], raw[k] * f.reshape((-1,) + (1,) * (raw[k].ndim - 1))), k
+    b.close()
+
+
 @pytest.mark.parametrize("walk", [0, 1])
 @pytest.mark.parametrize("layout", ["one", "row", "lattice"])
 @pytest.mark.parametrize("rays", [1, 33, 300])
