@@ -116,9 +116,11 @@ typedef struct {
     int32_t blocks_per_sm;         /* resident blocks per SM to launch; 0 = occupancy maximum */
     int32_t wave_kilo_items;       /* octave rays per wave, in units of 1024; 0 = default (8192; 4096
                                       in each of the loops a run is shared out to) */
-    int32_t ring_log2;             /* ring queue capacity 2^ring_log2 octave rays; 0 = default (2^22..2^28 by
-                                      the run's primaries, 2048 rays each; runs of more than 256
-                                      primaries: three rings of a quarter, at least 2^22 each) */
+    int32_t ring_log2;             /* ring queue capacity 2^ring_log2 octave rays of 64 bytes; 0 = default: 2^22..2^28
+                                      by the run's primaries, 2048 rays each, and at least 2^24 for batches and
+                                      scenes of up to 64 triangles; runs of more than 256 primaries have three
+                                      rings of a quarter of that, at least 2^22 each (batches 2^23).  When this
+                                      memory cannot be had, one ring, at last of 2^22..2^28 by the primaries alone */
     int32_t kernel_timing;         /* 1: CUDA events around every kernel (per-kernel times in pach_stats) */
     int32_t ray_sort;              /* 1: order each wave by (direction octant, origin cell) before tracing;
                                       0 = default (off: measured +6 % walk rate in the 20k-triangle

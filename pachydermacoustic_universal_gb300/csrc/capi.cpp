@@ -19,6 +19,7 @@
 #include <vector>
 
 #include "engine.h"
+#include "ring_plan.h"
 
 using namespace pach;
 
@@ -687,13 +688,8 @@ void run_worker_body(pach_run *run) {
         const bool by_planes = bounce && *std::min_element(planes.begin(), planes.end()) > 0;
         if (bounce) TRY(bounce_occupancy(threads, receiver_smem_bytes(R), &bps_sh, by_planes));
 
-        // ring and wave sizing
-        // default ring: room for the run's rays at up to 2048 live octave rays per primary, 2^22..2^28
-        // (17 GB); default wave 8M rays -- measured against 2M: +7 % on a 20k-triangle hall and a
-        // 500k-triangle arena, +19 % on a 12-triangle shoebox (fewer, fuller iterations)
-        // a batch's pilots run several rooms at a time, and rays of small scenes leave several children a wave
-        int ring_default = n_rooms > 1 || bounce ? kRingMin : 22;
-        while (ring_default < 28 && (1ull << ring_default) < (unsigned long long)rprim_total(run) * 2048ull) ++ring_default;
+        // ring and wave sizing (ring_plans); default wave 8M rays -- measured against 2M: +7 % on a 20k-triangle hall
+        // and a 500k-triangle arena, +19 % on a 12-triangle shoebox (fewer, fuller iterations)
         const bool sorting = run->p.ray_sort > 0;
         const bool timing = run->p.kernel_timing != 0;
         const bool conv_mode = run->conv_mode >= 0;
@@ -707,39 +703,43 @@ void run_worker_body(pach_run *run) {
         // one, 9.2 with two; 300: 13.6, 9.7, with three 9.3).  Runs that the caller shapes (ring, feed, sorted
         // waves, kernel times) and convergence runs, whose revolutions are smaller, keep one.
         const long long N = rprim[n_rooms] - rprim[0];
-        P = timing || conv_mode || sorting || run->p.ring_log2 > 0 || run->p.feed_batch > 0 || N <= kPilotPrimaries ? 1 : kPipes;
-        const int ring_log2 = run->p.ring_log2 > 0 ? std::min(32, std::max(16, run->p.ring_log2)) : ring_default;
-        // A loop's ring is a quarter of the whole one, but no less than what keeps its waves full (a batch's pilots run
-        // several rooms at a time: 8 rooms of 500 primaries 258 ms with 2^22 rays, 248 with 2^23, 257 with 2^24).
-        const int pipe_log2 = std::max(n_rooms > 1 ? 23 : 22, ring_log2 - 2);
-        if (bound * 4 > (1ull << pipe_log2)) P = 1;
-        unsigned long long ring_cap = 1ull << (P > 1 ? pipe_log2 : ring_log2);
-        const unsigned long long max_wave =
-            run->p.wave_kilo_items > 0 ? 1024ull * run->p.wave_kilo_items : (1ull << (P > 1 ? 22 : 23));
+        const bool shared = !(timing || conv_mode || sorting || run->p.ring_log2 > 0 || run->p.feed_batch > 0 || N <= kPilotPrimaries);
+        const std::vector<RingPlan> rings =
+            ring_plans(run->p.ring_log2, rprim_total(run), n_rooms, shared, n_rooms > 1 || bounce, bound);
+        if (rings.empty()) {
+            const int l = ring_plans(run->p.ring_log2, rprim_total(run), n_rooms, false, n_rooms > 1 || bounce, 0)[0].log2;
+            status = PACH_ERR_BOUNDS;
+            msg = "the ring queue (2^" + std::to_string(l) + " rays) cannot hold the phase-A output of one "
+                  "primary (" + std::to_string(bound) + " rays); raise ring_log2 or set max_broadband_bounces";
+            final_state = PACH_RUN_FAILED;
+            break;
+        }
+        unsigned long long ring_cap = 0, max_wave = 0;
+        // the first of the rings from `from` on whose memory can be had
+        auto take_rings = [&](size_t from) -> cudaError_t {
+            cudaError_t x = cudaErrorMemoryAllocation;
+            for (size_t k = from; k < rings.size(); ++k) {
+                P = rings[k].loops;
+                ring_cap = 1ull << rings[k].log2;
+                max_wave = run->p.wave_kilo_items > 0 ? 1024ull * run->p.wave_kilo_items : (1ull << (P > 1 ? 22 : 23));
+                max_wave = std::min(max_wave, ring_cap);
+                if (!(x = run->qa.alloc(P * ring_cap * sizeof(ORayItem))) && !(x = run->qs0.alloc(P * max_wave * sizeof(int4))) &&
+                    !(sorting && (x = run->qs1.alloc(max_wave * sizeof(ORayItem)))))
+                    return cudaSuccess;
+                if (x != cudaErrorMemoryAllocation) return x;
+                cudaGetLastError();  // memory for the next may be there
+                for (DevMem *m : {&run->qa, &run->qs0, &run->qs1}) m->release();
+            }
+            return x;
+        };
+        TRY(take_rings(0));
+        if (e) break;
         // Half the blocks that fit for each trace kernel: the loops' kernels run side by side instead of one after the
         // other (three loops, all blocks / half: hall with the map 44.3 / 42.3 ms, 20k primaries 148.4 / 142.5).
         const int tr_blocks = dev_sms * (P > 1 ? (std::max(bps_tr, 1) + 1) / 2 : std::max(bps_tr, 1));
         const int sh_blocks = dev_sms * std::max(bps_sh, 1);
         const int map_blocks = dev_sms * kMapBlocks;
-        if (bound * 4 > ring_cap) {
-            status = PACH_ERR_BOUNDS;
-            msg = "the ring queue (2^" + std::to_string(ring_log2) + " rays) cannot hold the phase-A output of one "
-                  "primary (" + std::to_string(bound) + " rays); raise ring_log2 or set max_broadband_bounces";
-            final_state = PACH_RUN_FAILED;
-            break;
-        }
-        if (P > 1 && (run->qa.alloc(P * ring_cap * sizeof(ORayItem)) || run->qs0.alloc(P * std::min(max_wave, ring_cap) * sizeof(int4)))) {
-            cudaGetLastError();  // memory for one ring may be left
-            run->qs0.release();
-            P = 1;
-            ring_cap = 1ull << ring_log2;
-        }
-        if (P == 1) {
-            TRY(run->qa.alloc(ring_cap * sizeof(ORayItem)));
-            TRY(run->qs0.alloc(std::min(max_wave, ring_cap) * sizeof(int4)));
-        }
         if (sorting) {
-            TRY(run->qs1.alloc(std::min(max_wave, ring_cap) * sizeof(ORayItem)));
             TRY(run->sortbins.alloc(2 * kSortBins * sizeof(unsigned)));
             TRY(cudaMemsetAsync(run->sortbins.p, 0, run->sortbins.bytes, stream));
         }
@@ -828,7 +828,7 @@ void run_worker_body(pach_run *run) {
         r.max_bounces = bounce ? kMaxBounces : 1;
         r.full_wave = kFullFactor * (unsigned long long)sh_blocks * threads;
         r.feed_bound = bound;
-        const long long fb_default = std::max<long long>(4096, (long long)(std::min(max_wave, ring_cap) / 32));
+        const long long fb_default = std::max<long long>(4096, (long long)(max_wave / 32));
         r.feed_batch = run->p.feed_batch > 0 ? run->p.feed_batch : fb_default;
         const int bb_threads = 128;
         const int bb_blocks = (int)std::max<long long>(1, std::min<long long>((r.feed_batch + bb_threads - 1) / bb_threads,
@@ -948,7 +948,7 @@ void run_worker_body(pach_run *run) {
                 q.r.ring = run->qa.as<ORayItem>() + k * ring_cap;
                 q.r.ring_cap = ring_cap;
                 q.r.ctl = reinterpret_cast<WaveCtl *>(run->qctl.as<char>() + k * kCtlStride);
-                q.r.max_wave = std::min(max_wave, ring_cap);
+                q.r.max_wave = max_wave;
                 q.r.hits = run->qs0.as<int4>() + k * q.r.max_wave;
                 q.r.low_water = std::min(ring_cap / 4, 2 * q.r.max_wave);
                 if (n > 1) {
@@ -1113,10 +1113,7 @@ void run_worker_body(pach_run *run) {
                                   &run->mP, &run->mDp, &run->mDn})
                     if (m->p) TRY(cudaMemsetAsync(m->p, 0, m->bytes, stream));
                 if (e) break;
-                P = 1;
-                ring_cap = 1ull << ring_log2;
-                TRY(run->qa.alloc(ring_cap * sizeof(ORayItem)));
-                TRY(run->qs0.alloc(std::min(max_wave, ring_cap) * sizeof(int4)));
+                TRY(take_rings(1));  // the plans after the first are one loop's
                 if (e) break;
                 run->segments = run->end_traces = 0;
                 std::memset(h_ctl, 0, kMaxPipes * sizeof(WaveCtl));

@@ -210,8 +210,7 @@ constexpr int kSmemReceivers = 256;
 inline int receiver_smem_bytes(int R) { return 20 * (R > 0 && R <= kSmemReceivers ? R : 1); }
 
 constexpr long long kPilotPrimaries = 256;
-constexpr int kPipes = 3;            // device loops that a run is shared out to
-constexpr int kMaxPipes = 4;
+constexpr int kMaxPipes = 4;         // kPipes at most
 
 // Mapping receivers on the device (PachMapReceiver).  The grid is the reference's: cells of
 // BoxDims / ceil(BoxDims / (4, 4, 2.5 increments)) over the spheres' bounding box; cell c lists
@@ -414,10 +413,6 @@ constexpr int kFuseMaxTris = 64;
 constexpr int kMaxBounces = 32;
 constexpr int kSmallBounces = 8;
 constexpr unsigned long long kFullFactor = 4;
-// Default ring of such runs and of batches that keep one device loop, at least (log2): 1 GB.  2^22 leaves a
-// 1003-primary shoebox room for one or two interactions a wave (96 waves, 12.9 ms; 30 waves, 9.6 ms with 2^24; three
-// loops of a third of the primaries and 2^22 rays each take 8.7 ms).
-constexpr int kRingMin = 24;
 cudaError_t launch_bounce(const DevRun &r, int blocks, int threads, cudaStream_t s, bool planes);
 cudaError_t bounce_occupancy(int threads, int smem, int *blocks_per_sm, bool planes);
 inline bool fused_walk(int traversal, int ntri) { return traversal == 3 || (traversal == 0 && ntri <= kFuseMaxTris); }
