@@ -541,8 +541,6 @@ void run_worker_body(pach_run *run) {
         TRY(run->hAn.alloc(std::max<size_t>(nD, 1) * 8));
         TRY(run->cnt.alloc(sizeof(DevCounters)));
         TRY(run->qctl.alloc(kMaxPipes * kCtlStride));
-        for (DevMem *m : {&run->hE, &run->hP, &run->hDp, &run->hDn, &run->hAn, &run->cnt, &run->qctl})
-            TRY(cudaMemsetAsync(m->p, 0, m->bytes, stream));
         if (e) break;
 
         // scene: the first room's own device arrays, or the concatenation of every room's
@@ -646,7 +644,6 @@ void run_worker_body(pach_run *run) {
         if (run->p.capture) {
             const size_t per = run->p.capture == 2 ? (size_t)(rprim_total(run)) : (size_t)kDirBins;
             TRY(run->dcap.alloc((size_t)std::max(R, 1) * kCaptureWindows * per * sizeof(float)));
-            TRY(cudaMemset(run->dcap.p, 0, run->dcap.bytes));
         }
 
         const bool map = run->has_map;
@@ -663,13 +660,9 @@ void run_worker_body(pach_run *run) {
             const size_t nm = (size_t)g.M * kBands * g.T;
             TRY(run->mE.alloc(nm * sizeof(double)));
             TRY(run->mP.alloc(nm * sizeof(double)));
-            TRY(cudaMemsetAsync(run->mE.p, 0, run->mE.bytes, stream));
-            TRY(cudaMemsetAsync(run->mP.p, 0, run->mP.bytes, stream));
             if (g.directional) {
                 TRY(run->mDp.alloc(3 * nm * sizeof(double)));
                 TRY(run->mDn.alloc(3 * nm * sizeof(double)));
-                TRY(cudaMemsetAsync(run->mDp.p, 0, run->mDp.bytes, stream));
-                TRY(cudaMemsetAsync(run->mDn.p, 0, run->mDn.bytes, stream));
             }
         }
 
@@ -734,15 +727,17 @@ void run_worker_body(pach_run *run) {
         };
         TRY(take_rings(0));
         if (e) break;
-        // Half the blocks that fit for each trace kernel: the loops' kernels run side by side instead of one after the
-        // other (three loops, all blocks / half: hall with the map 44.3 / 42.3 ms, 20k primaries 148.4 / 142.5).
-        const int tr_blocks = dev_sms * (P > 1 ? (std::max(bps_tr, 1) + 1) / 2 : std::max(bps_tr, 1));
+        int tr_blocks = 0, bb_blocks = 0;  // make_pipes
         const int sh_blocks = dev_sms * std::max(bps_sh, 1);
         const int map_blocks = dev_sms * kMapBlocks;
-        if (sorting) {
-            TRY(run->sortbins.alloc(2 * kSortBins * sizeof(unsigned)));
-            TRY(cudaMemsetAsync(run->sortbins.p, 0, run->sortbins.bytes, stream));
-        }
+        if (sorting) TRY(run->sortbins.alloc(2 * kSortBins * sizeof(unsigned)));
+        // what a run adds to or schedules by, before every attempt at it
+        auto zero_results = [&] {
+            for (DevMem *m : {&run->hE, &run->hP, &run->hDp, &run->hDn, &run->hAn, &run->cnt, &run->qctl, &run->dcap, &run->mE,
+                              &run->mP, &run->mDp, &run->mDn, &run->sortbins})
+                if (m->p) TRY(cudaMemsetAsync(m->p, 0, m->bytes, stream));
+            std::memset(h_ctl, 0, kMaxPipes * sizeof(WaveCtl));
+        };
         const int sort_blocks = dev_sms * 4;
         if (!timing) {
             TRY(cudaHostAlloc(&h_mirror, kMaxPipes * sizeof(HostMirror), cudaHostAllocMapped));
@@ -828,12 +823,7 @@ void run_worker_body(pach_run *run) {
         r.max_bounces = bounce ? kMaxBounces : 1;
         r.full_wave = kFullFactor * (unsigned long long)sh_blocks * threads;
         r.feed_bound = bound;
-        const long long fb_default = std::max<long long>(4096, (long long)(max_wave / 32));
-        r.feed_batch = run->p.feed_batch > 0 ? run->p.feed_batch : fb_default;
         const int bb_threads = 128;
-        const int bb_blocks = (int)std::max<long long>(1, std::min<long long>((r.feed_batch + bb_threads - 1) / bb_threads,
-                                                                              (long long)dev_sms * 8));
-        std::memset(h_ctl, 0, kMaxPipes * sizeof(WaveCtl));
         double t_trace = 0, t_shade = 0, t_bb = 0, t_sort = 0;
         long long launches = 0;
         bool cancelled = false;
@@ -916,6 +906,12 @@ void run_worker_body(pach_run *run) {
         auto make_pipes = [&]() -> cudaError_t {
             cudaError_t x;
             const int n = n_rooms;
+            // Half the blocks that fit for each trace kernel: the loops' kernels run side by side instead of one after
+            // the other (three loops, all blocks / half: hall with the map 44.3 / 42.3 ms, 20k primaries 148.4 / 142.5).
+            tr_blocks = dev_sms * (P > 1 ? (std::max(bps_tr, 1) + 1) / 2 : std::max(bps_tr, 1));
+            r.feed_batch = run->p.feed_batch > 0 ? run->p.feed_batch : std::max<long long>(4096, (long long)(max_wave / 32));
+            bb_blocks = (int)std::max<long long>(1, std::min<long long>((r.feed_batch + bb_threads - 1) / bb_threads,
+                                                                        (long long)dev_sms * 8));
             if (n > 1) {  // each pipe's feed order (DevRun::sched_off, sched_prim), then its live counts and peaks
                 const size_t each = 5 * (size_t)n + 1;
                 std::vector<long long> sched(each * P, 0);
@@ -966,7 +962,6 @@ void run_worker_body(pach_run *run) {
             }
             return cudaSuccess;
         };
-        TRY(make_pipes());
         double dev_ms_total = 0;
         long long done_before = 0;  // primaries of the ranges already run (progress offset)
         // Runs the device loop over primaries [p0, p1): the graph launch (progress and cancellation through
@@ -988,6 +983,7 @@ void run_worker_body(pach_run *run) {
                 if (n_rooms > 1) {  // positions of the pipe's own feed order
                     a = b = p0;
                     for (const RoomSpec &rm : run->rooms) b += share(rm.rays, k + 1, P) - share(rm.rays, k, P);
+                    if (P == 1) b = std::min(b, p1);
                 }
                 c.next_prim = a;
                 c.prim_end = b;
@@ -1023,8 +1019,8 @@ void run_worker_body(pach_run *run) {
                         ended = std::max(ended, (unsigned long long)h_mirror[k].end_traces);
                         run->segments = std::max<long long>(run->segments, (long long)h_mirror[k].segments);
                     }
-                    run->rays_done = done_before + fed;
-                    run->end_traces = (long long)ended;
+                    run->rays_done = std::max<long long>(run->rays_done, done_before + fed);
+                    run->end_traces = std::max<long long>(run->end_traces, (long long)ended);
                     if (q == cudaSuccess) break;
                     if (q != cudaErrorNotReady) { where = "graph run"; return q; }
                     const auto now = std::chrono::steady_clock::now();
@@ -1103,24 +1099,13 @@ void run_worker_body(pach_run *run) {
             return cudaSuccess;
         };
 #undef RTRY
-        if (!conv_mode) {
-            if ((e = run_range(rprim[0], rprim[0] + N)) != cudaSuccess || status) break;
-            bool full = false;
-            for (int k = 0; k < P; ++k) full = full || h_ctl[k].overflow;
-            if (full && P > 1 && !cancelled) {
-                // a pipe's ring was too small: once more from nothing, as one loop in the ring that one loop gets
-                for (DevMem *m : {&run->hE, &run->hP, &run->hDp, &run->hDn, &run->hAn, &run->cnt, &run->qctl, &run->dcap, &run->mE,
-                                  &run->mP, &run->mDp, &run->mDn})
-                    if (m->p) TRY(cudaMemsetAsync(m->p, 0, m->bytes, stream));
-                if (e) break;
-                TRY(take_rings(1));  // the plans after the first are one loop's
-                if (e) break;
-                run->segments = run->end_traces = 0;
-                std::memset(h_ctl, 0, kMaxPipes * sizeof(WaveCtl));
-                TRY(make_pipes());
-                if ((e = run_range(rprim[0], rprim[0] + N)) != cudaSuccess || status) break;
+        auto full = [&] { return std::any_of(h_ctl, h_ctl + P, [](const WaveCtl &c) { return c.overflow != 0; }); };
+        // Traces the first `todo` primaries of the feed order, or revolutions until the checks agree.
+        auto attempt = [&](long long todo) {
+            if (!conv_mode) {
+                e = run_range(rprim[0], rprim[0] + todo);
+                return;
             }
-        } else {
             // Convergence mode (TaskAll:300-330): revolutions of conv_period primaries until every check
             // agrees.  Chunks of revolutions run as one device loop that also records each revolution's
             // contribution to the two check receivers; the host replays the checks revolution by
@@ -1143,7 +1128,7 @@ void run_worker_body(pach_run *run) {
                 TRY(cudaMemsetAsync(run->conv.p, 0, (size_t)K * 2 * kConvKinds * T * sizeof(double), stream));
                 if (e) break;
                 done_before = done;
-                if ((e = run_range(rprim[0] + done, rprim[0] + done + K * period)) != cudaSuccess || status) break;
+                if ((e = run_range(rprim[0] + done, rprim[0] + done + K * period)) != cudaSuccess || status || full()) break;
                 TRY(cudaMemcpy(capbuf.data(), run->conv.p, (size_t)K * 2 * kConvKinds * T * sizeof(double),
                                cudaMemcpyDeviceToHost));
                 int stop = -1;
@@ -1167,7 +1152,8 @@ void run_worker_body(pach_run *run) {
                     for (int i = 0; i < 6; ++i)
                         TRY(cudaMemcpyAsync(live[i]->p, run->bak[i].p, live[i]->bytes, cudaMemcpyDeviceToDevice, stream));
                     if (e) break;
-                    if ((e = run_range(rprim[0] + done, rprim[0] + done + (stop + 1) * period)) != cudaSuccess || status)
+                    if ((e = run_range(rprim[0] + done, rprim[0] + done + (stop + 1) * period)) != cudaSuccess || status ||
+                        full())
                         break;
                 }
                 done += (stop >= 0 ? stop + 1 : K) * period;
@@ -1175,11 +1161,38 @@ void run_worker_body(pach_run *run) {
                 converged = stop >= 0;
                 chunk = std::min(chunk * 2, kConvChunk);
             }
-            if (e || status) break;
+            if (e || status || full()) return;
             run->rooms[0].rays = done;
             run->conv_revs = revs;
             run->conv_converged = converged;
             if (run->cancel) cancelled = true;
+        };
+        const std::vector<ConvCheck> checks = run->conv_checks;
+        zero_results();
+        if (e) break;
+        TRY(make_pipes());
+        attempt(N);
+        if (e || status) break;
+        const bool aborted = std::any_of(h_ctl, h_ctl + P, [](const WaveCtl &c) { return c.gave_up == 2; });
+        if (full() && !aborted) {
+            // The feed's forecast was wrong, or a share of the ring too small for its loop: once more from nothing, as
+            // one loop that feeds each room's pilot alone and plans with its whole peak, one interaction a wave.  A
+            // cancelled run traces the primaries that it had fed.
+            long long todo = N;
+            if (cancelled && !conv_mode) {
+                todo = 0;
+                for (int k = 0; k < P; ++k) todo += h_ctl[k].next_prim - pipes[k].p0;
+            }
+            r.careful = 1;
+            r.max_bounces = 1;
+            run->conv_checks = checks;
+            done_before = 0;
+            if (P > 1) TRY(take_rings(1));  // the plans after the first are one loop's
+            zero_results();
+            if (e) break;
+            TRY(make_pipes());
+            attempt(todo);
+            if (e || status) break;
         }
         const float dev_ms = (float)dev_ms_total;
         TRY(cudaMemcpy(h_cnt, run->cnt.p, sizeof(DevCounters), cudaMemcpyDeviceToHost));
@@ -1239,14 +1252,14 @@ void run_worker_body(pach_run *run) {
         run->rays_done = (long long)h_cnt->primaries;
         run->segments = s.segments;
         run->end_traces = s.end_traces;
-        if (all.overflow) {
-            status = PACH_ERR_BOUNDS;
-            msg = "ring queue full: raise ring_log2";
-            final_state = PACH_RUN_FAILED;
-        } else if (all.gave_up == 2) {
+        if (all.gave_up == 2) {
             status = PACH_ERR_CANCELLED;
             msg = "run cancelled; the loop stopped before every fed primary finished";
             final_state = PACH_RUN_CANCELLED;
+        } else if (all.overflow) {
+            status = PACH_ERR_BOUNDS;
+            msg = "ring queue full: raise ring_log2";
+            final_state = PACH_RUN_FAILED;
         } else if (all.gave_up) {
             status = PACH_ERR_GAVE_UP;
             msg = "wavefront loop stopped without finishing (iteration cap or no progress)";

@@ -291,6 +291,7 @@ struct DevRun {
                                    // pass loads normal and material directly, one dependent load fewer
     unsigned long long max_wave;   // items per wave at most
     int max_bounces;               // interactions per wave item at most (1: one; more: k_bounce)
+    int careful;                   // 1: every pilot alone and to its last ray (a run whose ring was full once)
     unsigned long long full_wave;  // items that fill the machine (smaller waves: at most kSmallBounces)
     long long feed_batch;          // primaries per phase-A launch at most
     unsigned long long feed_bound; // ring slots one primary can fill in phase A

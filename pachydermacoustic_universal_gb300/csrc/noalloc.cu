@@ -156,11 +156,6 @@ extern "C" pach_status pach_trace_run_noalloc(const pach_scene *scene, const pac
 
         // The scratch keeps the previous call's contents: clear the schedule and counters, and the
         // caller's histograms, which accumulate.
-        WaveCtl h_ctl;
-        std::memset(&h_ctl, 0, sizeof(h_ctl));
-        h_ctl.next_prim = p.ray_begin;
-        h_ctl.prim_end = p.ray_begin + p.ray_count;
-        h_ctl.prim_first = p.ray_begin;
         if (n_receivers > 0) NA_TRY(cudaMemcpyAsync(base + kOffRec, rec, n_receivers * sizeof(float4), cudaMemcpyHostToDevice, stream));
         NA_TRY(cudaMemcpyAsync(base + kOffSrc, src, n_sources * sizeof(float4), cudaMemcpyHostToDevice, stream));
         NA_TRY(cudaMemcpyAsync(base + kOffE0, e0, n_sources * kBands * sizeof(float), cudaMemcpyHostToDevice, stream));
@@ -187,13 +182,6 @@ extern "C" pach_status pach_trace_run_noalloc(const pach_scene *scene, const pac
         room.n_planes = scene_planes(scene);
         room.max_broad = (int)std::fmin((double)max_broad, (double)(1u << 30));
         NA_TRY(cudaMemcpyAsync(base + kOffRoom, &room, sizeof(room), cudaMemcpyHostToDevice, stream));
-        NA_TRY(cudaMemcpyAsync(base + kOffCtl, &h_ctl, sizeof(WaveCtl), cudaMemcpyHostToDevice, stream));
-        NA_TRY(cudaMemsetAsync(base + kOffCnt, 0, sizeof(DevCounters), stream));
-        NA_TRY(cudaMemsetAsync(d_energy, 0, nE * sizeof(double), stream));
-        NA_TRY(cudaMemsetAsync(d_pressure, 0, nE * sizeof(double), stream));
-        NA_TRY(cudaMemsetAsync(d_dir_pos, 0, nD * sizeof(double), stream));
-        NA_TRY(cudaMemsetAsync(d_dir_neg, 0, nD * sizeof(double), stream));
-        NA_TRY(cudaMemsetAsync(d_analysis, 0, nD * sizeof(double), stream));
 
         DevRun r{};
         r.S = *scene_dev(scene);
@@ -235,30 +223,48 @@ extern "C" pach_status pach_trace_run_noalloc(const pach_scene *scene, const pac
         const int tr_blocks = sms * (bps_tr > 0 ? bps_tr : 1), sh_blocks = sms * (bps_sh > 0 ? bps_sh : 1);
         r.full_wave = kFullFactor * (unsigned long long)sh_blocks * 256;
         long long launches = 0;
-        // Every iteration of the loop either traces a wave or feeds primaries, so the schedule moves on
-        // each time; if it stops moving for kNaStall synchronisations in a row (kNaStall x 32
-        // iterations) the call gives up instead of waiting on a loop that no longer progresses.
-        unsigned long long seen_waves = 0;
-        long long seen_prim = -1;
-        int stalls = 0;
+        // Once more from nothing when the split children of several interactions a wave have filled the ring: one
+        // interaction a wave holds the fewest.
+        WaveCtl h_ctl;
         for (;;) {
-            for (int k = 0; k < 32; ++k) {
-                NA_TRY(launch_feed(r, stream));
-                NA_TRY(launch_broadband(r, sms * 2, 128, stream, false, hs.ntri <= kFuseMaxTris));
-                if (!fused) NA_TRY(launch_trace(r, variant, tr_blocks, 256, stream));
-                NA_TRY(fused ? launch_bounce(r, sh_blocks, 256, stream, by_planes) : launch_shade(r, sh_blocks, 256, stream));
-                launches += fused ? 3 : 4;
+            std::memset(&h_ctl, 0, sizeof(h_ctl));
+            h_ctl.next_prim = p.ray_begin;
+            h_ctl.prim_end = p.ray_begin + p.ray_count;
+            h_ctl.prim_first = p.ray_begin;
+            NA_TRY(cudaMemcpyAsync(base + kOffCtl, &h_ctl, sizeof(WaveCtl), cudaMemcpyHostToDevice, stream));
+            NA_TRY(cudaMemsetAsync(base + kOffCnt, 0, sizeof(DevCounters), stream));
+            NA_TRY(cudaMemsetAsync(d_energy, 0, nE * sizeof(double), stream));
+            NA_TRY(cudaMemsetAsync(d_pressure, 0, nE * sizeof(double), stream));
+            NA_TRY(cudaMemsetAsync(d_dir_pos, 0, nD * sizeof(double), stream));
+            NA_TRY(cudaMemsetAsync(d_dir_neg, 0, nD * sizeof(double), stream));
+            NA_TRY(cudaMemsetAsync(d_analysis, 0, nD * sizeof(double), stream));
+            // Every iteration of the loop either traces a wave or feeds primaries, so the schedule moves on
+            // each time; if it stops moving for kNaStall synchronisations in a row (kNaStall x 32
+            // iterations) the call gives up instead of waiting on a loop that no longer progresses.
+            unsigned long long seen_waves = 0;
+            long long seen_prim = -1;
+            int stalls = 0;
+            for (;;) {
+                for (int k = 0; k < 32; ++k) {
+                    NA_TRY(launch_feed(r, stream));
+                    NA_TRY(launch_broadband(r, sms * 2, 128, stream, false, hs.ntri <= kFuseMaxTris));
+                    if (!fused) NA_TRY(launch_trace(r, variant, tr_blocks, 256, stream));
+                    NA_TRY(fused ? launch_bounce(r, sh_blocks, 256, stream, by_planes) : launch_shade(r, sh_blocks, 256, stream));
+                    launches += fused ? 3 : 4;
+                }
+                NA_TRY(cudaMemcpyAsync(&h_ctl, base + kOffCtl, sizeof(WaveCtl), cudaMemcpyDeviceToHost, stream));
+                NA_TRY(cudaStreamSynchronize(stream));
+                if (h_ctl.done) break;
+                if (h_ctl.waves == seen_waves && h_ctl.next_prim == seen_prim) {
+                    if (++stalls >= kNaStall) return na_fail(PACH_ERR_GAVE_UP, "wavefront loop stopped making progress");
+                } else {
+                    stalls = 0;
+                }
+                seen_waves = h_ctl.waves;
+                seen_prim = h_ctl.next_prim;
             }
-            NA_TRY(cudaMemcpyAsync(&h_ctl, base + kOffCtl, sizeof(WaveCtl), cudaMemcpyDeviceToHost, stream));
-            NA_TRY(cudaStreamSynchronize(stream));
-            if (h_ctl.done) break;
-            if (h_ctl.waves == seen_waves && h_ctl.next_prim == seen_prim) {
-                if (++stalls >= kNaStall) return na_fail(PACH_ERR_GAVE_UP, "wavefront loop stopped making progress");
-            } else {
-                stalls = 0;
-            }
-            seen_waves = h_ctl.waves;
-            seen_prim = h_ctl.next_prim;
+            if (!h_ctl.overflow || r.max_bounces == 1) break;
+            r.max_bounces = 1;
         }
         if (h_ctl.overflow)
             return na_fail(PACH_ERR_BOUNDS, "the split trees outgrew the no-alloc ring (65536 octave rays); "

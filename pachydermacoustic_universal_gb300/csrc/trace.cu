@@ -75,11 +75,16 @@ __device__ __forceinline__ unsigned long long warp_append(unsigned long long *ta
 // batch are counted separately (room_live), so after the first room's pilot the others run together, as
 // many as the plan lets into half the ring: 8 rooms x 500 primaries take 381 waves and 288 ms where one
 // pilot after another took about 1100 waves and 445 ms.
+//
+// Both are forecasts: a later room's trees may be many times the first room's, and a pilot may grow again.  A run
+// whose ring is full after all starts over in careful mode: each room's pilot alone in an empty ring and to its
+// last ray, one interaction a wave (run_worker_body).
 
 // Pilot footprint of the group in flight, or false while it may still grow.  All 32 lanes call.
 __device__ bool pilots_measured(const DevRun &r, WaveCtl *c, unsigned long long live, bool decaying,
                                 unsigned long long &pp) {
     const int lane = threadIdx.x & 31;
+    if (r.careful && live != 0) return false;
     if (r.n_rooms == 1) {
         if (live != 0 && !(decaying && live <= c->pilot_peak - c->pilot_peak / 8)) return false;
         pp = c->pilot_peak * 3 / (unsigned long long)c->pilot_count + 1;
@@ -154,7 +159,7 @@ __device__ void feed_step(const DevRun &r) {
         if (next >= first) {
             int k = c->pilot_room;
             unsigned long long n = 0;
-            if (r.n_rooms == 1 || c->per_prim == 0) {  // the first pilot runs alone
+            if (r.n_rooms == 1 || c->per_prim == 0 || r.careful) {  // the first pilot runs alone
                 if (live != 0) return;
                 n = r.n_rooms == 1 ? (unsigned long long)kPilotPrimaries
                                    : (unsigned long long)(__ldg(r.sched_off + k + 1) - next);

@@ -149,6 +149,38 @@ def test_batch_feed_order_traces_every_primary_once(rays, ring_log2, feed_batch)
         off += rays[i]
 
 
+@pytest.mark.parametrize("big,alpha,ring_log2,capture", [(4, 0.25, 20, 0), (4, 0.25, 19, 1), (2, 0.2, 20, 0), (40, 0.15, 0, 0)])
+def test_rooms_that_outgrow_the_first_are_traced_in_the_ring_they_fit(big, alpha, ring_log2, capture):
+    """A room of small trees first (alpha 0.6: 170 live rays a primary at most), then rooms of 9 to 30 times larger
+    ones: the plan from the first room lets the others' pilots in together, which fills the ring, given or (40
+    rooms) the three loops' own.  Each room alone fits, so the run starts over with the pilots one at a time and
+    every room equals its single run (FP64 sums in another order: 1e-9; FP32 capture sums 1e-4)."""
+    ws = [rooms.shoebox_c1() for _ in range(big + 1)]
+    for i, w in enumerate(ws):
+        w.scene.absorption = np.full_like(w.scene.absorption, alpha if i else 0.6)
+        w.cutoff_s = 1.0
+    ds = [tracer.DeviceScene(w.scene) for w in ws[:2]]
+    ds += [ds[1]] * (big - 1)
+    n = [256] * (big + 1)
+    p = tracer._batch_params(ws, n, 4, ring_log2=ring_log2, capture=capture)
+    run = tracer.BatchRun(ds, ws, n, p)
+    run.wait()
+    hb, sb = run.room_histograms(), run.stats()
+    assert sb["primaries"] == sum(n) and sb["queue_overflows"] == 0
+    cap = run.capture() if capture else None
+    run.close()
+    seg = det = 0
+    for i, w in enumerate(ws):
+        hs, ss = tracer.trace(w, dscene=ds[i], rays=256, seed=4, ray_begin=256 * i, capture=capture)
+        seg, det = seg + ss["segments"], det + ss["detections"]
+        for name in ("energy", "pressure", "dir_pos", "dir_neg", "analysis"):
+            np.testing.assert_allclose(hb[i][name], hs[name], rtol=1e-9, atol=1e-30, err_msg=f"{i} {name}")
+        if capture:
+            R = len(w.receivers)
+            np.testing.assert_allclose(cap[R * i:R * i + R].sum(axis=2), hs["capture"].sum(axis=2), rtol=1e-4)
+    assert sb["segments"] == seg and sb["detections"] == det
+
+
 def _l_room():
     """An L-shaped room (8 planes, not convex) of quads in two triangles."""
     x = [(0, 0), (8, 0), (8, 3), (4, 3), (4, 7), (0, 7)]
