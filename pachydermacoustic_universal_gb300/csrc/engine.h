@@ -60,13 +60,13 @@ pach_status guarded(F &&body, R &&report) noexcept {
 // Runs f(c0, c1) over [0, n) in chunks of `grain` elements on up to hardware_concurrency() threads;
 // inline when one chunk covers the range.  Chunk c is [c * grain, min(n, (c + 1) * grain)).
 template <class F>
-void parallel_chunks(size_t n, size_t grain, F &&f) {
+void parallel_chunks(size_t n, size_t grain, F &&f, size_t max_threads = SIZE_MAX) {
     const size_t nch = (n + grain - 1) / grain;
     if (nch <= 1) {
         if (n) f((size_t)0, n);
         return;
     }
-    const size_t nt = std::min(nch, (size_t)std::max(1u, std::thread::hardware_concurrency()));
+    const size_t nt = std::min({nch, max_threads, (size_t)std::max(1u, std::thread::hardware_concurrency())});
     auto run = [&](size_t t) {
         for (size_t c = t; c < nch; c += nt) f(c * grain, std::min(n, (c + 1) * grain));
     };
@@ -76,7 +76,7 @@ void parallel_chunks(size_t n, size_t grain, F &&f) {
     for (auto &p : parts) p.get();
 }
 
-// Gives every page of the given host ranges its memory, on several threads when there are many, and changes
+// Gives every page of the given host ranges its memory, on four threads when there are many, and changes
 // nothing in them: what is there stays when the copy then fails, when a range is an input of a copy still on its
 // way, and beside another thread's writes.  Memory that the caller has just allocated gets its pages here; left
 // to the copy they are faulted in by the GPU one after another, 55 us each (34 MB of fresh histogram arrays: 30 ms,
