@@ -294,6 +294,9 @@ typedef struct {
 pach_status pach_autotune(const pach_room_desc *rooms, int32_t n_rooms, const pach_trace_params *params,
                           int64_t sample_rays, const char *cache_path, int32_t force, pach_tune_result *out);
 pach_status pach_trace_poll(pach_run *run, pach_progress *progress);
+/* Stops feeding primaries; those already fed are finished, for at most two seconds.  A run of one room has then
+ * traced the primaries ray_begin .. ray_begin + rays_done - 1; a batch some primaries of every room (scaled
+ * histograms divide each room by its own). */
 pach_status pach_trace_cancel(pach_run *run);
 /* Blocks until the run stops or timeout_ms passes (timeout_ms < 0: no limit). */
 pach_status pach_trace_wait(pach_run *run, int64_t timeout_ms);

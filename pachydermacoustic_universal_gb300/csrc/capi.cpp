@@ -540,7 +540,7 @@ void run_worker_body(pach_run *run) {
         TRY(run->hDn.alloc(std::max<size_t>(nD, 1) * 8));
         TRY(run->hAn.alloc(std::max<size_t>(nD, 1) * 8));
         TRY(run->cnt.alloc(sizeof(DevCounters)));
-        TRY(run->qctl.alloc(kMaxPipes * kCtlStride));
+        TRY(run->qctl.alloc((kMaxPipes + 1) * kCtlStride));  // then the loops' common cursor
         if (e) break;
 
         // scene: the first room's own device arrays, or the concatenation of every room's
@@ -944,6 +944,8 @@ void run_worker_body(pach_run *run) {
                 q.r.ring = run->qa.as<ORayItem>() + k * ring_cap;
                 q.r.ring_cap = ring_cap;
                 q.r.ctl = reinterpret_cast<WaveCtl *>(run->qctl.as<char>() + k * kCtlStride);
+                q.r.cursor = P > 1 && n == 1 ? reinterpret_cast<unsigned long long *>(run->qctl.as<char>() + kMaxPipes * kCtlStride)
+                                             : nullptr;
                 q.r.max_wave = max_wave;
                 q.r.hits = run->qs0.as<int4>() + k * q.r.max_wave;
                 q.r.low_water = std::min(ring_cap / 4, 2 * q.r.max_wave);

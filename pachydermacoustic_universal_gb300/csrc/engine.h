@@ -259,6 +259,7 @@ struct DevRun {
     // sched_off[s + 1]) and starts at primary sched_prim[s]
     const long long *sched_off;   // [2 n_rooms + 1]
     const long long *sched_prim;  // [2 n_rooms]
+    unsigned long long *cursor;       // one room, several loops: primaries that the loops have fed together (else null)
     unsigned *room_live, *room_peak;  // [n_rooms] live rays of each room while pilots run, and their peaks
     // receivers of every room
     // each room's receivers ordered by the coordinate of their widest spread (measured 0.7-4.8 % faster

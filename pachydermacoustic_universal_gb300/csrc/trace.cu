@@ -110,6 +110,12 @@ __device__ bool pilots_measured(const DevRun &r, WaveCtl *c, unsigned long long 
     return true;
 }
 
+// First primary of the loop's next n.  Loops that share a room have shares of their own in number only: which
+// primaries they are goes by a common cursor, so that whatever a cancelled run has fed is the first of its primaries.
+__device__ __forceinline__ long long take_primaries(const DevRun &r, const WaveCtl *c, long long next, long long n) {
+    return r.cursor ? c->prim_first + (long long)atomicAdd(r.cursor, (unsigned long long)n) : next;
+}
+
 // Retires the last wave and decides what phase A gets next.  All 32 lanes call; lane 0 writes.
 __device__ void feed_step(const DevRun &r) {
     WaveCtl *c = r.ctl;
@@ -179,7 +185,7 @@ __device__ void feed_step(const DevRun &r) {
             if (n > (unsigned long long)kPilotPrimaries && r.n_rooms == 1) n = kPilotPrimaries;
             if (n > fit) n = fit;
             if (n < 1) n = 1;  // the ring holds the phase-A output of at least 4 primaries: checked at set-up
-            c->pa_begin = next;
+            c->pa_begin = take_primaries(r, c, next, (long long)n);
             c->pa_count = (long long)n;
             c->next_prim = next + (long long)n;
             c->pilot_count = (long long)n;
@@ -200,7 +206,7 @@ __device__ void feed_step(const DevRun &r) {
         if (soft < n) n = soft > 0 ? soft : (live == 0 ? 1 : 0);
         if (n > (unsigned long long)lim) n = (unsigned long long)lim;
         if (n > 0) {
-            c->pa_begin = next;
+            c->pa_begin = take_primaries(r, c, next, (long long)n);
             c->pa_count = (long long)n;
             c->next_prim = next + (long long)n;
             c->pressure = 0;

@@ -9,7 +9,7 @@ import pytest
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 sys.path.insert(0, ROOT)
 
-from pachydermacoustic_universal_gb300 import rooms, tracer  # noqa: E402
+from pachydermacoustic_universal_gb300 import _capi, rooms, tracer  # noqa: E402
 
 pytestmark = pytest.mark.gpu
 
@@ -179,6 +179,32 @@ def test_rooms_that_outgrow_the_first_are_traced_in_the_ring_they_fit(big, alpha
             R = len(w.receivers)
             np.testing.assert_allclose(cap[R * i:R * i + R].sum(axis=2), hs["capture"].sum(axis=2), rtol=1e-4)
     assert sb["segments"] == seg and sb["detections"] == det
+
+
+@pytest.mark.parametrize("kind", ["box", "hall"])
+def test_a_cancelled_run_has_traced_the_first_of_its_primaries(kind):
+    """However many loops shared them: what a cancelled run leaves equals a run of its first rays_done primaries, and
+    the run that goes on at ray_begin + rays_done adds the rest (FP64 sums in another order: 1e-9)."""
+    w = rooms.shoebox_c1() if kind == "box" else rooms.irregular_hall_c2(target_tris=2000)
+    w.cutoff_s = 0.4
+    ds = tracer.DeviceScene(w.scene)
+    p = dict(cutoff_length_m=w.cutoff_length_m, hist_cotime_ms=400.0, seed=6)
+    run = tracer.Run(ds, w.sources, w.receivers, tracer.make_params(rays=4_000_000, ray_begin=100, **p))
+    while run.poll()["rays_done"] < 3000:
+        pass
+    run.cancel()
+    with pytest.raises(_capi.PachError):
+        run.wait()
+    n = run.poll()["rays_done"]
+    h = run.histograms()
+    assert 3000 <= n < 4_000_000 and run.stats()["primaries"] == n
+    run.close()
+    first, _ = tracer.trace(w, dscene=ds, rays=n, seed=6, ray_begin=100)
+    for name in ("energy", "pressure", "dir_pos", "dir_neg", "analysis"):
+        np.testing.assert_allclose(h[name], first[name], rtol=1e-9, atol=1e-30, err_msg=name)
+    rest, _ = tracer.trace(w, dscene=ds, rays=500, seed=6, ray_begin=100 + n)
+    both, _ = tracer.trace(w, dscene=ds, rays=n + 500, seed=6, ray_begin=100)
+    np.testing.assert_allclose(h["energy"] + rest["energy"], both["energy"], rtol=1e-9, atol=1e-30)
 
 
 def _l_room():
