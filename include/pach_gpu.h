@@ -217,7 +217,7 @@ typedef struct {
     double sort_ms;
     int64_t waves;                 /* wavefront iterations that traced octave rays */
     int64_t kernel_launches;
-    int64_t peak_live_rays;        /* most octave rays held in the ring at once */
+    int64_t peak_live_rays;        /* most octave rays held in the ring (three loops: in their rings) at once */
     int64_t bvh_nodes_visited;     /* octave-ray traversal work: inner BVH nodes visited, and */
     int64_t tri_tests;             /* triangles tested (counted when kernel_timing = 1; else 0 on
                                       scenes walked by the speculative walk) */

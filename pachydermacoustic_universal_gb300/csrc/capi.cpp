@@ -944,6 +944,8 @@ void run_worker_body(pach_run *run) {
                 q.r.ring = run->qa.as<ORayItem>() + k * ring_cap;
                 q.r.ring_cap = ring_cap;
                 q.r.ctl = reinterpret_cast<WaveCtl *>(run->qctl.as<char>() + k * kCtlStride);
+                q.r.loops = run->qctl.as<WaveCtl>();
+                q.r.n_loops = P;
                 q.r.cursor = P > 1 && n == 1 ? reinterpret_cast<unsigned long long *>(run->qctl.as<char>() + kMaxPipes * kCtlStride)
                                              : nullptr;
                 q.r.max_wave = max_wave;
@@ -1206,7 +1208,6 @@ void run_worker_body(pach_run *run) {
             all.overflow += h_ctl[k].overflow;
             all.waves += h_ctl[k].waves;
             all.iters += h_ctl[k].iters;
-            all.peak_live += h_ctl[k].peak_live;
             all.gave_up = std::max(all.gave_up, h_ctl[k].gave_up);
             run->pipe_done[k] = h_ctl[k].next_prim - pipes[k].p0;
         }
@@ -1240,7 +1241,7 @@ void run_worker_body(pach_run *run) {
         s.sort_ms = t_sort;
         s.waves = (int64_t)all.waves;
         s.kernel_launches = timing ? launches : P + (long long)all.iters * ((sorting ? 7 : 4) - (fused ? 1 : 0) + (map ? 1 : 0));
-        s.peak_live_rays = (int64_t)all.peak_live;
+        s.peak_live_rays = (int64_t)(P > 1 ? h_cnt->peak_live : all.peak_live);
         s.bvh_nodes_visited = (int64_t)h_cnt->bvh_nodes;
         s.tri_tests = (int64_t)h_cnt->tri_tests;
         s.accel[0] = (int32_t)(n_rooms > 1 ? run->bbvh.bytes / (kBvhNodeFloats * sizeof(float)) : hs.bvh_nodes);

@@ -151,6 +151,7 @@ struct __align__(16) ORayItem {
 struct DevCounters {
     unsigned long long primaries, seg_broad, seg_b, seg_c, octave_rays, end_traces, detections, capped,
         retests, queue_overflow, stack_spills, lost_items, bvh_nodes, tri_tests;
+    unsigned long long peak_live;   // of several loops together (k_cond); one loop's: WaveCtl
     double lost_energy, initial_energy;
 };
 
@@ -177,6 +178,7 @@ struct WaveCtl {
     int bounces;                    // surface interactions a ray of this wave may take before it goes back (fused walk)
     unsigned bb_blocks;             // blocks of the phase-A launch that have finished
     int pressure;                   // the ring passed three quarters full since the last batch was fed
+    unsigned long long live_now;    // live rays when this loop's last wave was sized
 };
 
 constexpr size_t kCtlStride = 1024;  // bytes between the schedules of a run's device loops
@@ -260,6 +262,8 @@ struct DevRun {
     const long long *sched_off;   // [2 n_rooms + 1]
     const long long *sched_prim;  // [2 n_rooms]
     unsigned long long *cursor;       // one room, several loops: primaries that the loops have fed together (else null)
+    const WaveCtl *loops;             // the first loop's schedule (kCtlStride bytes apart) and their number
+    int n_loops;
     unsigned *room_live, *room_peak;  // [n_rooms] live rays of each room while pilots run, and their peaks
     // receivers of every room
     // each room's receivers ordered by the coordinate of their widest spread (measured 0.7-4.8 % faster

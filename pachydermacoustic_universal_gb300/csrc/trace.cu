@@ -230,6 +230,7 @@ __device__ void size_wave(const DevRun &r) {
     if (c->done) { c->m = 0; return; }
     const unsigned long long live = __ldcg(&c->tail) - c->head;
     if (live > c->peak_live) c->peak_live = live;
+    c->live_now = live;
     if (c->pilot_count > 0 && live > c->pilot_peak) c->pilot_peak = live;
     // the batches outgrew their plan: plan the next ones with twice the footprint per primary
     if (live > r.ring_cap / 4 * 3 && !c->pressure && c->per_prim) {
@@ -260,6 +261,13 @@ __device__ void size_wave(const DevRun &r) {
 __global__ void k_cond(DevRun r, cudaGraphConditionalHandle h) {
     WaveCtl *c = r.ctl;
     int stop = 0;
+    if (r.n_loops > 1) {  // the rays that all loops hold now, each as its last wave was sized
+        unsigned long long sum = 0;
+        if ((int)threadIdx.x < r.n_loops)
+            sum = __ldcg(&reinterpret_cast<const WaveCtl *>(reinterpret_cast<const char *>(r.loops) + threadIdx.x * kCtlStride)->live_now);
+        for (int o = 1; o < kMaxPipes; o <<= 1) sum += __shfl_xor_sync(FULL, sum, o);
+        if (threadIdx.x == 0) atomicMax(&r.cnt->peak_live, sum);
+    }
     if (threadIdx.x == 0) {
         ++c->iters;
         if (c->m == 0 && c->pa_count == 0 && !c->done) ++c->idle;

@@ -181,6 +181,19 @@ def test_rooms_that_outgrow_the_first_are_traced_in_the_ring_they_fit(big, alpha
     assert sb["segments"] == seg and sb["detections"] == det
 
 
+def test_peak_of_several_loops_is_of_one_time():
+    """The most rays that three loops hold at once: no more than the run's rays or the rings hold, and no less than a
+    third of a run of one loop that is fed the same pilot (each of the three pilots is a third of it or more)."""
+    w = rooms.shoebox_c1()
+    w.cutoff_s = 0.4
+    ds = tracer.DeviceScene(w.scene)
+    for rays in (300, 5000):
+        _, s3 = tracer.trace(w, dscene=ds, rays=rays, seed=6)
+        _, s1 = tracer.trace(w, dscene=ds, rays=rays, seed=6, ring_log2=24)
+        assert s3["kernel_launches"] != s1["kernel_launches"] and s3["octave_rays"] == s1["octave_rays"]
+        assert s1["peak_live_rays"] / 3 <= s3["peak_live_rays"] <= min(s3["octave_rays"], 3 << 22)
+
+
 @pytest.mark.parametrize("kind", ["box", "hall"])
 def test_a_cancelled_run_has_traced_the_first_of_its_primaries(kind):
     """However many loops shared them: what a cancelled run leaves equals a run of its first rays_done primaries, and
