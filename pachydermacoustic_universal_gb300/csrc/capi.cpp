@@ -268,7 +268,7 @@ static void expand_qnodes(const float *nodes, size_t count, float *out, int node
 
 // Appends the scene's planes (see kMaxPlanes); returns how many, 0 when the scene does not qualify.
 int append_planes(const HostScene &hs, SceneArrays &A, int tri_off, int plane_off) {
-    if (hs.ntri > kFuseMaxTris) return 0;
+    if (hs.ntri > kFuseMaxTris || plane_margin(hs) > 1e-5 * kPlanesReach * hs.scale) return 0;
     struct Rec {
         double n[3], d;
         int id;
@@ -546,7 +546,8 @@ void run_worker_body(pach_run *run) {
         // scene: the first room's own device arrays, or the concatenation of every room's
         if (n_rooms == 1) TRY(scene_upload(sc));
         DevScene S = sc->dev;
-        std::vector<int> roots(n_rooms, 0), planes(n_rooms, sc->n_planes), plane_begin(n_rooms, 0);
+        std::vector<int> roots(n_rooms, 0), planes(n_rooms, 0), plane_begin(n_rooms, 0);
+        if (n_rooms == 1) planes[0] = sc->n_planes;
         if (n_rooms > 1) {
             SceneArrays A;
             for (int i = 0; i < n_rooms; ++i) {
@@ -582,6 +583,7 @@ void run_worker_body(pach_run *run) {
             P.bvh_root = roots[i];
             P.plane_begin = plane_begin[i];
             P.n_planes = planes[i];
+            P.plane_eps = (float)plane_margin(hs);
             P.t_eps = (float)(2e-7 * hs.scale);
             P.rec_begin = k;
             P.R = (int)rm.rec.size();

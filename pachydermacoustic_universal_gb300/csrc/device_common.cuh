@@ -383,16 +383,16 @@ __device__ __noinline__ bool trace_ray_again(const DevScene &S, int root, float 
     return trace_ray<int>(S, root, t_eps, o, d, skip, t_best, tri_best, w);
 }
 
-// Nearest hit in a scene of at most kMaxPlanes planes (see PlaneSet in engine.h): the distances to the planes
+// Nearest hit in a scene of at most kMaxPlanes planes (see kMaxPlanes): the distances to the planes
 // first, then the triangles of the nearest ones, nearest plane first, until the next plane begins beyond the hit.
-// A plane begins at its distance less a margin, kPlaneMargin t_eps / |n d| (1e-5 of the room's extent along the
-// normal: the planes' and distances' rounding is at most a tenth of it); a nearly parallel plane counts as near.
+// A plane begins at its distance less a margin, plane_eps / |n d| (plane_margin: the planes' and distances'
+// rounding is at most a tenth of it); a nearly parallel plane counts as near.
 // So every triangle that the BVH could find nearer has been tested, with the same test; ties go to the BVH.  In a
 // convex room a ray tests the two triangles of one plane, without a branch but near edges: about 260
 // instructions where the two-level BVH walk takes 600.
-constexpr float kPlaneMargin = 50.f;  // x t_eps (2e-7 of the extent)
-__device__ __forceinline__ bool plane_walk(const DevScene &S, const float4 *planes, int n, int root, float t_eps, float3 o,
-                                           float3 d, int skip, float &t_best, int &tri_best, TraceWork &w) {
+__device__ __forceinline__ bool plane_walk(const DevScene &S, const float4 *planes, int n, float plane_eps, int root,
+                                           float t_eps, float3 o, float3 d, int skip, float &t_best, int &tri_best,
+                                           TraceWork &w) {
     float tl[kMaxPlanes];
 #pragma unroll
     for (int k = 0; k < kMaxPlanes; ++k) {
@@ -402,7 +402,7 @@ __device__ __forceinline__ bool plane_walk(const DevScene &S, const float4 *plan
         const float nd = fmaf(N.x, d.x, fmaf(N.y, d.y, N.z * d.z));
         const float no = fmaf(N.x, o.x, fmaf(N.y, o.y, fmaf(N.z, o.z, N.w)));
         const float inv = __fdividef(1.0f, nd);
-        const float t = -no * inv, e = kPlaneMargin * t_eps * fabsf(inv);
+        const float t = -no * inv, e = plane_eps * fabsf(inv);
         const bool parallel = fabsf(nd) < 3e-4f;
         if ((parallel || t + e > 0.f) && __float_as_int(planes[2 * k + 1].z) != skip) tl[k] = parallel ? -1.f : t - e;
     }

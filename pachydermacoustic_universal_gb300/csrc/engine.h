@@ -115,9 +115,19 @@ constexpr int kLeafDefault = 3;  // leaf size used when the scene does not ask f
 
 // Scenes of at most kFuseMaxTris triangles in at most kMaxPlanes planes (shoeboxes, simple shells) also carry
 // their planes: two float4 each, (unit normal, offset: n x + offset = 0) and (first entry, entries, coplanar group
-// as int bits) into a list of triangles.  Every vertex lies within 1e-6 of the extent of its plane and no
-// triangle is a sliver (sine of an angle below 0.05), which the walk over planes relies on.
+// as int bits) into a list of triangles.  Every vertex lies within 1e-6 of the extent of its plane, no triangle is a
+// sliver (sine of an angle below 0.05) and no coordinate is more than 16 extents from the origin, which the walk over
+// planes relies on.
 constexpr int kMaxPlanes = 8;
+constexpr double kPlanesReach = 16.0;
+// What the walk allows a distance to a plane to be off by: 1e-5 of the extent, or of the largest coordinate where the
+// room lies off the origin.  Its own rounding is below a tenth of that: n x + offset in FP32 is at most 2^-24 (9 |x| +
+// |offset|) off, 1e-6 of the largest coordinate.
+inline double plane_margin(const HostScene &hs) {
+    double far = hs.scale;
+    for (int k = 0; k < 3; ++k) far = std::max({far, std::fabs(hs.bmin[k]), std::fabs(hs.bmax[k])});
+    return 1e-5 * far;
+}
 
 // Device scene view (passed by value to kernels).
 struct DevScene {
@@ -204,6 +214,7 @@ struct RoomParams {
     int src_begin, nsrc;             // its sources
     int h_oct, oct_lo, oct_hi, is_order, pure_specular, max_broad;
     int plane_begin, n_planes;       // its planes (0: walk the BVH)
+    float plane_eps;                 // plane_margin
 };
 constexpr int kMaxRooms = 4096;
 // Receiver tables up to this size are staged in shared memory by the detection kernels.

@@ -180,6 +180,7 @@ extern "C" pach_status pach_trace_run_noalloc(const pach_scene *scene, const pac
         room.is_order = p.is_order;
         room.pure_specular = p.pure_specular;
         room.n_planes = scene_planes(scene);
+        room.plane_eps = (float)plane_margin(hs);
         room.max_broad = (int)std::fmin((double)max_broad, (double)(1u << 30));
         NA_TRY(cudaMemcpyAsync(base + kOffRoom, &room, sizeof(room), cudaMemcpyHostToDevice, stream));
 

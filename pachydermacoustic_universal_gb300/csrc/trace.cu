@@ -1094,8 +1094,8 @@ __global__ void __launch_bounds__(256, 3) k_bounce(DevRun r) {
             const int root = r.n_rooms > 1 ? P.bvh_root : 0;
             const float teps = r.n_rooms > 1 ? P.t_eps : S.t_eps;
             if constexpr (PLANES)
-                hit = plane_walk(S, r.n_rooms == 1 ? s_plane : S.plane + 2 * P.plane_begin, P.n_planes, root, teps, R.p,
-                                 R.d, R.plane, t, tri, tw);
+                hit = plane_walk(S, r.n_rooms == 1 ? s_plane : S.plane + 2 * P.plane_begin, P.n_planes, P.plane_eps, root,
+                                 teps, R.p, R.d, R.plane, t, tri, tw);
             else
                 hit = trace_ray<int>(S, root, teps, R.p, R.d, R.plane, t, tri, tw);
             L.v[C_RET] += tw.retests;

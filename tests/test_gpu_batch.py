@@ -262,6 +262,27 @@ def test_rays_kept_over_interactions_equal_one_walk_per_launch(kind, ring_log2, 
         np.testing.assert_allclose(ha[name], hb[name], rtol=1e-9, atol=1e-30, err_msg=name)
 
 
+@pytest.mark.parametrize("offset", [40.0, 150.0, 1000.0, 3000.0])
+@pytest.mark.parametrize("kind", ["box", "l"])
+def test_small_rooms_off_the_origin_walk_as_the_bvh_does(kind, offset):
+    """A room that lies many times its extent from the origin: FP32 coordinates there are rounded by more than the
+    margin of a room at the origin.  The walk over planes (up to 16 extents out) and what is used beyond find the
+    BVH walk's hits; at 16 extents the BVH's own boxes are rounded by a tenth of their padding, so a hit may
+    differ in 1e5 segments."""
+    w = rooms.shoebox_c1() if kind == "box" else _l_room()
+    s = np.array([offset, -0.7 * offset, 0.1 * offset])
+    w.scene.vertices = w.scene.vertices + s
+    w.sources = [rooms.SourceSpec(tuple(np.add(x.origin, s)), x.power_db, x.kind) for x in w.sources]
+    w.receivers = [rooms.ReceiverSpec(tuple(np.add(x.origin, s)), x.radius) for x in w.receivers]
+    w.cutoff_s = 0.5
+    ds = tracer.DeviceScene(w.scene)
+    ha, sa = tracer.trace(w, dscene=ds, rays=300, seed=8)
+    hb, sb = tracer.trace(w, dscene=ds, rays=300, seed=8, traversal=1)
+    assert abs(sa["segments"] - sb["segments"]) <= 1e-5 * sb["segments"]
+    assert ha["energy"].sum() == pytest.approx(hb["energy"].sum(), rel=1e-4)
+    assert sa["lost_energy"] == pytest.approx(sb["lost_energy"], rel=1e-3, abs=1e-5 * sb["initial_energy"])
+
+
 @pytest.mark.parametrize("kind", ["hall", "map", "capture", "batch"])
 @pytest.mark.parametrize("rays", [256, 257, 1001])
 def test_primaries_shared_out_to_several_loops_equal_one_loop(kind, rays):
