@@ -399,7 +399,9 @@ __global__ void __launch_bounds__(256) k_ntt_env(FilterJob J, Bufs B, int nj) {
     // factors of the band: P's, and P / E's for the directions (0 where E = 0)
     const double f = J.scale ? J.pmod[b] * J.scale[r] : J.pmod[b];
     const double q = e == 0.0 ? 0.0 : p / e * f;
-    const bool direct = __double2hiint(fabs(q)) >= 0x7FF00000;  // P / E out of range: P Dir / E may not be
+    // P / E out of range or subnormal: P Dir / E may not be
+    const int qh = __double2hiint(fabs(q));
+    const bool direct = qh >= 0x7FF00000 || (qh < 0x00100000 && p != 0.0 && e != 0.0);
     const double pf = p * f, att = in && b == 7 ? B.att[t] : 0.0;
     const int ec = B.ec[b] + kExpBias, ec8 = B.ec[8] + kExpBias;
     // exponent of a value: v 2^ec < 2^(top - kExpBias)
@@ -525,7 +527,7 @@ struct Garner {
 // R-point transforms over the classes, remaindering, scaling: grid (4096 / 128, job).
 template <int R>
 __global__ void __launch_bounds__(128) k_ntt_out(__grid_constant__ const Tables t, __grid_constant__ const Garner G, Bufs B,
-                                                 double *out, int L, int job0) {
+                                                 const double *scale, int kinds, double *out, int L, int job0) {
     const int tp = blockIdx.x * 128 + threadIdx.x, job = blockIdx.y;
     u32 x[kPrimes][R];
 #pragma unroll
@@ -549,6 +551,8 @@ __global__ void __launch_bounds__(128) k_ntt_out(__grid_constant__ const Tables 
     const int ef = B.ef[job];
     const int sh = ef - kExpBias - B.ec[9] - B.ec[10];
     double *o = out + (size_t)(job0 + job) * L;
+    // the envelopes are magnitudes: a receiver's factor below zero turns its filters here
+    const bool turn = scale && scale[(job0 + job) / kinds] < 0.0;
 #pragma unroll
     for (int q = 0; q < R; ++q) {
         int j = 0;  // q bit-reversed
@@ -590,7 +594,7 @@ __global__ void __launch_bounds__(128) k_ntt_out(__grid_constant__ const Tables 
             hi += lo < pl;
         }
         double d = fma((double)v[4], G.m3, (double)hi * 18446744073709551616.0 + (double)lo);
-        d = neg ? -d : d;
+        d = neg != turn ? -d : d;
         o[n] = ef >= kExpNan ? __longlong_as_double(0x7FF8000000000000ll) : (ef == 0 ? 0.0 : scalbn(d, sh));
     }
 }
@@ -720,9 +724,9 @@ cudaError_t ntt_filters(FilterJob J, int n, int fs, double add, int L, double *o
         k_ntt_env_res<<<dim3((9 * T + 255) / 256, nj), 256, 0, st>>>(t, B, T);
         k_ntt_class<<<dim3(R, nj, kPrimes), 256, smem, st>>>(t, B, T);
         const dim3 grid(kN / 128, nj);
-        if (R == 4) k_ntt_out<4><<<grid, 128, 0, st>>>(t, G, B, out, L, j0);
-        else if (R == 8) k_ntt_out<8><<<grid, 128, 0, st>>>(t, G, B, out, L, j0);
-        else k_ntt_out<16><<<grid, 128, 0, st>>>(t, G, B, out, L, j0);
+        if (R == 4) k_ntt_out<4><<<grid, 128, 0, st>>>(t, G, B, J.scale, J.kinds, out, L, j0);
+        else if (R == 8) k_ntt_out<8><<<grid, 128, 0, st>>>(t, G, B, J.scale, J.kinds, out, L, j0);
+        else k_ntt_out<16><<<grid, 128, 0, st>>>(t, G, B, J.scale, J.kinds, out, L, j0);
     }
     return cudaGetLastError();
 }

@@ -142,6 +142,44 @@ def test_device_form_in_several_passes_equals_one_pass():
     _close(outs[0], ref)
 
 
+@pytest.mark.parametrize("kinds", [1, 7])
+@pytest.mark.parametrize("T", [500, 49154])
+def test_receiver_factors_of_any_sign(kinds, T):
+    """d_scale multiplies a receiver's envelopes as it is, a factor below zero (phase reversal) or of zero too, for the
+    integer transforms and (T + 16383 > 65536) the FP64 ones: the filters are the plain ones times the factor."""
+    torch = pytest.importorskip("torch")
+    dev = torch.device("cuda:0")
+    E, P, Dp, Dn = (torch.from_numpy(x).to(dev) for x in _synthetic_histograms(4, T, 9))
+    L = _capi.lib()
+    wsb = L.pach_filters_workspace_bytes(4 * kinds, T)
+    ws = torch.empty(wsb, dtype=torch.uint8, device=dev)
+    got = []
+    f = [1.0, -1.0, -0.375, 0.0]
+    for scale in (None, torch.tensor(f, dtype=torch.float64, device=dev)):
+        out = torch.full((4, kinds, T + 12287), np.nan, dtype=torch.float64, device=dev)
+        _capi.check(L.pach_filters_device(E.data_ptr(), P.data_ptr(), Dp.data_ptr(), Dn.data_ptr(),
+                                          None if scale is None else scale.data_ptr(), 4, T, kinds, 1000, None, 4096,
+                                          out.data_ptr(), ws.data_ptr(), wsb, C.c_void_p(torch.cuda.current_stream().cuda_stream)))
+        torch.cuda.synchronize()
+        got.append(out.cpu().numpy())
+    for r in range(4):
+        for k in range(kinds):
+            peak = np.abs(got[0][r, k]).max()
+            assert peak > 0 and np.abs(got[1][r, k] - f[r] * got[0][r, k]).max() <= 1e-14 * peak, (r, k)
+
+
+def test_directions_of_energies_at_the_ends_of_the_range():
+    """P Dir / E where P / E alone leaves the normal range, upwards or downwards, and the result does not."""
+    E, P, Dp, Dn = _synthetic_histograms(3, 300, 4)
+    ref = tracer.receiver_filters(P, E, Dp, Dn, sample_rate=1000)
+    big, small = 2.0**1000, 2.0**-60  # (P small) / (E big) is subnormal; times (Dir big) it is P Dir / E small again
+    got = tracer.receiver_filters(P * small, E * big, Dp * big, Dn * big, sample_rate=1000)
+    for r in range(3):
+        for k in range(7):
+            peak = np.abs(ref[r, k]).max()
+            assert np.abs(got[r, k] / small - ref[r, k]).max() <= 1e-14 * peak, (r, k)
+
+
 def _device_filters(P, wsb):
     torch = pytest.importorskip("torch")
     dev = torch.device("cuda:0")
