@@ -32,6 +32,7 @@
 
 #include "engine.h"
 #include "mlp_plan.h"
+#include "quotient.h"
 #include "../../include/pach_proposal.h"
 
 namespace pach {
@@ -401,8 +402,8 @@ __device__ __forceinline__ float warp_max(float v) {
 // memory -- a lobe over an eighth of the bins (gradient sums).  Bound: instruction issue, about 30 a bin and
 // lobe.  With a lobe per lane throughout, every bin took two 5-step warp reductions for its maximum and
 // sum: 316 us at 1200 rows, 86 us now.  Every sum keeps the order it had then (lobes pairwise k, k + 16,
-// k + 8, ..; warp w the bins w, w + 8, ..), so the results are the same bits: the gradients are rounded to
-// BF16 next, where a last-bit difference can become a visible one.
+// k + 8, ..; warp w the bins w, w + 8, ..), so the results are the same bits (but for responsibilities below 1e-29, see
+// quotient): the gradients are rounded to BF16 next, where a last-bit difference can become a visible one.
 constexpr int kRespStride = kLobes + 1;  // no bank conflicts in either direction
 __global__ void __launch_bounds__(256) k_vmf_loss(Loss a) {
     __shared__ float4 s_lobe[kLobes];             // mean direction, kappa
@@ -469,13 +470,9 @@ __global__ void __launch_bounds__(256) k_vmf_loss(Loss a) {
 #pragma unroll
                 for (int k = 0; k < h; ++k) t[k] += t[k + h];
             const float q = t[0];
-            // x / q correctly rounded from the rounded reciprocal and one residual step (Markstein 1990)
             const float rq = 1.f / q;
 #pragma unroll
-            for (int k = 0; k < kLobes; ++k) {
-                const float y = x[k] * rq;
-                resp[k] = p * fmaf(fmaf(-q, y, x[k]), rq, y);
-            }
+            for (int k = 0; k < kLobes; ++k) resp[k] = p * quotient(x[k], q, rq);
             s_log[tid] = mx + logf(q);
         } else {
 #pragma unroll
