@@ -848,14 +848,13 @@ void run_worker_body(pach_run *run) {
             const DevRun &r = q.r;
             const cudaStream_t stream = q.stream;
             if (timing && (x = launch_feed(r, stream))) return x;  // graph mode: k_cond feeds
-            if (timing && (x = cudaEventRecord(kev[6 * k], stream))) return x;
+            if (timing && (x = cudaEventRecord(kev[5 * k], stream))) return x;
             if ((x = launch_broadband(r, bb_blocks, bb_threads, stream, map, ntri_max <= kFuseMaxTris))) return x;
-            if (timing && (x = cudaEventRecord(kev[6 * k + 1], stream))) return x;
-            if (timing && (x = cudaEventRecord(kev[6 * k + 2], stream))) return x;
+            if (timing && (x = cudaEventRecord(kev[5 * k + 1], stream))) return x;
             if (sorting && (x = launch_sort(r, sort_blocks, stream))) return x;
-            if (timing && (x = cudaEventRecord(kev[6 * k + 3], stream))) return x;
+            if (timing && (x = cudaEventRecord(kev[5 * k + 2], stream))) return x;
             if (!fused && (x = launch_trace(r, tr_variant, tr_blocks, threads, stream))) return x;
-            if (timing && (x = cudaEventRecord(kev[6 * k + 4], stream))) return x;
+            if (timing && (x = cudaEventRecord(kev[5 * k + 3], stream))) return x;
             // the map's kernel only reads the wave: beside the shading kernel, unless that finds the hits or is timed
             const bool beside = map && !fused && !timing;
             if (beside) {
@@ -870,7 +869,7 @@ void run_worker_body(pach_run *run) {
             if (beside) x = cudaStreamWaitEvent(stream, q.join, 0);
             else if (map) x = launch_map(r, map_blocks, stream);
             if (x) return x;
-            if (timing && (x = cudaEventRecord(kev[6 * k + 5], stream))) return x;
+            if (timing && (x = cudaEventRecord(kev[5 * k + 4], stream))) return x;
             return cudaSuccess;
         };
         // the whole loop of a pipe as one graph launch: feed, then while (k_cond says so) { one iteration }
@@ -1051,7 +1050,7 @@ void run_worker_body(pach_run *run) {
                 int batch = 8;
                 for (long long it = 0;;) {
                     // one batch of iterations, no host synchronisation inside
-                    while (kev.size() < (size_t)batch * 6) {
+                    while (kev.size() < (size_t)batch * 5) {
                         cudaEvent_t x;
                         RTRY(cudaEventCreate(&x));
                         kev.push_back(x);
@@ -1065,10 +1064,10 @@ void run_worker_body(pach_run *run) {
                     RTRY(cudaStreamSynchronize(stream));
                     for (int k = 0; k < batch; ++k) {
                         float a = 0, b = 0, c = 0, so = 0;
-                        RTRY(cudaEventElapsedTime(&a, kev[6 * k], kev[6 * k + 1]));
-                        RTRY(cudaEventElapsedTime(&so, kev[6 * k + 2], kev[6 * k + 3]));
-                        RTRY(cudaEventElapsedTime(&b, kev[6 * k + 3], kev[6 * k + 4]));
-                        RTRY(cudaEventElapsedTime(&c, kev[6 * k + 4], kev[6 * k + 5]));
+                        RTRY(cudaEventElapsedTime(&a, kev[5 * k], kev[5 * k + 1]));
+                        RTRY(cudaEventElapsedTime(&so, kev[5 * k + 1], kev[5 * k + 2]));
+                        RTRY(cudaEventElapsedTime(&b, kev[5 * k + 2], kev[5 * k + 3]));
+                        RTRY(cudaEventElapsedTime(&c, kev[5 * k + 3], kev[5 * k + 4]));
                         t_bb += a;
                         t_sort += so;
                         t_trace += b;

@@ -1022,7 +1022,9 @@ __device__ __forceinline__ ORayItem load_item(const ORayItem *q, unsigned long l
 // ------------------------------------------------------------------------------------------
 // counters
 // ------------------------------------------------------------------------------------------
-// Work of one thread in one launch (32-bit: a thread takes a few hundred rays at most; blocks sum into 64 bits).
+// Work of one thread in one launch, and of a block in shared memory, 32-bit; blocks sum into 64 bits.  A block of the
+// largest default wave (2^23 rays over at least 152 blocks, 32 interactions each) has 1.8 M segments, which a counter
+// holds 2400 times over: as many detections a segment as a room has receivers at most (2048).
 struct LocalCounters {
     unsigned v[11] = {0};  // prim, seg_broad, seg_b, seg_c, oct, end_traces, det, capped, retests, overflow, spills
     double lost = 0, init = 0;

@@ -57,10 +57,10 @@ struct Prime {
 
 struct Tables {                 // kernel argument
     Prime P[kPrimes];
-    int W, R, logR;
+    int W, R;
 };
 
-// Powers of w_W: hi[m >> 8], lo[m & 255] (host-made, 8 KB of kernel argument).
+// Powers of w_W: hi[m >> 8], lo[m & 255] (host-made, 10 KB of kernel argument).
 struct Powers {
     u32 hi[kPrimes][256], lo[kPrimes][256];
 };

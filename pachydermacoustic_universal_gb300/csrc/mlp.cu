@@ -14,9 +14,10 @@
 //
 // Blocked layout ("canonical K-major, no swizzle"): a [rows][K] matrix (rows padded to 128, K a
 // multiple of 16) is a sequence of 128-row tiles; a tile is K/8 slabs of 8 columns, 2048 bytes each;
-// a slab is 16 core matrices of 8 rows x 16 bytes.  So a 128 x 64 chunk of a tile is one contiguous
-// 16 KB block (one bulk copy), and the MMA descriptors use leading (K-direction) byte offset 2048 and
-// stride (row-direction) byte offset 128.
+// a slab is 16 core matrices of 8 rows x 16 bytes.  So a 128 x 128 chunk of A is one contiguous 32 KB block (one bulk
+// copy) with a leading (K-direction) byte offset of 2048 in its MMA descriptors, and 32 rows of a slab of B are 512
+// contiguous bytes (one copy each, laid out with a leading byte offset of 512); the stride (row-direction) byte
+// offset is 128.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
